@@ -130,6 +130,11 @@ struct Params {
     int brick;
     int nb[3];
     const float* majorant;
+    /* fixed-step march: per brick of 2^occ_shift voxels a side, 0 or the distance
+       in bricks to the nearest brick where sigma may be nonzero; NULL: no map */
+    const uint8_t* occ;
+    int occ_shift;
+    int occ_nb[3];
     float gm_inv_max;        /* 1 / max gradient magnitude (hybrid switch) */
     /* camera (Source/camera.h:98-116) */
     int film[2];

@@ -44,6 +44,13 @@ cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, con
    into the empty bricks of a majorant grid; tmp holds 2 bytes per brick */
 cudaError_t er_launch_empty_skip(float* majorant, const int nb[3], uint8_t* tmp, cudaStream_t s);
 
+/* the empty-space map of the fixed-step march: per brick of 2^shift voxels a
+   side, 0 or the Chebyshev distance in bricks (at most 32) to the nearest
+   brick where sigma may be nonzero; count: n words, minmax: one word and tmp:
+   2 bytes per brick */
+cudaError_t er_launch_march_map(const uint16_t* vox, const int res[3], int shift, const int nb[3], const float* sigma, int n,
+                                uint32_t* count, uint32_t* minmax, uint8_t* tmp, uint8_t* occ, cudaStream_t s);
+
 /* the differentiable medium (er_medium.cu) */
 struct DmParams {
     const float* rho;    /* density grid, the tracer volume's resolution, x fastest */
@@ -129,8 +136,7 @@ struct WavefrontBuffers {
                             object-handling variants (at the default occupancy) */
     int pt_primary;      /* the persistent-lane primary stage runs (every view delta-tracks) */
     int pt_shadow;       /* the persistent-lane shadow stage runs (every view delta-tracks) */
-    int skip_primary;    /* the free-flight stage compiles the empty-space skip */
-    int skip_shadow;     /* the shadow stage compiles the empty-space skip */
+    int free_flight;     /* WF_MARCH, WF_DELTA (every view uses that estimator) or WF_MIXED */
     int refill_eighths;  /* persistent stages refill a warp when fewer than this many eighths of its
                             tracking lanes still track (1..7) */
     int sort_shade;      /* a view's shader switch mixes BRDF and phase events: the shade stage runs as

@@ -16,6 +16,11 @@
 
 namespace erd {
 
+/* the free-flight estimators of a launch's views */
+#define WF_MARCH 0
+#define WF_DELTA 1
+#define WF_MIXED 2
+
 #define ER_PI_F 3.141592654f
 #define ER_INV_PI_F 0.31830988618379067154f
 #define ER_INV_TWO_PI_F 0.15915494309189533577f
@@ -387,6 +392,13 @@ ER_D float sigma_point(const Params& P, v3 p)
 {
     if (P.clip_count > 0 && clipped(P, p)) return 0.0f;
     return sigma_at(P, get_intensity(P, p));
+}
+
+/* sigma_point where the march has the point's local coordinates already */
+ER_D float sigma_march(const Params& P, v3 p, float Lx, float Ly, float Lz)
+{
+    if (P.clip_count > 0 && clipped(P, p)) return 0.0f;
+    return sigma_at(P, get_intensity_local(P, Lx, Ly, Lz));
 }
 
 /* sigma_point at a tentative collision of a tracker in majorant brick
@@ -798,6 +810,82 @@ ER_D long long march_budget(float t0, float t1, float step)
     return (long long)(2.0f * n) + 64;
 }
 
+/* The fixed-step march through empty space.  A step whose lookup gives sigma
+   = 0 adds nothing to the march's sum: what is left of it is t += step and
+   the loop's tests.  Most steps are such ones (2067 lookups a sample on the
+   c2 shells, a step a tenth of a voxel, against about 20 in the tissue), so
+   the march asks the empty-space map (Params::occ, er_volume.cu) after a
+   lookup that gave zero, and in an empty brick moves t on, without lookups,
+   to the exit of the cube of empty bricks around it.
+
+   Same t's, same sum, bit for bit:
+   - march_exit evaluates the march's own local coordinates at the exit and
+     gives an exit only if they lie in the cube.  They are monotone in t (each
+     is a chain of rounded monotone operations), so every step before the exit
+     looks up inside the cube, where sigma is zero at every intensity;
+   - march_skip makes the additions t + step one by one, or, while t stays
+     between two powers of two, by their count: there t and the sum's rounding
+     are multiples of one ulp, and once two successive additions have moved t
+     by the same d every further one does (a tie of the rounding, which goes
+     to the even neighbour, leaves t even from its first on).  m d and t + m d
+     are then multiples of the ulp below 2^24 of it: exact.
+
+   Measured: the reference's frame on the 512^3 shells (1024^2) 16.4 -> 3.1 ms,
+   its march at 64 samples a pixel of the 128^3 blobs (256^2) 12.9 -> 4.4 ms;
+   building the map is part of a tracer's build (0.2 ms at 512^3). */
+ER_D float march_exit(const Params& P, const Ray& R, const v3& invd, float Lx, float Ly, float Lz)
+{
+    const float B = (float)(1 << P.occ_shift);
+    const int bx = iclamp((int)floorf(Lx) >> P.occ_shift, 0, P.occ_nb[0] - 1);
+    const int by = iclamp((int)floorf(Ly) >> P.occ_shift, 0, P.occ_nb[1] - 1);
+    const int bz = iclamp((int)floorf(Lz) >> P.occ_shift, 0, P.occ_nb[2] - 1);
+    const int k = __ldg(P.occ + ((size_t)bz * (size_t)P.occ_nb[1] + (size_t)by) * (size_t)P.occ_nb[0] + (size_t)bx);
+    if (k == 0) return -FLT_MAX;
+    const float x0 = (float)(bx - k + 1) * B, x1 = (float)(bx + k) * B;
+    const float y0 = (float)(by - k + 1) * B, y1 = (float)(by + k) * B;
+    const float z0 = (float)(bz - k + 1) * B, z1 = (float)(bz + k) * B;
+    /* the exit a hundredth of a voxel inside the faces (in world units from
+       the box corner: local = (p - minp) * inv_size * res) */
+    const float m = 0.01f;
+    const float ex = (R.D.x > 0.0f ? x1 - m : x0 + m) / (P.inv_size[0] * (float)P.res[0]) + P.minp[0];
+    const float ey = (R.D.y > 0.0f ? y1 - m : y0 + m) / (P.inv_size[1] * (float)P.res[1]) + P.minp[1];
+    const float ez = (R.D.z > 0.0f ? z1 - m : z0 + m) / (P.inv_size[2] * (float)P.res[2]) + P.minp[2];
+    const float tx = R.D.x != 0.0f ? (ex - R.O.x) * invd.x : FLT_MAX;
+    const float ty = R.D.y != 0.0f ? (ey - R.O.y) * invd.y : FLT_MAX;
+    const float tz = R.D.z != 0.0f ? (ez - R.O.z) * invd.z : FLT_MAX;
+    const float te = fminf(fminf(tx, ty), tz);
+    float ax, ay, az;
+    local_coords(P, vadd(R.O, vscale(R.D, te)), ax, ay, az);
+    const bool in = ax >= x0 && ax <= x1 && ay >= y0 && ay <= y1 && az >= z0 && az <= z1;
+    return in ? te : -FLT_MAX;
+}
+
+/* returns whether t moved; every addition is counted in the budget, so a march
+   that calls this ends with it */
+ER_D bool march_skip(float& t, float step, float te, float t_max, long long& budget)
+{
+    const float t0 = t;
+    while (t <= te && t < t_max) {
+        const float u1 = t + step, u2 = u1 + step, u3 = u2 + step;
+        const float d = u3 - u2;
+        const uint32_t e = __float_as_uint(u3) & 0x7f800000u;
+        const float lim = fminf(fminf(te, t_max), __uint_as_float(e + 0x00800000u));
+        if (u2 - u1 == d && d > 0.0f && u1 > 0.0f && (__float_as_uint(u1) & 0x7f800000u) == e && u3 + 4.0f * d < lim) {
+            const float m = truncf((lim - u3) / d) - 1.0f;
+            t = u3 + m * d;
+            budget -= (long long)m + 3;
+        } else {
+            t = u1;
+            if (--budget < 0) break;
+        }
+    }
+    return t > t0;
+}
+
+/* zero lookups between two looks at the map, less one (a power of two less
+   one): in a brick that is not empty the look is in vain */
+#define ER_MARCH_LOOK 3
+
 /* SampleVolume - Source/raymarching.h:30-71 */
 template <bool WITH_NORMAL = true>
 ER_D void sample_volume(const Params& P, const Ray& R, Rng& rng, Event& SE)
@@ -813,11 +901,24 @@ ER_D void sample_volume(const Params& P, const Ray& R, Rng& rng, Event& SE)
     const float StepSize = P.step_primary * P.min_step;
     MinT += rng.get1() * StepSize;
     long long budget = march_budget(MinT, MaxT, StepSize);
+    const v3 invd = V3(1.0f / R.D.x, 1.0f / R.D.y, 1.0f / R.D.z);
+    int zeros = 1;
     while (Sum < S) {
         Ps = vadd(R.O, vscale(R.D, MinT));
         if (MinT >= MaxT) return;
+        float Lx, Ly, Lz;
+        local_coords(P, Ps, Lx, Ly, Lz);
+        if (P.occ && (zeros & ER_MARCH_LOOK) == 1) {
+            zeros++;
+            const float te = march_exit(P, R, invd, Lx, Ly, Lz);
+            if (MinT < te && march_skip(MinT, StepSize, te, MaxT, budget)) {
+                zeros = 1;
+                if (budget >= 0) continue;
+            }
+        }
         if (--budget < 0) { atomicOr(P.err, 1); return; }
-        const float SigmaT = sigma_point(P, Ps);
+        const float SigmaT = sigma_march(P, Ps, Lx, Ly, Lz);
+        zeros = SigmaT == 0.0f ? zeros + 1 : 0;
         Sum += SigmaT * StepSize;
         MinT += StepSize;
     }
@@ -842,11 +943,26 @@ ER_D bool scatter_event_in_volume(const Params& P, const Ray& R, Rng& rng)
     const float StepSize = P.step_shadow * P.min_step;
     MinT += rng.get1() * StepSize;
     long long budget = march_budget(MinT, MaxT, StepSize);
+    const v3 invd = V3(1.0f / R.D.x, 1.0f / R.D.y, 1.0f / R.D.z);
+    /* a shadow ray starts in matter: the first look after the first zero */
+    int zeros = 0;
     while (Sum < S) {
         const v3 Ps = vadd(R.O, vscale(R.D, MinT));
         if (MinT > MaxT) return false;
+        float Lx, Ly, Lz;
+        local_coords(P, Ps, Lx, Ly, Lz);
+        if (P.occ && (zeros & ER_MARCH_LOOK) == 1) {
+            zeros++;
+            const float te = march_exit(P, R, invd, Lx, Ly, Lz);
+            if (MinT < te && march_skip(MinT, StepSize, te, MaxT, budget)) {
+                zeros = 1;
+                if (budget >= 0) continue;
+            }
+        }
         if (--budget < 0) { atomicOr(P.err, 1); return false; }
-        Sum += sigma_point(P, Ps) * StepSize;
+        const float SigmaT = sigma_march(P, Ps, Lx, Ly, Lz);
+        zeros = SigmaT == 0.0f ? zeros + 1 : 0;
+        Sum += SigmaT * StepSize;
         MinT += StepSize;
     }
     return true;
@@ -1081,11 +1197,7 @@ ER_D void dda_jump(const Params& P, Dda& d, int k)
 
 /* Delta tracking of the primary ray: sigma_t = DensityScale^2 * Opacity(I),
    the extinction the reference's march integrates (Source/raymarching.h:45,64-66) */
-/* SKIP: compile the empty-space jump.  Every delta-tracking caller passes
-   true (the tracker's grid carries skip distances, and the jump sets the
-   face times the tracker continues from); false compiles the stages of the
-   fixed-step march, which never run this tracker, with fewer registers. */
-template <bool WITH_NORMAL = true, bool SKIP = true>
+template <bool WITH_NORMAL = true>
 ER_D void sample_volume_delta(const Params& P, const Ray& R, Rng& rng, Event& SE, float u0 = -1.0f)
 {
     Isect Int; Int.invalid();
@@ -1126,7 +1238,7 @@ ER_D void sample_volume_delta(const Params& P, const Ray& R, Rng& rng, Event& SE
                 if (++guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); return; }
                 tau = -er_logf(rng.get1());
             }
-        } else if (SKIP && mu <= -2.0f) {
+        } else if (mu <= -2.0f) {
             dda_jump(P, d, (int)(-mu));
             continue;
         }
@@ -1164,7 +1276,6 @@ ER_D void delta_begin(const Params& P, const Ray& R, Rng& rng, DeltaTracker& k, 
     k.done = false;
 }
 
-template <bool SKIP = true>
 ER_D void delta_step(const Params& P, const Ray& R, Rng& rng, DeltaTracker& k)
 {
     if (!k.in_brick) {
@@ -1186,7 +1297,7 @@ ER_D void delta_step(const Params& P, const Ray& R, Rng& rng, DeltaTracker& k)
         }
         k.tau = k.tau - k.mu * (k.e - k.t);
         if (k.tau < 0.0f) k.tau = 0.0f;
-    } else if (SKIP && k.mu <= -2.0f) {
+    } else if (k.mu <= -2.0f) {
         dda_jump(P, k.d, (int)(-k.mu));
         k.in_brick = false;
         if (k.d.done) k.done = true;
@@ -1229,7 +1340,6 @@ ER_D void ratio_begin(const Params& P, const Ray& R, Rng& rng, RatioTracker& k)
     k.done = false;
 }
 
-template <bool SKIP = true>
 ER_D void ratio_step(const Params& P, const Ray& R, Rng& rng, RatioTracker& k)
 {
     if (!k.in_brick) {
@@ -1256,7 +1366,7 @@ ER_D void ratio_step(const Params& P, const Ray& R, Rng& rng, RatioTracker& k)
         }
         k.tau = k.tau - k.mu * (k.e - k.t);
         if (k.tau < 0.0f) k.tau = 0.0f;
-    } else if (SKIP && k.mu <= -2.0f) {
+    } else if (k.mu <= -2.0f) {
         dda_jump(P, k.d, (int)(-k.mu));
         k.in_brick = false;
         if (k.d.done) k.done = true;
@@ -1269,7 +1379,6 @@ ER_D void ratio_step(const Params& P, const Ray& R, Rng& rng, RatioTracker& k)
 
 /* the same tracking as one loop (the one-kernel paths and the non-persistent
    shadow stage, where it compiles to fewer registers) */
-template <bool SKIP = true>
 ER_D float transmittance_ratio(const Params& P, const Ray& R, Rng& rng)
 {
     Isect Int; Int.invalid();
@@ -1307,7 +1416,7 @@ ER_D float transmittance_ratio(const Params& P, const Ray& R, Rng& rng)
                 if (++guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); return Tr; }
                 tau = -er_logf(rng.get1());
             }
-        } else if (SKIP && mu <= -2.0f) {
+        } else if (mu <= -2.0f) {
             dda_jump(P, d, (int)(-mu));
             continue;
         }
@@ -1330,14 +1439,15 @@ ER_D Ray shadow_ray(const Params& P, v3 P1, v3 P2)
     return R;
 }
 
-template <bool OBJ = true, bool SKIP = true>
+/* FF: as the wavefront stages' (WF_MIXED: read from the parameters) */
+template <bool OBJ = true, int FF = WF_MIXED>
 ER_D float visibility(const Params& P, v3 P1, v3 P2, Rng& rng)
 {
     if (!P.shadows) return 1.0f;
     const Ray R = shadow_ray(P, P1, P2);
     if (intersects_light(P, R)) return 0.0f;
     if (OBJ && P.object_count > 0 && intersects_object(P, R)) return 0.0f;
-    if (P.free_flight == 1) return transmittance_ratio<SKIP>(P, R, rng);
+    if (FF == WF_DELTA || (FF == WF_MIXED && P.free_flight == 1)) return transmittance_ratio(P, R, rng);
     return scatter_event_in_volume(P, R, rng) ? 0.0f : 1.0f;
 }
 

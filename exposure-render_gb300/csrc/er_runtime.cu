@@ -104,6 +104,9 @@ uint64_t fnv1a(uint64_t h, const void* data, size_t n)
 /* items of one wavefront window: 8M samples, 1.5 GB of queues */
 constexpr size_t kWindowCap = (size_t)8 << 20;
 
+/* bricks of the march's empty-space map: 2^2 = 4 voxels a side */
+constexpr int kMarchBrickShift = 2;
+
 /* the persistent stages' refill threshold in eighths of a warp's tracking
    lanes: 2, or ER_PT_REFILL (1..7) for measurements (with the empty-space
    jump and tight bricks, C2 / C3 at 2, 3, 4, 5 eighths: 1336 / 2322, 1333 /
@@ -160,8 +163,7 @@ struct WfQueues {
         B.objects = 0;
         B.pt_primary = 0;
         B.pt_shadow = 0;
-        B.skip_primary = 0;
-        B.skip_shadow = 0;
+        B.free_flight = 2;
         return cudaSuccess;
     }
     /* the shading records of the sorted shade stage, when a view mixes shaders */
@@ -251,6 +253,8 @@ struct TracerItem {
     DevBuf<int> light_ids;
     DevBuf<float> majorant, rmq;   /* majorant: per brick, or -(distance to a non-empty brick) when empty */
     DevBuf<uint8_t> skip_tmp;
+    DevBuf<uint8_t> occ;           /* the march's empty-space map */
+    DevBuf<uint32_t> nonzero;      /* running count of the nonzero entries of the sigma table */
     DevBuf<uint32_t> minmax;
     DevBuf<int> err;
     DevBuf<float> autofocus;       /* er_get_auto_focus_distance's result */
@@ -475,15 +479,12 @@ er_status init_lanes(TracerItem& t)
     return ER_OK;
 }
 
-/* which tracking stages run persistent lanes (ER_PERSISTENT_*; delta
-   tracking only).  Delta-tracking stages always compile the empty-space
-   jump: it sets the face times the tracker continues from, so every path
-   (and the oracle) takes it; the ER_TUNE_NO_SKIP_* bits are accepted and
-   ignored. */
-void persistent_stages(int mode, bool all_delta, WavefrontBuffers& B)
+/* the launch's free-flight estimators, and which tracking stages run
+   persistent lanes (ER_PERSISTENT_*; delta tracking only).  The
+   ER_TUNE_NO_SKIP_* bits are accepted and ignored. */
+void tracking_stages(int mode, bool all_delta, bool any_delta, WavefrontBuffers& B)
 {
-    B.skip_primary = all_delta;
-    B.skip_shadow = all_delta;
+    B.free_flight = all_delta ? ER_FREE_FLIGHT_DELTA : (any_delta ? 2 : ER_FREE_FLIGHT_MARCH);   /* WF_MIXED = 2 */
     mode &= 3;
     B.pt_primary = all_delta && (mode == ER_PERSISTENT_BOTH || mode == ER_PERSISTENT_PRIMARY);
     B.pt_shadow = all_delta && (mode == ER_PERSISTENT_SHADOW || mode == ER_PERSISTENT_BOTH);
@@ -595,6 +596,21 @@ er_status build(TracerItem& t)
         P.brick = brick;
         for (int i = 0; i < 3; i++) P.nb[i] = nb[i];
         P.majorant = t.majorant.p;
+    } else if (v.normalize) {
+        /* the march's empty-space map; without room for it the march makes every lookup */
+        const int shift = kMarchBrickShift;
+        int nb[3];
+        for (int i = 0; i < 3; i++) nb[i] = (v.res[i] + (1 << shift) - 1) >> shift;
+        const size_t total = (size_t)nb[0] * nb[1] * nb[2];
+        if (t.occ.ensure(total) == cudaSuccess && t.minmax.ensure(total) == cudaSuccess && t.skip_tmp.ensure(2 * total) == cudaSuccess &&
+            t.nonzero.ensure((size_t)n) == cudaSuccess) {
+            ER_CUDA(er_launch_march_map(v.vox.p, v.res, shift, nb, t.sigma.p, n, t.nonzero.p, t.minmax.p, t.skip_tmp.p, t.occ.p, st));
+            P.occ = t.occ.p;
+            P.occ_shift = shift;
+            for (int i = 0; i < 3; i++) P.occ_nb[i] = nb[i];
+        } else {
+            cudaGetLastError();
+        }
     }
     /* lights in LightIDs order */
     const int lc = d.light_count;
@@ -797,7 +813,8 @@ er_status trace_sum(TracerItem& t, int spp, uint32_t view, uint32_t first, float
     B.tune_shadow = t.d.settings.tune_shadow > 0 ? t.d.settings.tune_shadow : 4;
     B.tune_shade = t.d.settings.tune_shade > 0 ? t.d.settings.tune_shade : 2;
     B.objects = t.P.object_count > 0;
-    persistent_stages(t.d.settings.tune_stages, t.P.free_flight == ER_FREE_FLIGHT_DELTA, B);
+    const bool delta = t.P.free_flight == ER_FREE_FLIGHT_DELTA;
+    tracking_stages(t.d.settings.tune_stages, delta, delta, B);
     ER_CUDA(t.wf.ensure_sorted(plan, mixes_shaders(t.P), B));
     WfView V;
     memset(&V, 0, sizeof(V));
@@ -893,13 +910,14 @@ er_status batch_plan(BatchItem& b)
     b.B.tune_shadow = b.tune_shadow;
     b.B.tune_shade = b.tune_shade;
     b.B.objects = 0;
-    bool all_delta = true, mixed = false;
+    bool all_delta = true, any_delta = false, mixed = false;
     for (const WfView& hv : b.host_views) {
         b.B.objects |= hv.P.object_count > 0;
         all_delta = all_delta && hv.P.free_flight == ER_FREE_FLIGHT_DELTA;
+        any_delta = any_delta || hv.P.free_flight == ER_FREE_FLIGHT_DELTA;
         mixed = mixed || mixes_shaders(hv.P);
     }
-    persistent_stages(b.tune_stages, all_delta, b.B);
+    tracking_stages(b.tune_stages, all_delta, any_delta, b.B);
     ER_CUDA(b.wf.ensure_sorted(b.plan, mixed, b.B));
     if (b.flags & ER_BATCH_GRAPH) {
         if (!b.capture_stream) ER_CUDA(cudaStreamCreateWithFlags(&b.capture_stream, cudaStreamNonBlocking));

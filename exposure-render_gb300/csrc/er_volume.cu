@@ -1,16 +1,17 @@
 /*
- * er_volume.cu - per-volume pre-passes of the delta tracker.
+ * er_volume.cu - per-volume pre-passes of the free-flight estimators.
  *
  *   k_brick_minmax : min and max voxel of every brick's footprint: voxels
  *                    b B .. (b + 1) B per axis, every corner a trilinear
  *                    lookup (Source/buffer3d.h:222-242) at local coordinates
  *                    in [b B, (b + 1) B] can blend with a nonzero weight (the
  *                    trackers clamp their lookups to that range,
- *                    er_path.cuh sigma_point_in_brick).  One warp per brick,
- *                    coalesced reads along x.
- *   k_rmq_level    : level k of a sparse table of running maxima over the
- *                    sigma table (sigma[I] = DensityScale * Opacity(I)).
+ *                    er_path.cuh sigma_point_in_brick).
+ *   k_rmq          : sparse table of running maxima over the sigma table
+ *                    (sigma[I] = DensityScale * Opacity(I)).
  *   k_majorant     : majorant[brick] = DensityScale * max sigma[lo..hi].
+ *   k_skip_pass    : distances to the nearest non-empty brick.
+ *   k_occupancy    : the empty bricks of the fixed-step march.
  *
  * A lookup inside a brick is a truncated trilinear blend of voxels in
  * [lo, hi]; float rounding of a blend (1 - t) a + t b can fall just below
@@ -27,49 +28,110 @@
 #include "er_capi.h"
 #include "er_kernels.h"
 
-__global__ void k_brick_minmax(const uint16_t* __restrict__ vox, int rx, int ry, int rz, int B, int nbx, int nby, int nbz,
-                               uint32_t* __restrict__ minmax)
+/* Min and max voxel of every brick's footprint, lo | hi << 16.
+
+   Bound by the read of the volume.  A block owns one row of bricks in y, a
+   range of bricks in z and BM_X voxels in x, and walks z plane by plane:
+   each thread reduces the B + 1 rows of its VEC voxels in a plane (coalesced
+   along x, rows of a plane independent loads), a plane that two bricks share
+   in z is read once, and the rows that neighbouring blocks share in y come
+   from L2.  When a brick's last plane is in, the per-x values go through
+   shared memory and one thread per brick takes the B + 1 values of its x
+   range.  One warp per brick, which it replaces, put 5 voxels of a row on 32
+   lanes at 4^3 bricks and took 3.79 ms at 512^3; an edit of the transfer
+   function of that volume with a one-sample picture went from 5.8 to 1.9 ms
+   with this kernel, k_rmq and the outward k_skip_pass. */
+#define BM_THREADS 160
+
+template <int VEC>
+__global__ void __launch_bounds__(BM_THREADS) k_brick_minmax(const uint16_t* __restrict__ vox, int rx, int ry, int rz, int B, int nbx,
+                                                             int nby, int nbz, int xbricks, int zbricks, int xblocks,
+                                                             uint32_t* __restrict__ minmax)
 {
-    const int lane = threadIdx.x & 31;
-    const long long total = (long long)nbx * nby * nbz;
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    /* one warp per brick, grid-stride over the bricks (2^27 at 1^3 bricks of 512^3) */
-    for (long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < total; warp += nwarps) {
-    const int bx = (int)(warp % nbx), by = (int)((warp / nbx) % nby), bz = (int)(warp / ((long long)nbx * nby));
-    const int x0 = bx * B, y0 = by * B, z0 = bz * B;
-    int x1 = (bx + 1) * B, y1 = (by + 1) * B, z1 = (bz + 1) * B;
-    x1 = x1 > rx - 1 ? rx - 1 : x1; y1 = y1 > ry - 1 ? ry - 1 : y1; z1 = z1 > rz - 1 ? rz - 1 : z1;
-    const int wx = x1 - x0 + 1;
-    const int rows = (y1 - y0 + 1) * (z1 - z0 + 1);
-    unsigned int lo = 65535u, hi = 0u;
-    for (int r = 0; r < rows; r++) {
-        const int y = y0 + r % (y1 - y0 + 1);
-        const int z = z0 + r / (y1 - y0 + 1);
-        const uint16_t* row = vox + ((size_t)z * ry + y) * (size_t)rx + x0;
-        for (int x = lane; x < wx; x += 32) {
-            const unsigned int v = __ldg(row + x);
-            lo = v < lo ? v : lo;
-            hi = v > hi ? v : hi;
-        }
-    }
+    /* per-x values of the open brick row: (lo, 65535 - hi) packed, so that one
+       packed minimum serves both; two buffers, so that one barrier a brick suffices */
+    __shared__ uint32_t cols[2][BM_THREADS * VEC];
+    const unsigned row_id = blockIdx.x / (unsigned)xblocks;
+    const int by = (int)(row_id % (unsigned)nby);
+    const int bx0 = (int)(blockIdx.x % (unsigned)xblocks) * xbricks, bx1 = min(bx0 + xbricks, nbx);
+    const int bz0 = (int)(row_id / (unsigned)nby) * zbricks, bz1 = min(bz0 + zbricks, nbz);
+    const int xs = bx0 * B;
+    const int xw = min(bx1 * B, rx - 1) - xs + 1;                 /* voxels of the block's rows */
+    const int y0 = by * B, y1 = min(y0 + B, ry - 1);
+    const int x = (int)threadIdx.x * VEC;
+    const bool in = x < xw;
+    /* a pair's second voxel may lie past the row's last used one but not past the row (rx is even then) */
+    uint32_t open[VEC], plane[VEC];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned int a = __shfl_xor_sync(0xffffffffu, lo, o);
-        const unsigned int b = __shfl_xor_sync(0xffffffffu, hi, o);
-        lo = a < lo ? a : lo;
-        hi = b > hi ? b : hi;
-    }
-    if (lane == 0) minmax[warp] = lo | (hi << 16);
+    for (int v = 0; v < VEC; v++) open[v] = 0xffffffffu;
+    int buf = 0;
+    const int z_end = min(bz1 * B, rz - 1);
+    int z = bz0 * B, bz = bz0;
+    for (; z <= z_end; z++) {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) plane[v] = 0xffffffffu;
+        if (in) {
+            const uint16_t* row = vox + ((size_t)z * ry + y0) * (size_t)rx + xs + x;
+#pragma unroll 4
+            for (int y = y0; y <= y1; y++, row += rx) {
+                if (VEC == 2) {
+                    const uint32_t w = __ldg((const uint32_t*)row);
+                    const uint32_t a = w & 0xffffu, b = w >> 16;
+                    plane[0] = __vminu2(plane[0], a | ((0xffffu ^ a) << 16));
+                    plane[VEC - 1] = __vminu2(plane[VEC - 1], b | ((0xffffu ^ b) << 16));
+                } else {
+                    const uint32_t a = __ldg(row);
+                    plane[0] = __vminu2(plane[0], a | ((0xffffu ^ a) << 16));
+                }
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < VEC; v++) open[v] = __vminu2(open[v], plane[v]);
+        /* brick bz ends with plane (bz + 1) B, or with the volume */
+        if (z == (bz + 1) * B || z == rz - 1) {
+#pragma unroll
+            for (int v = 0; v < VEC; v++) {
+                cols[buf][x + v] = open[v];
+                open[v] = plane[v];
+            }
+            __syncthreads();
+            for (int b = bx0 + (int)threadIdx.x; b < bx1; b += BM_THREADS) {
+                const int c0 = b * B - xs, c1 = min((b + 1) * B, rx - 1) - xs;
+                uint32_t m = 0xffffffffu;
+                for (int c = c0; c <= c1; c++) m = __vminu2(m, cols[buf][c]);
+                minmax[((size_t)bz * nby + by) * (size_t)nbx + b] = m ^ 0xffff0000u;
+            }
+            buf ^= 1;
+            bz++;
+            /* the last voxel plane of a volume that bricks divide without a
+               remainder plus one also closes the brick after it */
+            if (z == rz - 1 && bz < bz1) {
+                z--;
+#pragma unroll
+                for (int v = 0; v < VEC; v++) open[v] = 0xffffffffu;
+            }
+        }
     }
 }
 
-__global__ void k_rmq_level(const float* __restrict__ prev, float* __restrict__ next, int n, int half)
+/* the sparse table of running maxima, level 0 a copy of the sigma table, by
+   one block: a level needs the one before it, and at n <= 65536 a level is a
+   few iterations of the block (a launch a level cost 3 us each, 33 us at
+   n = 2600) */
+__global__ void __launch_bounds__(1024) k_rmq(const float* __restrict__ sigma, float* __restrict__ table, int n, int levels)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float a = prev[i];
-    const float b = (i + half < n) ? prev[i + half] : a;
-    next[i] = b > a ? b : a;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) table[i] = sigma[i];
+    for (int k = 1; k < levels; k++) {
+        __syncthreads();
+        const float* prev = table + (size_t)(k - 1) * n;
+        float* next = table + (size_t)k * n;
+        const int half = 1 << (k - 1);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float a = prev[i];
+            const float b = (i + half < n) ? prev[i + half] : a;
+            next[i] = b > a ? b : a;
+        }
+    }
 }
 
 __global__ void k_majorant(const uint32_t* __restrict__ minmax, const float* __restrict__ table, int n, int levels, float ds,
@@ -92,50 +154,86 @@ __global__ void k_majorant(const uint32_t* __restrict__ minmax, const float* __r
     majorant[i] = ds * m;
 }
 
+/* launches k_brick_minmax: blocks of at most BM_THREADS voxel pairs (or
+   voxels, when the rows are not 4-byte aligned) in x, evenly filled, and z
+   ranges short enough for about 16 blocks per SM (each range reads one plane
+   more than its bricks) */
+static void launch_minmax(const uint16_t* vox, const int res[3], int B, const int nb[3], uint32_t* minmax, cudaStream_t s)
+{
+    const bool pairs = (res[0] & 1) == 0 && ((uintptr_t)vox & 3u) == 0;
+    const int most = (BM_THREADS * (pairs ? 2 : 1) - 1) / B;
+    int xblocks = (nb[0] + most - 1) / most;
+    int xbricks = (nb[0] + xblocks - 1) / xblocks;
+    /* a pair starts at an even voxel: an even number of voxels per block */
+    if (pairs && ((xbricks * B) & 1)) xbricks += xbricks < most ? 1 : -1;
+    if (xbricks < 1) xbricks = 1;
+    xblocks = (nb[0] + xbricks - 1) / xbricks;
+    const long long rows = (long long)xblocks * nb[1];
+    const long long want = 152ll * 16;
+    int zblocks = rows >= want ? 1 : (int)((want + rows - 1) / rows);
+    if (zblocks > nb[2]) zblocks = nb[2];
+    const int zbricks = (nb[2] + zblocks - 1) / zblocks;
+    zblocks = (nb[2] + zbricks - 1) / zbricks;
+    const unsigned grid = (unsigned)(rows * zblocks);
+    if (pairs)
+        k_brick_minmax<2><<<grid, BM_THREADS, 0, s>>>(vox, res[0], res[1], res[2], B, nb[0], nb[1], nb[2], xbricks, zbricks, xblocks, minmax);
+    else
+        k_brick_minmax<1><<<grid, BM_THREADS, 0, s>>>(vox, res[0], res[1], res[2], B, nb[0], nb[1], nb[2], xbricks, zbricks, xblocks, minmax);
+}
+
 cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, const int nb[3], const float* sigma, int n,
                                float* rmq, int levels, uint32_t* minmax, float density_scale, float* majorant, cudaStream_t s)
 {
     const long long total = (long long)nb[0] * nb[1] * nb[2];
-    const long long want = (total * 32 + 255) / 256;
-    k_brick_minmax<<<(unsigned)(want < 65536 ? want : 65536), 256, 0, s>>>(vox, res[0], res[1], res[2], B, nb[0], nb[1], nb[2],
-                                                                           minmax);
-    cudaError_t e = cudaMemcpyAsync(rmq, sigma, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
-    for (int k = 1; k < levels; k++)
-        k_rmq_level<<<(n + 255) / 256, 256, 0, s>>>(rmq + (size_t)(k - 1) * n, rmq + (size_t)k * n, n, 1 << (k - 1));
+    launch_minmax(vox, res, B, nb, minmax, s);
+    k_rmq<<<1, 1024, 0, s>>>(sigma, rmq, n, levels);
     k_majorant<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(minmax, rmq, n, levels, density_scale, majorant, total);
     return cudaGetLastError();
 }
 
-/* Empty-space distances of the majorant grid.  For an empty brick (majorant
-   0) dist = min over non-empty bricks q of max_a |b_a - q_a| (Chebyshev
-   distance in bricks), capped at ER_SKIP_CAP; computed exactly by three 1D
-   passes (x: nearest non-empty along the row; y and z: min over offsets of
-   max(offset, previous pass)).  The last pass writes -dist into the empty
-   bricks of the majorant grid: a tracker in such a brick knows every brick
-   within dist-1 of it is empty too (er_path.cuh dda_jump). */
+/* Empty-space distances of a brick grid.  For an empty brick dist = min over
+   non-empty bricks q of max_a |b_a - q_a| (Chebyshev distance in bricks),
+   capped at ER_SKIP_CAP; computed exactly by three 1D passes (x: nearest
+   non-empty along the row; y and z: min over offsets of max(offset, previous
+   pass)).  A pass looks outwards from its brick and stops at the first
+   offset that is no smaller than the best distance so far, so its length is
+   the distance it finds, not the 63 bricks of the cap's window (94 us a pass
+   at 128^3 bricks of a half-filled volume).  For the delta trackers
+   (k_skip_pass<0>) a brick is empty where its majorant is not positive, and
+   the last pass writes -dist into the empty bricks of the majorant grid; for
+   the fixed-step march (k_skip_pass<1>) the x pass reads the occupancy bytes
+   of k_occupancy and the last pass writes dist (0: not empty) as bytes.  A
+   ray in a brick at distance dist knows every brick within dist-1 of it is
+   empty too (er_path.cuh dda_jump, march_skip). */
 #define ER_SKIP_CAP 32
 
+template <int MARCH>
 __global__ void k_skip_pass(const float* __restrict__ majorant, const uint8_t* __restrict__ in, uint8_t* __restrict__ out,
                             float* __restrict__ majorant_out, int axis, int nbx, int nby, int nbz, long long total)
 {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int b[3] = { (int)(i % nbx), (int)((i / nbx) % nby), (int)(i / ((long long)nbx * nby)) };
         const int n = axis == 0 ? nbx : (axis == 1 ? nby : nbz);
         const long long step = axis == 0 ? 1 : (axis == 1 ? (long long)nbx : (long long)nbx * nby);
-        int best = ER_SKIP_CAP;
-        for (int o = -(ER_SKIP_CAP - 1); o <= ER_SKIP_CAP - 1; o++) {
-            const int c = b[axis] + o;
-            if (c < 0 || c >= n) continue;
-            const int ao = o < 0 ? -o : o;
-            if (ao >= best) continue;
-            const long long j = i + (long long)o * step;
-            const int v = axis == 0 ? (majorant[j] > 0.0f ? 0 : ER_SKIP_CAP) : (int)in[j];
-            const int d = v > ao ? v : ao;
-            best = d < best ? d : best;
+        const int c = (int)((i / step) % n);
+        auto at = [&](long long j) -> int {
+            if (!MARCH && axis == 0) return majorant[j] > 0.0f ? 0 : ER_SKIP_CAP;
+            return (int)in[j];
+        };
+        int best = at(i);
+        for (int o = 1; o < best; o++) {
+            if (c - o >= 0) {
+                const int v = at(i - o * step);
+                const int d = v > o ? v : o;
+                best = d < best ? d : best;
+            }
+            if (c + o < n) {
+                const int v = at(i + o * step);
+                const int d = v > o ? v : o;
+                best = d < best ? d : best;
+            }
         }
-        if (axis < 2) out[i] = (uint8_t)best;
+        if (MARCH || axis < 2) out[i] = (uint8_t)best;
         else if (!(majorant_out[i] > 0.0f)) majorant_out[i] = -(float)best;
     }
 }
@@ -145,9 +243,66 @@ cudaError_t er_launch_empty_skip(float* majorant, const int nb[3], uint8_t* tmp,
     const long long total = (long long)nb[0] * nb[1] * nb[2];
     const long long want = (total + 255) / 256;
     const unsigned blocks = (unsigned)(want < 65536 ? want : 65536);
-    k_skip_pass<<<blocks, 256, 0, s>>>(majorant, nullptr, tmp, nullptr, 0, nb[0], nb[1], nb[2], total);
-    k_skip_pass<<<blocks, 256, 0, s>>>(majorant, tmp, tmp + total, nullptr, 1, nb[0], nb[1], nb[2], total);
-    k_skip_pass<<<blocks, 256, 0, s>>>(majorant, tmp + total, nullptr, majorant, 2, nb[0], nb[1], nb[2], total);
+    k_skip_pass<0><<<blocks, 256, 0, s>>>(majorant, nullptr, tmp, nullptr, 0, nb[0], nb[1], nb[2], total);
+    k_skip_pass<0><<<blocks, 256, 0, s>>>(nullptr, tmp, tmp + total, nullptr, 1, nb[0], nb[1], nb[2], total);
+    k_skip_pass<0><<<blocks, 256, 0, s>>>(nullptr, tmp + total, nullptr, majorant, 2, nb[0], nb[1], nb[2], total);
+    return cudaGetLastError();
+}
+
+/* The empty-space map of the fixed-step march: dist bytes of bricks of
+   2^shift voxels a side (k_skip_pass<1>).  A brick is empty when sigma is
+   exactly zero (of either sign) at every intensity a lookup in it can have,
+   lo - 1 .. hi as for the majorant: a step there adds nothing to the march's
+   sum, so the march may leave the lookup out.  A negative or NaN sigma counts
+   as not empty. */
+__global__ void __launch_bounds__(1024) k_nonzero_prefix(const float* __restrict__ sigma, uint32_t* __restrict__ count, int n)
+{
+    __shared__ uint32_t part[32];
+    const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int i0 = min((int)threadIdx.x * per, n), i1 = min(i0 + per, n);
+    uint32_t mine = 0;
+    for (int i = i0; i < i1; i++) mine += sigma[i] != 0.0f ? 1u : 0u;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) part[w] = incl;
+    __syncthreads();
+    uint32_t run = incl - mine;
+    for (int k = 0; k < w; k++) run += part[k];
+    for (int i = i0; i < i1; i++) {
+        run += sigma[i] != 0.0f ? 1u : 0u;
+        count[i] = run;
+    }
+}
+
+__global__ void k_occupancy(const uint32_t* __restrict__ minmax, const uint32_t* __restrict__ count, int n, uint8_t* __restrict__ occ,
+                            long long total)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const uint32_t mm = minmax[i];
+    int lo = (int)(mm & 0xffffu) - 1, hi = (int)(mm >> 16);
+    lo = lo < 0 ? 0 : (lo > n - 1 ? n - 1 : lo);
+    hi = hi > n - 1 ? n - 1 : hi;
+    const uint32_t below = lo > 0 ? count[lo - 1] : 0u;
+    occ[i] = count[hi] == below ? ER_SKIP_CAP : 0;
+}
+
+cudaError_t er_launch_march_map(const uint16_t* vox, const int res[3], int shift, const int nb[3], const float* sigma, int n,
+                                uint32_t* count, uint32_t* minmax, uint8_t* tmp, uint8_t* occ, cudaStream_t s)
+{
+    const long long total = (long long)nb[0] * nb[1] * nb[2];
+    const long long want = (total + 255) / 256;
+    const unsigned blocks = (unsigned)(want < 65536 ? want : 65536);
+    launch_minmax(vox, res, 1 << shift, nb, minmax, s);
+    k_nonzero_prefix<<<1, 1024, 0, s>>>(sigma, count, n);
+    k_occupancy<<<(unsigned)want, 256, 0, s>>>(minmax, count, n, occ, total);
+    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, occ, tmp, nullptr, 0, nb[0], nb[1], nb[2], total);
+    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, tmp, tmp + total, nullptr, 1, nb[0], nb[1], nb[2], total);
+    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, tmp + total, occ, nullptr, 2, nb[0], nb[1], nb[2], total);
     return cudaGetLastError();
 }
 
