@@ -38,6 +38,11 @@ struct Plf {                 /* PiecewiseLinearFunction<128> (Source/plf.h:26-92
     float range0, range1;
     float pos[128];
     float val[128];
+    /* where an evaluation's scan starts (plf_start): [range0, range1] in 64
+       buckets of width 1 / bucket_scale, each with the first segment that
+       meets it; built with the record (er_runtime.cu to_plf) */
+    float bucket_scale;
+    uint8_t first[64];
 };
 
 struct Tfs {                 /* the four colour/scalar TFs read at scatter events */
@@ -250,18 +255,32 @@ struct Rng {
 /* transfer functions - Source/plf.h:68-91                              */
 /* ------------------------------------------------------------------ */
 
+/* the first segment that the scan for x has to look at (x within the range):
+   no segment before it meets x's bucket, in whatever order the nodes lie, so
+   the scan from here finds the segment that the scan from the first node
+   finds (64 nodes: about 2 tests instead of 32) */
+template <typename Real>
+ER_D int plf_start(const Plf& p, Real x)
+{
+    const Real u = (x - (Real)p.range0) * (Real)p.bucket_scale;
+    const int j = (int)u;
+    return p.first[j < 0 ? 0 : (j > 63 ? 63 : j)];
+}
+
 ER_D float plf_eval(const Plf& p, float x)
 {
     const int n = p.count;
     if (n <= 0) return 0.0f;
     if (x < p.range0) return p.val[0];
     if (x > p.range1) return p.val[n - 1];
-    for (int i = 1; i < n; i++) {
+    for (int i = plf_start<float>(p, x); i < n; i++) {
         const float P1 = p.pos[i - 1];
         const float P2 = p.pos[i];
-        const float DeltaP = P2 - P1;
-        const float LerpT = (x - P1) / DeltaP;
-        if (x >= P1 && x < P2) return p.val[i - 1] + LerpT * (p.val[i] - p.val[i - 1]);
+        if (x >= P1 && x < P2) {
+            const float DeltaP = P2 - P1;
+            const float LerpT = (x - P1) / DeltaP;
+            return p.val[i - 1] + LerpT * (p.val[i] - p.val[i - 1]);
+        }
     }
     return 0.0f;
 }

@@ -10,7 +10,7 @@
  * u = 2 + rho * (n - 5), C2 in rho on [-1/(n-5), 1 + 1/(n-5)] and linear in
  * the values.
  *
- * Estimator (one thread per sample): the camera ray's tentative collisions
+ * Estimator: the camera ray's tentative collisions
  * come from a fixed majorant grid (the delta tracker's DDA); at each, with
  * probability q (a draw independent of the medium) a next-event estimate to
  * one uniformly picked light with a ratio-tracked shadow segment, weighted
@@ -50,14 +50,6 @@ struct DmLookup {
     Real rho;
 };
 
-ER_D uint32_t dm_index(const Params& P, int x, int y, int z)
-{
-    const int cx = x < 0 ? 0 : (x > P.res[0] - 1 ? P.res[0] - 1 : x);
-    const int cy = y < 0 ? 0 : (y > P.res[1] - 1 ? P.res[1] - 1 : y);
-    const int cz = z < 0 ? 0 : (z > P.res[2] - 1 ? P.res[2] - 1 : z);
-    return (uint32_t)cz * (uint32_t)P.res[0] * (uint32_t)P.res[1] + (uint32_t)cy * (uint32_t)P.res[0] + (uint32_t)cx;
-}
-
 template <typename Real>
 ER_D void dm_density(const Params& P, const DmParams& M, v3 p, DmLookup<Real>& k)
 {
@@ -68,11 +60,17 @@ ER_D void dm_density(const Params& P, const DmParams& M, v3 p, DmLookup<Real>& k
     const int vx = (int)floorf(Lx), vy = (int)floorf(Ly), vz = (int)floorf(Lz);
     const float dx = Lx - (float)vx, dy = Ly - (float)vy, dz = Lz - (float)vz;
     const float ex = 1.0f - dx, ey = 1.0f - dy, ez = 1.0f - dz;
+    /* clamping per axis and the eight sums of the two corners' offsets: the
+       indices of a clamp per corner in a third of its instructions */
+    const uint32_t rx = (uint32_t)P.res[0], slice = rx * (uint32_t)P.res[1];
+    const uint32_t x0 = (uint32_t)iclamp(vx, 0, P.res[0] - 1), x1 = (uint32_t)iclamp(vx + 1, 0, P.res[0] - 1);
+    const uint32_t y0 = (uint32_t)iclamp(vy, 0, P.res[1] - 1) * rx, y1 = (uint32_t)iclamp(vy + 1, 0, P.res[1] - 1) * rx;
+    const uint32_t z0 = (uint32_t)iclamp(vz, 0, P.res[2] - 1) * slice, z1 = (uint32_t)iclamp(vz + 1, 0, P.res[2] - 1) * slice;
     Real r = 0.0f;
 #pragma unroll
     for (int c = 0; c < 8; c++) {
         const int ox = c & 1, oy = (c >> 1) & 1, oz = (c >> 2) & 1;
-        k.idx[c] = dm_index(P, vx + ox, vy + oy, vz + oz);
+        k.idx[c] = (ox ? x1 : x0) + (oy ? y1 : y0) + (oz ? z1 : z0);
         k.w[c] = (ox ? dx : ex) * (oy ? dy : ey) * (oz ? dz : ez);
         r = r + (Real)k.w[c] * (Real)__ldg(M.rho + k.idx[c]);
     }
@@ -100,12 +98,12 @@ ER_D Real dm_plf(const Plf& p, const float* vals, Real x, int& i0, int& nb, Real
     if (n <= 0) return 0.0f;
     if (x < (Real)p.range0) { nb = 1; b[0] = 1.0f; return (Real)__ldg(vals); }
     if (x > (Real)p.range1) { nb = 1; i0 = n - 1; b[0] = 1.0f; return (Real)__ldg(vals + n - 1); }
-    for (int i = 1; i < n; i++) {
+    for (int i = plf_start<Real>(p, x); i < n; i++) {
         const Real P1 = p.pos[i - 1];
         const Real P2 = p.pos[i];
-        const Real DeltaP = P2 - P1;
-        const Real LerpT = (x - P1) / DeltaP;
         if (x >= P1 && x < P2) {
+            const Real DeltaP = P2 - P1;
+            const Real LerpT = (x - P1) / DeltaP;
             const Real v0 = __ldg(vals + i - 1), v1 = __ldg(vals + i);
             i0 = i - 1;
             nb = 2;
@@ -129,10 +127,12 @@ ER_D Real dm_tf_value(const Plf& p, Real x)
         if (n <= 0) return 0.0;
         if (x < (Real)p.range0) return p.val[0];
         if (x > (Real)p.range1) return p.val[n - 1];
-        for (int i = 1; i < n; i++) {
+        for (int i = plf_start<Real>(p, x); i < n; i++) {
             const Real P1 = p.pos[i - 1], P2 = p.pos[i];
-            const Real LerpT = (x - P1) / (P2 - P1);
-            if (x >= P1 && x < P2) return (Real)p.val[i - 1] + LerpT * ((Real)p.val[i] - (Real)p.val[i - 1]);
+            if (x >= P1 && x < P2) {
+                const Real LerpT = (x - P1) / (P2 - P1);
+                return (Real)p.val[i - 1] + LerpT * ((Real)p.val[i] - (Real)p.val[i - 1]);
+            }
         }
         return 0.0;
     }
@@ -141,7 +141,7 @@ ER_D Real dm_tf_value(const Plf& p, Real x)
 ER_D float dm_tf_slope(const Plf& p, float x)
 {
     if (p.count <= 0 || x < p.range0 || x > p.range1) return 0.0f;
-    for (int i = 1; i < p.count; i++) {
+    for (int i = plf_start<float>(p, x); i < p.count; i++) {
         const float P1 = p.pos[i - 1], P2 = p.pos[i];
         if (x >= P1 && x < P2) return (p.val[i] - p.val[i - 1]) / (P2 - P1);
     }
@@ -186,17 +186,17 @@ ER_D void dm_opacity(const Params& P, const DmParams& M, Real rho, DmTf<Real>& o
     o.dalpha = slope ? du * (d0 * v0 + d1 * v1 + d2 * v2 + d3 * v3) : (Real)0.0f;
 }
 
-/* dLoss/dsigma = a at one lookup, scattered into the gradients */
-ER_D void dm_scatter(const DmParams& M, const DmLookup<float>& k, const DmTf<float>& o, float a, float* g_rho, float* s_tf)
+/* dLoss/dsigma = a and dLoss/dI = aI at one lookup, scattered into the gradients */
+ER_D void dm_scatter(const DmParams& M, const DmLookup<float>& k, const DmTf<float>& o, float a, float aI, float* g_rho, float* s_tf)
 {
     const float as = a * M.scale;
-    if (s_tf) {
+    if (s_tf && a != 0.0f) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
             if (j < o.nb) atomicAdd(s_tf + o.i0 + j, as * o.b[j]);
     }
-    if (g_rho && o.dalpha != 0.0f) {
-        const float ar = as * o.dalpha;
+    const float ar = as * o.dalpha + aI;
+    if (g_rho && ar != 0.0f) {
 #pragma unroll
         for (int c = 0; c < 8; c++) atomicAdd(g_rho + k.idx[c], ar * k.w[c]);
     }
@@ -272,7 +272,10 @@ ER_D void dm_shade_prepare(const Params& P, const DmParams& M, v3 Pt, Real I, co
     }
     h.gm = dm_sqrt(sum);
     const Real NGM = h.gm * (Real)M.gm_inv;
-    const Real Exponent = (Real)25.0f * dm_pow((Real)P.gradient_factor, (Real)3.0f) * NGM;
+    Real gf3;
+    if constexpr (sizeof(Real) == sizeof(float)) gf3 = M.gf3;
+    else gf3 = dm_pow((Real)P.gradient_factor, (Real)3.0f);
+    const Real Exponent = (Real)25.0f * gf3 * NGM;
     h.pb = P.opacity_modulated ? o.alpha * ((Real)1.0f - dm_exp(-Exponent)) : (Real)1.0f - dm_exp(-Exponent);
 }
 
@@ -373,7 +376,7 @@ ER_D void dm_shade_adjoint(const Params& P, const DmParams& M, const DmShade<flo
     const Tfs& T = *P.tfs;
     if (h.type == 2) {
         const float apb = aS[0] * (Sb[0] - Sp[0]) + aS[1] * (Sb[1] - Sp[1]) + aS[2] * (Sb[2] - Sp[2]);
-        const float GF3 = er_powf(P.gradient_factor, 3.0f);
+        const float GF3 = M.gf3;
         const float ex = er_expf(-25.0f * GF3 * h.gm * M.gm_inv);
         const float mod = P.opacity_modulated ? o.alpha : 1.0f;
         if (P.opacity_modulated) aop += apb * (1.0f - ex);
@@ -480,9 +483,9 @@ ER_D bool dm_segment(const Params& P, const Ray& R, float& t0, float& t1)
     return t0 < t1;
 }
 
-/* ratio-tracked shadow transmittance; ADJ scatters -a_scale / (mu - sigma) */
-template <bool ADJ, int MODEL, typename Real = float>
-ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng, float a_scale, float* g_rho, float* s_tf)
+/* ratio-tracked shadow transmittance as one loop (the binary64 evaluation) */
+template <int MODEL, typename Real>
+ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng)
 {
     if (!P.shadows) return 1.0f;
     const v3 W = vnorm(vsub(P2, P1));
@@ -517,7 +520,6 @@ ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng, 
                 DmTf<Real> o;
                 dm_opacity<Real, MODEL>(P, M, k.rho, o);
                 const Real sig = (Real)M.scale * o.alpha;
-                if constexpr (ADJ) dm_scatter(M, k, o, -a_scale / (mu - sig), g_rho, s_tf);
                 Tr = Tr * ((Real)1.0f - sig / (Real)mu);
                 if (++guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); return Tr; }
                 tau = -er_logf(rng.get1());
@@ -662,28 +664,49 @@ ER_D void dm_walk(const Params& P, const DmParams& M, int x, int y, Rng& rng, Vi
 /* ---- the wavefront estimator ------------------------------------------
    A window of items (item = s * npix + pixel, s counted from the window's
    first sample row):
-     k_dm_count   : walk, count the item's shadow jobs, reserve their slots
-     k_dm_jobs    : walk again, write the jobs in order (point, light
-                    sample, unshadowed estimate, T * w, stream index)
-     k_dm_shadow  : one thread per job: the ratio-tracked transmittance
+     k_dm_count   : walk without the medium (the draws do not depend on it),
+                    count the item's next-event estimates, reserve their slots
+     k_dm_jobs    : walk again, write the estimates in order (point, T * w,
+                    stream index, the random state of the light sample)
+     k_dm_shade   : one thread per job: light sample, shading, the
+                    unshadowed estimate A0
+     k_dm_shadow  : the jobs' ratio-tracked transmittances
      k_dm_gather  : per item, L = sum over its jobs in order of (A0 Tr) (T w)
-   adjoint (after the four above):
+   adjoint (after the five above):
      k_dm_adj_primary : walk again with each job's transmittance: the
                         collision terms, and g . c per job
-     k_dm_adj_shadow  : one thread per job: the shadow-segment terms
-   Every float operation and its order are the oracle's. */
+     k_dm_adj_shade   : model 1, one thread per job: through the shading
+     k_dm_adj_shadow  : the shadow-segment terms
+   Every float operation and its order are the oracle's.
+
+   What bounds the walks is lanes: with the shading inside the walk, k_dm_jobs
+   ran 5.8 of 32 lanes at 8 warps an SM and waited for instructions on most
+   cycles (4.8 warps an issue; its adjoint 9.1, at 5.4 lanes and 128
+   registers).  So the shading, which only needs the collision's point and
+   random state, runs one thread per job with full warps, and the walks are
+   small loops over persistent lanes (dm_lanes).  Forward and adjoint of the
+   tracer's model, 128^3 grid, 256^2 x 32 samples: 99.3 -> 11.7 ms; of the
+   B-spline model, 72 x 65 x 81, 150 x 111 x 16: 2.8 -> 1.6 ms. */
 
 struct DmJobs {
     float4* P;         /* Pt, T * w */
     float4* S;         /* light sample, g . c (adjoint) */
     float4* A;         /* A0, transmittance */
-    uint2* id;         /* item in the window, k_nee */
+    uint2* id;         /* item in the window, index of the estimate along the ray (DM_DARK: no light sample) */
+    uint2* rng;        /* random state before the light sample's draws */
     uint32_t* off;     /* per item: first job */
     uint32_t* cnt;     /* per item: jobs */
-    uint32_t* total;   /* jobs of the window */
+    uint32_t* total;   /* jobs of the window; items or jobs taken by the walks follow (DM_FETCH_*) */
     uint32_t cap;      /* job slots */
     float4* E;         /* model 1: per item, the emission summed along the walk (NULL for model 0) */
 };
+
+#define DM_DARK 0x80000000u
+#define DM_FETCH_JOBS 1
+#define DM_FETCH_SHADOW 2
+#define DM_FETCH_ADJ_PRIMARY 3
+#define DM_FETCH_ADJ_SHADOW 4
+#define DM_COUNTERS 5
 
 struct DmWindow {
     uint32_t npix;
@@ -701,7 +724,126 @@ ER_D void dm_item(const Params& P, const DmWindow& W, uint32_t i, uint32_t& pix,
     y = (int)(pix / (uint32_t)P.film[0]);
 }
 
-template <int MODEL>
+/* a ray's tentative collisions, one brick or collision per step */
+struct DmTrack {
+    Ray R;
+    Dda d;
+    float tau, t, e, mu;
+    int guard;
+    bool in_brick, done;
+};
+
+ER_D void dm_track_begin(const Params& P, Rng& rng, DmTrack& k)
+{
+    k.done = true;
+    k.in_brick = false;
+    k.guard = 0;
+    float t0, t1;
+    if (!dm_segment(P, k.R, t0, t1)) return;
+    dda_init(P, k.R, t0, t1, k.d);
+    k.tau = -er_logf(rng.get1());
+    k.done = k.d.done;
+}
+
+/* moves to the next collision in this brick (true, at k.t) or to the next brick */
+ER_D bool dm_track_step(const Params& P, DmTrack& k)
+{
+    if (!k.in_brick) {
+        k.e = dda_exit(k.d);
+        k.mu = dda_majorant(P, k.d);
+        k.t = k.d.t;
+    }
+    k.in_brick = false;
+    if (k.mu > 0.0f) {
+        const float dt = k.tau / k.mu;
+        if (k.t + dt < k.e) {
+            k.t = k.t + dt;
+            k.in_brick = true;
+            return true;
+        }
+        k.tau = k.tau - k.mu * (k.e - k.t);
+        if (k.tau < 0.0f) k.tau = 0.0f;
+    }
+    dda_advance(P, k.d, k.e);
+    k.done = k.d.done;
+    return false;
+}
+
+/* after a collision: the next optical distance */
+ER_D void dm_track_next(const Params& P, Rng& rng, DmTrack& k)
+{
+    if (++k.guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); k.done = true; return; }
+    k.tau = -er_logf(rng.get1());
+}
+
+/* The persistent lanes of a walk.  A warp's lanes cross bricks together until
+   few of them still do (a quarter), then those at a collision make their
+   lookups together; lanes whose ray ended take new work when a quarter of the
+   warp waits, one atomic per warp.  begin(i): sets the lane's ray up for work
+   item i (tracker not done) or leaves it done; collide(): the lane's
+   collision; end(): the ray is done. */
+template <typename Begin, typename Collide, typename End>
+ER_D void dm_lanes(const Params& P, DmTrack& k, uint32_t n, uint32_t* fetch, Begin begin, Collide collide, End end)
+{
+    const int lane = threadIdx.x & 31;
+    bool have = false, exhausted = false;
+    for (;;) {
+        const unsigned free_lanes = __ballot_sync(0xffffffffu, !have && !exhausted);
+        const unsigned busy = __ballot_sync(0xffffffffu, have);
+        if (!free_lanes && !busy) break;
+        if (free_lanes && (!busy || __popc(free_lanes) >= 8)) {
+            uint32_t base = 0;
+            const int leader = __ffs(free_lanes) - 1;
+            if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(free_lanes));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (!have && !exhausted) {
+                const uint32_t i = base + (uint32_t)__popc(free_lanes & ((1u << lane) - 1u));
+                if (i < n) {
+                    begin(i);
+                    have = true;
+                } else {
+                    exhausted = true;
+                }
+            }
+            __syncwarp();
+        }
+        bool hit = false;
+        const int start = __popc(__ballot_sync(0xffffffffu, have && !k.done));
+        for (;;) {
+            const bool crossing = have && !k.done && !hit;
+            const unsigned m = __ballot_sync(0xffffffffu, crossing);
+            if (4 * __popc(m) <= start) break;
+            if (crossing) hit = dm_track_step(P, k);
+        }
+        if (hit) collide();
+        __syncwarp();
+        if (have && k.done) {
+            end();
+            have = false;
+        }
+        __syncwarp();
+    }
+}
+
+/* the camera ray of an item and the state its walk starts from */
+ER_D void dm_item_ray(const Params& P, const DmWindow& W, uint32_t i, Rng& rng, Ray& R)
+{
+    uint32_t pix, sample;
+    int x, y;
+    dm_item(P, W, i, pix, sample, x, y);
+    er_seed_lanes(P.seed, W.view, pix, sample, &rng.s0, &rng.s1);
+    const v2 film_uv = rng.get2();
+    const v2 lens_uv = rng.get2();
+    R = sample_camera(P, x, y, film_uv, lens_uv);
+}
+
+/* the draws of dm_nee */
+ER_D void dm_nee_draws(Rng& rng)
+{
+    rng.get1();
+    rng.get3();
+}
+
 __global__ void __launch_bounds__(256) k_dm_count(const Params P, const DmParams M, const DmWindow W, DmJobs J)
 {
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -709,14 +851,18 @@ __global__ void __launch_bounds__(256) k_dm_count(const Params P, const DmParams
         const uint32_t i = base + threadIdx.x;
         uint32_t n = 0;
         if (i < W.items) {
-            uint32_t pix, sample;
-            int x, y;
-            dm_item(P, W, i, pix, sample, x, y);
             Rng rng;
-            er_seed_lanes(P.seed, W.view, pix, sample, &rng.s0, &rng.s1);
-            auto count = [&](const DmHit<float>& h, const DmLookup<float>&, const DmTf<float>&, float, float, float,
-                             const DmShade<float>&) { n += h.has ? 1u : 0u; };
-            dm_walk<float, MODEL>(P, M, x, y, rng, count);
+            DmTrack k;
+            dm_item_ray(P, W, i, rng, k.R);
+            dm_track_begin(P, rng, k);
+            while (!k.done) {
+                if (!dm_track_step(P, k)) continue;
+                if (rng.get1() < M.q) {
+                    dm_nee_draws(rng);
+                    n++;
+                }
+                dm_track_next(P, rng, k);
+            }
         }
         /* warp-aggregated reservation of the item's job slots */
         const int lane = threadIdx.x & 31;
@@ -736,49 +882,145 @@ __global__ void __launch_bounds__(256) k_dm_count(const Params P, const DmParams
 }
 
 template <int MODEL>
-__global__ void __launch_bounds__(256) k_dm_jobs(const Params P, const DmParams M, const DmWindow W, DmJobs J)
+__global__ void __launch_bounds__(256, 3) k_dm_jobs(const Params P, const DmParams M, const DmWindow W, DmJobs J)
 {
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.items; i += stride) {
-        uint32_t pix, sample;
-        int x, y;
-        dm_item(P, W, i, pix, sample, x, y);
-        Rng rng;
-        er_seed_lanes(P.seed, W.view, pix, sample, &rng.s0, &rng.s1);
-        uint32_t j = J.off[i];
-        const uint32_t end = j + J.cnt[i];
-        c3 E = C3(0, 0, 0);
-        auto write = [&](const DmHit<float>& h, const DmLookup<float>&, const DmTf<float>&, float, float w, float T,
-                         const DmShade<float>&) {
-            if (MODEL == 1) E = cadd(E, cscale(C3(h.Le[0], h.Le[1], h.Le[2]), T * w));
-            if (!h.has || j >= end || j >= J.cap) return;
-            J.P[j] = make_float4(h.Pt.x, h.Pt.y, h.Pt.z, T * w);
-            J.S[j] = make_float4(h.S.x, h.S.y, h.S.z, 0.0f);
-            J.A[j] = make_float4(h.A0[0], h.A0[1], h.A0[2], 0.0f);
-            J.id[j] = make_uint2(i, h.k_nee);
-            j++;
-        };
-        dm_walk<float, MODEL>(P, M, x, y, rng, write);
-        if (J.E) J.E[i] = make_float4(E.r, E.g, E.b, 0.0f);
-    }
+    uint32_t i = 0, j = 0, end = 0, nee = 0;
+    float T = 1.0f;
+    c3 E = C3(0, 0, 0);
+    Rng rng;
+    DmTrack k;
+    dm_lanes(P, k, W.items, J.total + DM_FETCH_JOBS,
+        [&](uint32_t item) {
+            i = item;
+            j = J.off[i];
+            end = j + J.cnt[i];
+            nee = 0;
+            T = 1.0f;
+            E = C3(0, 0, 0);
+            dm_item_ray(P, W, i, rng, k.R);
+            dm_track_begin(P, rng, k);
+        },
+        [&]() {
+            const v3 Pt = vadd(k.R.O, vscale(k.R.D, k.t));
+            DmLookup<float> l;
+            dm_density(P, M, Pt, l);
+            DmTf<float> o;
+            dm_opacity<float, MODEL>(P, M, l.rho, o);
+            const float sig = M.scale * o.alpha;
+            if (!(sig < k.mu)) atomicOr(P.err, 4);   /* the majorant no longer bounds sigma */
+            const float w = sig / k.mu;
+            if (MODEL == 1) {
+                c3 Le = C3(0, 0, 0);
+                if (M.emissive) Le = ctf_eval(P.tfs->emission, l.rho);
+                E = cadd(E, cscale(Le, T * w));
+            }
+            if (rng.get1() < M.q) {
+                if (j < end && j < J.cap) {
+                    J.P[j] = make_float4(Pt.x, Pt.y, Pt.z, T * w);
+                    J.id[j] = make_uint2(i, nee);
+                    J.rng[j] = make_uint2(rng.s0, rng.s1);
+                    j++;
+                }
+                nee++;
+                dm_nee_draws(rng);
+            }
+            T = T * (1.0f - w);
+            dm_track_next(P, rng, k);
+        },
+        [&]() {
+            if (J.E) J.E[i] = make_float4(E.r, E.g, E.b, 0.0f);
+        });
+}
+
+/* minus the camera ray's direction of a job's item */
+ER_D v3 dm_job_wo(const Params& P, const DmWindow& W, uint32_t item)
+{
+    Rng rng;
+    Ray R;
+    dm_item_ray(P, W, item, rng, R);
+    return vneg(R.D);
 }
 
 template <int MODEL>
-__global__ void __launch_bounds__(256) k_dm_shadow(const Params P, const DmParams M, const DmWindow W, DmJobs J)
+__global__ void __launch_bounds__(128) k_dm_shade(const Params P, const DmParams M, const DmWindow W, DmJobs J)
 {
     const uint32_t n = min(*J.total, J.cap);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const uint2 id = J.id[j];
-        uint32_t pix, sample;
-        int x, y;
-        dm_item(P, W, id.x, pix, sample, x, y);
-        Rng sh;
-        dm_shadow_stream(P.seed, W.view, pix, sample, id.y, sh);
-        const float4 p = J.P[j], s = J.S[j];
-        const float Tr = dm_shadow<false, MODEL>(P, M, V3(p.x, p.y, p.z), V3(s.x, s.y, s.z), sh, 0.0f, nullptr, nullptr);
-        J.A[j].w = Tr;
+        const float4 p = J.P[j];
+        const uint2 id = J.id[j], st = J.rng[j];
+        const v3 Pt = V3(p.x, p.y, p.z);
+        Rng rng;
+        rng.s0 = st.x;
+        rng.s1 = st.y;
+        v3 S = V3(0, 0, 0), Wi;
+        c3 LiK;
+        bool has;
+        const c3 a0 = dm_nee(P, M, Pt, rng, S, has, Wi, LiK);
+        c3 A = C3(0, 0, 0);
+        if (has) {
+            A = a0;
+            if (MODEL == 1) {
+                DmLookup<float> l;
+                dm_density(P, M, Pt, l);
+                DmTf<float> o;
+                dm_opacity<float, MODEL>(P, M, l.rho, o);
+                DmShade<float> sd;
+                dm_shade_prepare<float>(P, M, Pt, l.rho, o, sd);
+                float Sv[3], Sb[3], Sp[3];
+                dm_shade_eval<float>(P, sd, dm_job_wo(P, W, id.x), Wi, Sv, Sb, Sp);
+                A = C3(Sv[0] * a0.r, Sv[1] * a0.g, Sv[2] * a0.b);
+            }
+        } else {
+            J.id[j] = make_uint2(id.x, id.y | DM_DARK);
+        }
+        J.S[j] = make_float4(S.x, S.y, S.z, 0.0f);
+        J.A[j] = make_float4(A.r, A.g, A.b, 0.0f);
     }
+}
+
+/* sets a job's shadow segment up in the tracker; false: nothing lies on it
+   (transmittance 1) */
+ER_D void dm_shadow_begin(const Params& P, const DmWindow& W, uint2 id, float4 p, float4 s, Rng& rng, DmTrack& k)
+{
+    k.done = true;
+    k.in_brick = false;
+    if (!P.shadows) return;
+    uint32_t pix, sample;
+    int x, y;
+    dm_item(P, W, id.x, pix, sample, x, y);
+    dm_shadow_stream(P.seed, W.view, pix, sample, id.y, rng);
+    k.R = shadow_ray(P, V3(p.x, p.y, p.z), V3(s.x, s.y, s.z));
+    dm_track_begin(P, rng, k);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(256, 3) k_dm_shadow(const Params P, const DmParams M, const DmWindow W, DmJobs J)
+{
+    const uint32_t n = min(*J.total, J.cap);
+    uint32_t j = 0;
+    float Tr = 1.0f;
+    Rng rng;
+    DmTrack k;
+    dm_lanes(P, k, n, J.total + DM_FETCH_SHADOW,
+        [&](uint32_t job) {
+            j = job;
+            Tr = 1.0f;
+            k.done = true;
+            const uint2 id = J.id[j];
+            if (!(id.y & DM_DARK)) dm_shadow_begin(P, W, id, J.P[j], J.S[j], rng, k);
+        },
+        [&]() {
+            const v3 Pt = vadd(k.R.O, vscale(k.R.D, k.t));
+            DmLookup<float> l;
+            dm_density(P, M, Pt, l);
+            DmTf<float> o;
+            dm_opacity<float, MODEL>(P, M, l.rho, o);
+            const float sig = M.scale * o.alpha;
+            Tr = Tr * (1.0f - sig / k.mu);
+            dm_track_next(P, rng, k);
+        },
+        [&]() { J.A[j].w = Tr; });
 }
 
 /* L of every item of the window in sample order; out = the item's slot of the
@@ -790,6 +1032,7 @@ __global__ void k_dm_gather(const DmWindow W, const DmJobs J, uint64_t base, flo
     c3 L = C3(0, 0, 0);
     const uint32_t j0 = J.off[i], j1 = j0 + J.cnt[i];
     for (uint32_t j = j0; j < j1 && j < J.cap; j++) {
+        if (J.id[j].y & DM_DARK) continue;
         const float4 a = J.A[j];
         const float Tw = J.P[j].w;
         const c3 A = cscale(C3(a.x, a.y, a.z), a.w);
@@ -826,79 +1069,91 @@ ER_D void dm_tf_flush(const DmParams& M, const float* row, float* g_tf)
 }
 
 template <int MODEL>
-__global__ void __launch_bounds__(256) k_dm_adj_primary(const Params P, const DmParams M, const DmWindow W, DmJobs J, uint64_t base,
-                                                        const float* __restrict__ dimg, const float* __restrict__ fwd,
-                                                        float* __restrict__ g_rho, float* __restrict__ g_tf)
+__global__ void __launch_bounds__(256, 3) k_dm_adj_primary(const Params P, const DmParams M, const DmWindow W, DmJobs J, uint64_t base,
+                                                           const float* __restrict__ dimg, const float* __restrict__ fwd,
+                                                           float* __restrict__ g_rho, float* __restrict__ g_tf)
 {
     __shared__ float rows[DM_WARPS][ER_MAX_TF_NODES];
     float* row = dm_tf_row(rows);
     float* s_tf = g_tf ? row : nullptr;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < W.items; i += stride) {
-        uint32_t pix, sample;
-        int x, y;
-        dm_item(P, W, i, pix, sample, x, y);
-        const c3 g = C3(dimg[3 * pix], dimg[3 * pix + 1], dimg[3 * pix + 2]);
-        if (g.r == 0.0f && g.g == 0.0f && g.b == 0.0f) continue;
-        const uint64_t q = 3 * (base + i);
-        const c3 Lt = C3(fwd[q], fwd[q + 1], fwd[q + 2]);
-        Rng rng;
-        er_seed_lanes(P.seed, W.view, pix, sample, &rng.s0, &rng.s1);
-        uint32_t j = J.off[i];
-        const uint32_t end = j + J.cnt[i];
-        c3 L = C3(0, 0, 0), E = C3(0, 0, 0);
-        auto adj = [&](const DmHit<float>& h, const DmLookup<float>& k, const DmTf<float>& o, float sig, float w, float T,
-                       const DmShade<float>& sd) {
+    uint32_t j = 0, end = 0;
+    float T = 1.0f;
+    c3 g = C3(0, 0, 0), Lt = C3(0, 0, 0), L = C3(0, 0, 0), E = C3(0, 0, 0);
+    Rng rng;
+    DmTrack k;
+    dm_lanes(P, k, W.items, J.total + DM_FETCH_ADJ_PRIMARY,
+        [&](uint32_t i) {
+            const uint32_t pix = i % W.npix;
+            k.done = true;
+            g = C3(dimg[3 * pix], dimg[3 * pix + 1], dimg[3 * pix + 2]);
+            j = J.off[i];
+            end = j + J.cnt[i];
+            if (g.r == 0.0f && g.g == 0.0f && g.b == 0.0f) {
+                /* kept jobs may hold an earlier adjoint's g . c */
+                for (; j < end && j < J.cap; j++) J.S[j].w = 0.0f;
+                return;
+            }
+            const uint64_t q = 3 * (base + i);
+            Lt = C3(fwd[q], fwd[q + 1], fwd[q + 2]);
+            T = 1.0f;
+            L = E = C3(0, 0, 0);
+            dm_item_ray(P, W, i, rng, k.R);
+            dm_track_begin(P, rng, k);
+        },
+        [&]() {
+            const v3 Pt = vadd(k.R.O, vscale(k.R.D, k.t));
+            DmLookup<float> l;
+            dm_density(P, M, Pt, l);
+            DmTf<float> o;
+            dm_opacity<float, MODEL>(P, M, l.rho, o);
+            const float sig = M.scale * o.alpha;
+            const float w = sig / k.mu;
             c3 A = C3(0, 0, 0);
-            float Tr = 0.0f;
-            bool shaded = false;
-            if (h.has && j < end && j < J.cap) {
-                const float4 a = J.A[j];
-                Tr = a.w;
-                A = cscale(C3(a.x, a.y, a.z), a.w);
-                const c3 c = cscale(A, T * w);
-                L = cadd(L, c);
-                J.S[j].w = g.r * c.r + g.g * c.g + g.b * c.b;
-                j++;
-                shaded = MODEL == 1;
+            if (rng.get1() < M.q) {
+                if (j < end && j < J.cap) {
+                    const float4 a = J.A[j];
+                    float gc = 0.0f;
+                    if (!(J.id[j].y & DM_DARK)) {
+                        A = cscale(C3(a.x, a.y, a.z), a.w);
+                        const c3 c = cscale(A, T * w);
+                        L = cadd(L, c);
+                        gc = g.r * c.r + g.g * c.g + g.b * c.b;
+                    }
+                    J.S[j].w = gc;
+                    j++;
+                }
+                dm_nee_draws(rng);
             }
             /* dL/dsigma = T A / mu - (Ltot - L_<=k) / (mu - sigma), A the
-               collision's whole contribution before T w */
-            const c3 Le = C3(h.Le[0], h.Le[1], h.Le[2]);
-            if (MODEL == 1) E = cadd(E, cscale(Le, T * w));
-            const c3 Ak = MODEL == 1 ? cadd(Le, A) : A;
-            const c3 rest = csub(Lt, MODEL == 1 ? cadd(L, E) : L);
-            const c3 dLds = csub(cscale(Ak, T / h.mu), cdivs(rest, h.mu - sig));
-            const float a = g.r * dLds.r + g.g * dLds.g + g.b * dLds.b;
-            if (MODEL == 1) {
-                /* through the emission and shading at I, and the hybrid's
-                   opacity modulation */
+               collision's whole contribution before T w; through I, model 1's
+               emission (its shading: k_dm_adj_shade) */
+            float aI = 0.0f;
+            c3 Ak = A;
+            if (MODEL == 1 && M.emissive) {
+                const Tfs& F = *P.tfs;
+                const c3 Le = ctf_eval(F.emission, l.rho);
+                E = cadd(E, cscale(Le, T * w));
+                Ak = cadd(Le, A);
                 const c3 gA = cscale(g, T * w);
-                float aI = 0.0f, aop = 0.0f;
-                if (M.emissive)
-                    aI += gA.r * dm_tf_slope(P.tfs->emission[0], k.rho) + gA.g * dm_tf_slope(P.tfs->emission[1], k.rho) +
-                          gA.b * dm_tf_slope(P.tfs->emission[2], k.rho);
-                if (shaded) {
-                    float ag[6];
-                    const float aS[3] = { gA.r * Tr * h.LiK.r, gA.g * Tr * h.LiK.g, gA.b * Tr * h.LiK.b };
-                    dm_shade_adjoint(P, M, sd, o, k.rho, h.Wo, h.Wi, aS, aI, aop, ag);
-                    if (sd.type != 1) dm_scatter_gradient_lookups(P, M, h.Pt, ag, g_rho);
-                }
-                dm_scatter_rho(k, aI, g_rho);
-                const float at = a + aop / M.scale;
-                if (at != 0.0f) dm_scatter(M, k, o, at, g_rho, s_tf);
-            } else if (a != 0.0f) {
-                dm_scatter(M, k, o, a, g_rho, s_tf);
+                aI = gA.r * dm_tf_slope(F.emission[0], l.rho) + gA.g * dm_tf_slope(F.emission[1], l.rho) +
+                     gA.b * dm_tf_slope(F.emission[2], l.rho);
             }
-        };
-        dm_walk<float, MODEL>(P, M, x, y, rng, adj);
-    }
+            const c3 rest = csub(Lt, MODEL == 1 ? cadd(L, E) : L);
+            const c3 dLds = csub(cscale(Ak, T / k.mu), cdivs(rest, k.mu - sig));
+            const float a = g.r * dLds.r + g.g * dLds.g + g.b * dLds.b;
+            dm_scatter(M, l, o, a, aI, g_rho, s_tf);
+            T = T * (1.0f - w);
+            dm_track_next(P, rng, k);
+        },
+        [&]() {});
     if (g_tf) dm_tf_flush(M, row, g_tf);
 }
 
-template <int MODEL>
-__global__ void __launch_bounds__(256) k_dm_adj_shadow(const Params P, const DmParams M, const DmWindow W, DmJobs J,
-                                                       float* __restrict__ g_rho, float* __restrict__ g_tf)
+/* model 1: a job's adjoint through its shading - the transfer functions at
+   its intensity, the hybrid's opacity modulation and the normal */
+__global__ void __launch_bounds__(256, 2) k_dm_adj_shade(const Params P, const DmParams M, const DmWindow W, DmJobs J,
+                                                         const float* __restrict__ dimg, float* __restrict__ g_rho,
+                                                         float* __restrict__ g_tf)
 {
     __shared__ float rows[DM_WARPS][ER_MAX_TF_NODES];
     float* row = dm_tf_row(rows);
@@ -906,17 +1161,67 @@ __global__ void __launch_bounds__(256) k_dm_adj_shadow(const Params P, const DmP
     const uint32_t n = min(*J.total, J.cap);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) {
-        const float gc = J.S[j].w;
-        if (gc == 0.0f) continue;
-        const uint2 id = J.id[j];
-        uint32_t pix, sample;
-        int x, y;
-        dm_item(P, W, id.x, pix, sample, x, y);
-        Rng sh;
-        dm_shadow_stream(P.seed, W.view, pix, sample, id.y, sh);
-        const float4 p = J.P[j], s = J.S[j];
-        dm_shadow<true, MODEL>(P, M, V3(p.x, p.y, p.z), V3(s.x, s.y, s.z), sh, gc, g_rho, s_tf);
+        const uint2 id = J.id[j], st = J.rng[j];
+        if (id.y & DM_DARK) continue;
+        const uint32_t pix = id.x % W.npix;
+        const c3 g = C3(dimg[3 * pix], dimg[3 * pix + 1], dimg[3 * pix + 2]);
+        if (g.r == 0.0f && g.g == 0.0f && g.b == 0.0f) continue;
+        const float4 p = J.P[j];
+        const float Tr = J.A[j].w;
+        const v3 Pt = V3(p.x, p.y, p.z);
+        Rng rng;
+        rng.s0 = st.x;
+        rng.s1 = st.y;
+        v3 S, Wi;
+        c3 LiK;
+        bool has;
+        dm_nee(P, M, Pt, rng, S, has, Wi, LiK);
+        DmLookup<float> l;
+        dm_density(P, M, Pt, l);
+        DmTf<float> o;
+        dm_opacity<float, 1>(P, M, l.rho, o);
+        DmShade<float> sd;
+        dm_shade_prepare<float>(P, M, Pt, l.rho, o, sd);
+        const c3 gA = cscale(g, p.w);
+        const float aS[3] = { gA.r * Tr * LiK.r, gA.g * Tr * LiK.g, gA.b * Tr * LiK.b };
+        float aI = 0.0f, aop = 0.0f, ag[6];
+        dm_shade_adjoint(P, M, sd, o, l.rho, dm_job_wo(P, W, id.x), Wi, aS, aI, aop, ag);
+        if (sd.type != 1) dm_scatter_gradient_lookups(P, M, Pt, ag, g_rho);
+        dm_scatter(M, l, o, aop / M.scale, aI, g_rho, s_tf);
     }
+    if (g_tf) dm_tf_flush(M, row, g_tf);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(256, 3) k_dm_adj_shadow(const Params P, const DmParams M, const DmWindow W, DmJobs J,
+                                                          float* __restrict__ g_rho, float* __restrict__ g_tf)
+{
+    __shared__ float rows[DM_WARPS][ER_MAX_TF_NODES];
+    float* row = dm_tf_row(rows);
+    float* s_tf = g_tf ? row : nullptr;
+    const uint32_t n = min(*J.total, J.cap);
+    float gc = 0.0f;
+    Rng rng;
+    DmTrack k;
+    dm_lanes(P, k, n, J.total + DM_FETCH_ADJ_SHADOW,
+        [&](uint32_t j) {
+            k.done = true;
+            const float4 s = J.S[j];
+            gc = s.w;
+            const uint2 id = J.id[j];
+            if (gc != 0.0f && !(id.y & DM_DARK)) dm_shadow_begin(P, W, id, J.P[j], s, rng, k);
+        },
+        [&]() {
+            const v3 Pt = vadd(k.R.O, vscale(k.R.D, k.t));
+            DmLookup<float> l;
+            dm_density(P, M, Pt, l);
+            DmTf<float> o;
+            dm_opacity<float, MODEL>(P, M, l.rho, o);
+            const float sig = M.scale * o.alpha;
+            dm_scatter(M, l, o, -gc / (k.mu - sig), 0.0f, g_rho, s_tf);
+            dm_track_next(P, rng, k);
+        },
+        [&]() {});
     if (g_tf) dm_tf_flush(M, row, g_tf);
 }
 
@@ -946,7 +1251,7 @@ __global__ void __launch_bounds__(256) k_dm_forward64(const Params P, const DmPa
             if (!h.has) return;
             Rng sh;
             dm_shadow_stream(P.seed, view, pix, first + s, h.k_nee, sh);
-            const double Tr = dm_shadow<false, MODEL, double>(P, M, h.Pt, h.S, sh, 0.0f, nullptr, nullptr);
+            const double Tr = dm_shadow<MODEL, double>(P, M, h.Pt, h.S, sh);
             L0 += h.A0[0] * Tr * T * w;
             L1 += h.A0[1] * Tr * T * w;
             L2 += h.A0[2] * Tr * T * w;
@@ -1060,7 +1365,7 @@ unsigned grid_for(uint64_t items, int per_sm)
 /* job storage of the wavefront medium estimator, grown on demand */
 struct DmWorkspace {
     float4 *P = nullptr, *S = nullptr, *A = nullptr;
-    uint2* id = nullptr;
+    uint2 *id = nullptr, *rng = nullptr;
     uint32_t *off = nullptr, *cnt = nullptr, *total = nullptr, *host_total = nullptr;
     float4* E = nullptr;       /* model 1: per item emission sums */
     size_t cap = 0, item_cap = 0;
@@ -1071,13 +1376,13 @@ struct DmWorkspace {
     uint32_t kept_jobs = 0;    /* the kept walk's job count */
     ~DmWorkspace()
     {
-        cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id); cudaFree(off); cudaFree(cnt); cudaFree(total); cudaFree(E);
+        cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id); cudaFree(rng); cudaFree(off); cudaFree(cnt); cudaFree(total); cudaFree(E);
         if (host_total) cudaFreeHost(host_total);
     }
     cudaError_t ensure_items(size_t n)
     {
         if (!total) {
-            cudaError_t e = cudaMalloc(&total, sizeof(uint32_t));
+            cudaError_t e = cudaMalloc(&total, DM_COUNTERS * sizeof(uint32_t));
             if (e == cudaSuccess) e = cudaMallocHost(&host_total, sizeof(uint32_t));
             if (e != cudaSuccess) return e;
         }
@@ -1095,13 +1400,14 @@ struct DmWorkspace {
     {
         if (n <= cap) return cudaSuccess;
         n = n + n / 4;
-        cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id);
+        cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id); cudaFree(rng);
         P = S = A = nullptr;
-        id = nullptr;
+        id = rng = nullptr;
         cudaError_t e = cudaMalloc(&P, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&S, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&A, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&id, n * sizeof(uint2));
+        if (e == cudaSuccess) e = cudaMalloc(&rng, n * sizeof(uint2));
         cap = e == cudaSuccess ? n : 0;
         return e;
     }
@@ -1146,35 +1452,48 @@ static cudaError_t dm_windows(const Params& P, const DmParams& M, int spp, uint3
         W.view = view;
         W.first = first;
         DmJobs J;
-        J.P = ws.P; J.S = ws.S; J.A = ws.A; J.id = ws.id; J.off = ws.off; J.cnt = ws.cnt; J.total = ws.total;
+        J.P = ws.P; J.S = ws.S; J.A = ws.A; J.id = ws.id; J.rng = ws.rng; J.off = ws.off; J.cnt = ws.cnt; J.total = ws.total;
         J.E = M.model == 1 ? ws.E : nullptr;
         J.cap = (uint32_t)ws.cap;
         const uint64_t base = (uint64_t)s0 * npix;
         uint32_t njobs = ws.kept_jobs;
+        /* the walks run one resident wave of persistent lanes */
+        const unsigned wave = (unsigned)sm_count() * 3;
         if (!reuse) {
-            if ((e = cudaMemsetAsync(ws.total, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
-            if (M.model == 1) k_dm_count<1><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J);
-            else k_dm_count<0><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J);
+            if ((e = cudaMemsetAsync(ws.total, 0, DM_COUNTERS * sizeof(uint32_t), s)) != cudaSuccess) return e;
+            k_dm_count<<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J);
             if ((e = cudaMemcpyAsync(ws.host_total, ws.total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
             if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
             njobs = *ws.host_total;
             if ((e = ws.ensure_jobs(njobs)) != cudaSuccess) return e;
-            J.P = ws.P; J.S = ws.S; J.A = ws.A; J.id = ws.id; J.cap = (uint32_t)ws.cap;
-            if (M.model == 1) k_dm_jobs<1><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J);
-            else k_dm_jobs<0><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J);
-            if (njobs && M.model == 1) k_dm_shadow<1><<<grid_for(njobs, 16), 256, 0, s>>>(P, M, W, J);
-            else if (njobs) k_dm_shadow<0><<<grid_for(njobs, 16), 256, 0, s>>>(P, M, W, J);
+            J.P = ws.P; J.S = ws.S; J.A = ws.A; J.id = ws.id; J.rng = ws.rng; J.cap = (uint32_t)ws.cap;
+            if (M.model == 1) k_dm_jobs<1><<<wave, 256, 0, s>>>(P, M, W, J);
+            else k_dm_jobs<0><<<wave, 256, 0, s>>>(P, M, W, J);
+            if (njobs) {
+                const unsigned jobs_grid = grid_for((uint64_t)njobs * 2, 32);
+                if (M.model == 1) {
+                    k_dm_shade<1><<<jobs_grid, 128, 0, s>>>(P, M, W, J);
+                    k_dm_shadow<1><<<wave, 256, 0, s>>>(P, M, W, J);
+                } else {
+                    k_dm_shade<0><<<jobs_grid, 128, 0, s>>>(P, M, W, J);
+                    k_dm_shadow<0><<<wave, 256, 0, s>>>(P, M, W, J);
+                }
+            }
             ws.kept_jobs = njobs;
+        } else {
+            if ((e = cudaMemsetAsync(ws.total + 1, 0, (DM_COUNTERS - 1) * sizeof(uint32_t), s)) != cudaSuccess) return e;
         }
-        if (!dimg || samples) {
-            /* forward values: written by the forward, read by the adjoint */
-            if (!dimg) k_dm_gather<<<(W.items + 255) / 256, 256, 0, s>>>(W, J, base, samples);
-        }
+        /* forward values: written by the forward, read by the adjoint */
+        if (!dimg) k_dm_gather<<<(W.items + 255) / 256, 256, 0, s>>>(W, J, base, samples);
         if (dimg) {
-            if (M.model == 1) k_dm_adj_primary<1><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J, base, dimg, samples, g_rho, g_tf);
-            else k_dm_adj_primary<0><<<grid_for(W.items, 16), 256, 0, s>>>(P, M, W, J, base, dimg, samples, g_rho, g_tf);
-            if (njobs && M.model == 1) k_dm_adj_shadow<1><<<grid_for(njobs, 16), 256, 0, s>>>(P, M, W, J, g_rho, g_tf);
-            else if (njobs) k_dm_adj_shadow<0><<<grid_for(njobs, 16), 256, 0, s>>>(P, M, W, J, g_rho, g_tf);
+            if (M.model == 1) {
+                k_dm_adj_primary<1><<<wave, 256, 0, s>>>(P, M, W, J, base, dimg, samples, g_rho, g_tf);
+                if (njobs) k_dm_adj_shade<<<grid_for(njobs, 16), 256, 0, s>>>(P, M, W, J, dimg, g_rho, g_tf);
+                if (njobs) k_dm_adj_shadow<1><<<wave, 256, 0, s>>>(P, M, W, J, g_rho, g_tf);
+            } else {
+                k_dm_adj_primary<0><<<wave, 256, 0, s>>>(P, M, W, J, base, dimg, samples, g_rho, g_tf);
+                if (njobs) k_dm_adj_shadow<0><<<wave, 256, 0, s>>>(P, M, W, J, g_rho, g_tf);
+            }
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }

@@ -358,6 +358,26 @@ void to_plf(erd::Plf& o, const er_plf& s)
     o.range0 = s.node_range[0];
     o.range1 = s.node_range[1];
     for (int i = 0; i < 128; i++) { o.pos[i] = s.position[i]; o.val[i] = s.value[i]; }
+    /* the buckets of erd::plf_start: segment i = [pos[i-1], pos[i]) goes into
+       every bucket it meets, each bucket a hundredth wider on both sides than
+       the device's float bucket index can be off (some 1e-5 of a bucket) */
+    const int n = std::min(std::max(s.count, 0), ER_MAX_TF_NODES);
+    const double lo = s.node_range[0], width = (double)s.node_range[1] - lo;
+    const float scale = (float)(64.0 / width);
+    const bool usable = width > 0.0 && width < 1e37 && std::isfinite(scale) && std::isfinite(lo) && scale > 0.0f;
+    o.bucket_scale = usable ? scale : 0.0f;
+    for (int j = 0; j < 64; j++) o.first[j] = usable ? (uint8_t)n : (uint8_t)1;
+    if (!usable) return;
+    for (int i = n - 1; i >= 1; i--) {
+        const double a = ((double)s.position[i - 1] - lo) * scale - 0.01, b = ((double)s.position[i] - lo) * scale + 0.01;
+        if (!(a <= b) || !(b >= 0.0) || !(a < 64.01)) {
+            if (s.position[i - 1] < s.position[i] && !(b < 0.0) && !(a >= 64.01))
+                for (int j = 0; j < 64; j++) o.first[j] = (uint8_t)i;   /* not finite: looked at from everywhere */
+            continue;
+        }
+        const int j0 = a > 0.0 ? (int)std::min(a, 63.0) : 0, j1 = (int)std::min(b, 63.0);
+        for (int j = j0; j <= j1; j++) o.first[j] = (uint8_t)i;
+    }
 }
 
 /* Shape (Source/shape.h): transforms, type, sizes and the area */
@@ -1956,6 +1976,7 @@ static er_status medium_params(int32_t tracer_id, const er_medium_desc* m, erd::
     M.q = m->nee_probability;
     M.model = m->model;
     M.gm_inv = m->model == ER_MEDIUM_TRACER ? m->gradient_magnitude_inv : 0.0f;
+    M.gf3 = er_powf(ts.gradient_factor, 3.0f);
     M.emissive = 0;
     if (m->model == ER_MEDIUM_TRACER)
         for (int c = 0; c < 3; c++)
