@@ -71,6 +71,8 @@ struct Light {               /* ErLight + Shape (Source/erlight.h, Source/shape.
     float tex_rgb[3];
     float inner_c[3];        /* sphere lights with a rigid transform: the centre in world space and */
     float inner_r2;          /* (0.9 radius)^2 (< 0 otherwise): a segment with both ends inside cannot hit */
+    float ball_c[3];         /* planes, disks, rings and spheres with a rigid transform: a ball around the */
+    float ball_r2;           /* shape, (1.1 radius)^2 (< 0 otherwise): a line that misses it cannot hit */
 };
 
 struct Object {              /* ErObject (Source/erobject.h:27-67) */
@@ -109,6 +111,8 @@ struct Clip {                /* ErClippingObject (Source/erclippingobject.h:27-5
     int invert;
 };
 
+enum { QUADS_NONE = 0, QUADS_INDEX32 = 1, QUADS_INDEX64 = 2, QUADS_BRICKED = 3 };
+
 struct Params {
     /* volume (Source/volume.h:140-149) */
     const uint16_t* vox;
@@ -120,6 +124,10 @@ struct Params {
                                 pixels (1: 8x4, 2: 4x8, the default, 3: 16x2; films whose sides are
                                 multiples of the tile's), else (0) row by row */
     int res[3];
+    float resf[3];           /* (float)res */
+    int quad_mode;           /* how a lookup reads the corner quads: QUADS_* */
+    int index32;             /* fewer than 2^32 voxels (and so bricks): indices in 32 bits */
+    uint32_t slice32;        /* res[0] * res[1] then */
     float minp[3];
     float inv_size[3];
     float half_size[3];      /* BoundingBox.MaxP = 0.5 * Size */
@@ -133,6 +141,7 @@ struct Params {
     /* delta tracking: majorant per brick of `brick`^3 voxels */
     int free_flight;
     int brick;
+    float brickf;            /* (float)brick */
     int nb[3];
     const float* majorant;
     /* fixed-step march: per brick of 2^occ_shift voxels a side, 0 or the distance

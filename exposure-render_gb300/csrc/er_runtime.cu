@@ -107,17 +107,29 @@ constexpr size_t kWindowCap = (size_t)8 << 20;
 /* bricks of the march's empty-space map: 2^2 = 4 voxels a side */
 constexpr int kMarchBrickShift = 2;
 
-/* the persistent stages' refill threshold in eighths of a warp's tracking
-   lanes: 2, or ER_PT_REFILL (1..7) for measurements (with the empty-space
-   jump and tight bricks, C2 / C3 at 2, 3, 4, 5 eighths: 1336 / 2322, 1333 /
-   2266, 1317 / 2183, 1278 / 2051 Msamples/s) */
-int refill_eighths()
+/* the persistent stages' lanes (er_wavefront.cu): a warp's crossing ends when
+   5 eighths of its crossing lanes still cross (ER_PT_REFILL=0..7 for
+   measurements), its collisions when 7 eighths of the colliding ones still
+   collide; the primary stage sets rays up when the whole warp has ended (its
+   set-up and finish, some 1500 instructions, cost more than the lanes that
+   wait), the shadow stage when 14 lanes have.  Measured, ms:
+   - gates of 8, 16, 24 and 32 lanes, primary stage of the c2 shells 16.7,
+     13.1, 11.5, 9.4, of the c3 views 56.1, 48.9, 45.7, 43.9, of the c5 views
+     42.4, 35.6, 32.0, 28.1; 8, 12, 16 and 24 lanes, shadow stage of the c5
+     views 10.9, 10.6, 10.7, 11.2;
+   - crossing / collision eighths (6 c3 views with 8^3, 2^3 bricks; shadow
+     stage of c5): 3 / one pass 59.9, 17.8, 10.4; 7 / 7 56.7, 17.5, 11.6;
+     5 / 7 55.4, 17.3, 10.6; 5 / 5 60.6, 17.2, 10.8.  Large bricks hold many
+     collisions each, so a warp that waits for its last colliding lanes is
+     the worse there. */
+constexpr int kGatePrimary = 32, kGateShadow = 14, kCollideEighths = 7;
+int cross_eighths()
 {
-    static int v = 0;
-    if (!v) {
+    static int v = -1;
+    if (v < 0) {
         const char* e = getenv("ER_PT_REFILL");
-        const int r = e ? atoi(e) : 2;
-        v = (r >= 1 && r <= 7) ? r : 2;
+        const int r = e ? atoi(e) : 5;
+        v = (r >= 0 && r <= 7) ? r : 5;
     }
     return v;
 }
@@ -155,7 +167,10 @@ struct WfQueues {
         B.partial = partial.p;
         B.records = nullptr;
         B.sort_shade = 0;
-        B.refill_eighths = refill_eighths();
+        B.cross_eighths = cross_eighths();
+        B.collide_eighths = kCollideEighths;
+        B.gate_primary = kGatePrimary;
+        B.gate_shadow = kGateShadow;
         B.counters = counters.p;
         B.tune_primary = 4;
         B.tune_shadow = 4;
@@ -393,6 +408,34 @@ void to_shape(erd::Light& o, const er_shape& sh)
     o.outer_radius = sh.outer_radius;
 }
 
+/* the balls of shape_missed (er_path.cuh): the exact test maps the ray with
+   InvTM, so the shape is centred where InvTM = (R, t) sends a point to the
+   origin, c = -R^T t for a rigid one */
+void shape_balls(erd::Light& l)
+{
+    l.inner_r2 = l.ball_r2 = -1.0f;
+    double radius = -1.0;
+    switch (l.type) {
+    case ER_SHAPE_PLANE: radius = 0.5 * std::sqrt((double)l.size[0] * l.size[0] + (double)l.size[1] * l.size[1]); break;
+    case ER_SHAPE_DISK: case ER_SHAPE_RING: case ER_SHAPE_SPHERE: radius = l.outer_radius; break;
+    default: return;
+    }
+    if (!(radius > 0.0) || !std::isfinite(radius)) return;
+    for (int r = 0; r < 3; r++)
+        for (int c = 0; c < 3; c++) {
+            double d = 0.0;
+            for (int k = 0; k < 3; k++) d += (double)l.inv_tm[k][r] * (double)l.inv_tm[k][c];
+            if (!(std::fabs(d - (r == c ? 1.0 : 0.0)) <= 1e-5)) return;
+        }
+    for (int k = 0; k < 3; k++) {
+        double c = 0.0;
+        for (int r = 0; r < 3; r++) c -= (double)l.inv_tm[r][k] * (double)l.inv_tm[r][3];
+        l.ball_c[k] = l.inner_c[k] = (float)c;
+    }
+    l.ball_r2 = (float)(1.21 * radius * radius + 1e-5);
+    if (l.type == ER_SHAPE_SPHERE) l.inner_r2 = (float)(0.81 * radius * radius);
+}
+
 void to_light(erd::Light& o, const er_light_desc& s)
 {
     to_shape(o, s.shape);
@@ -432,12 +475,16 @@ void volume_geometry(const VolumeItem& v, erd::Params& P)
     for (int i = 0; i < 3; i++) size[i] = (float)v.res[i] * sp[i];
     for (int i = 0; i < 3; i++) {
         P.res[i] = v.res[i];
+        P.resf[i] = (float)v.res[i];
         P.spacing[i] = sp[i];
         P.inv_size[i] = 1.0f / size[i];
         P.minp[i] = size[i] * -0.5f;
         P.half_size[i] = size[i] * 0.5f;
     }
+    P.index32 = (unsigned long long)v.res[0] * v.res[1] * v.res[2] < (1ull << 32) ? 1 : 0;
+    P.slice32 = (uint32_t)v.res[0] * (uint32_t)v.res[1];
     P.min_step = smin_h(sp[0], smin_h(sp[1], sp[2]));
+    P.quad_mode = !v.quad.p ? erd::QUADS_NONE : (v.qb_nbx > 0 ? erd::QUADS_BRICKED : (P.index32 ? erd::QUADS_INDEX32 : erd::QUADS_INDEX64));
     P.vox = v.vox.p;
     P.quad = v.quad.p;
     P.qb_nbx = v.qb_nbx;
@@ -614,6 +661,7 @@ er_status build(TracerItem& t)
         ER_CUDA(t.skip_tmp.ensure(2 * total));
         ER_CUDA(er_launch_empty_skip(t.majorant.p, nb, t.skip_tmp.p, st));
         P.brick = brick;
+        P.brickf = (float)brick;
         for (int i = 0; i < 3; i++) P.nb[i] = nb[i];
         P.majorant = t.majorant.p;
     } else if (v.normalize) {
@@ -644,30 +692,9 @@ er_status build(TracerItem& t)
         to_light(L[i], *it->second);
         valid[i] = 1;
     }
-    /* sphere lights with a rigid transform: the inner ball of the shadow
-       rays' occlusion early-out (intersects_light) */
-    for (int i = 0; i < lc; i++) {
-        erd::Light& l = L[i];
-        l.inner_r2 = -1.0f;
-        if (!valid[i] || l.type != ER_SHAPE_SPHERE || !(l.outer_radius > 0.0f)) continue;
-        /* the exact test maps the ray with InvTM: the sphere is centred where
-           InvTM sends a point to the origin, c = -R^T t for InvTM = (R, t) */
-        bool rigid = true;
-        for (int r = 0; r < 3; r++)
-            for (int c = 0; c < 3; c++) {
-                double d = 0.0;
-                for (int k = 0; k < 3; k++) d += (double)l.inv_tm[k][r] * (double)l.inv_tm[k][c];
-                if (std::fabs(d - (r == c ? 1.0 : 0.0)) > 1e-5) rigid = false;
-            }
-        if (!rigid) continue;
-        for (int k = 0; k < 3; k++) {
-            double c = 0.0;
-            for (int r = 0; r < 3; r++) c -= (double)l.inv_tm[r][k] * (double)l.inv_tm[r][3];
-            l.inner_c[k] = (float)c;
-        }
-        const double ri = 0.9 * (double)l.outer_radius;
-        l.inner_r2 = (float)(ri * ri);
-    }
+    for (int i = 0; i < lc; i++)
+        if (valid[i]) shape_balls(L[i]);
+        else L[i].inner_r2 = L[i].ball_r2 = -1.0f;
     /* lights whose texture is uniform (or unbound: black) get its value here,
        as EvaluateTexture computes it: colour * OutputLevel in float
        (Source/textures.h:63-111) */
@@ -709,6 +736,7 @@ er_status build(TracerItem& t)
         erd::Object o;
         memset(&o, 0, sizeof(o));
         to_shape(o.shape, kv.second->shape);
+        shape_balls(o.shape);
         o.diffuse_texture_id = kv.second->diffuse_texture_id;
         o.specular_texture_id = kv.second->specular_texture_id;
         o.glossiness_texture_id = kv.second->glossiness_texture_id;
@@ -1966,6 +1994,7 @@ static er_status medium_params(int32_t tracer_id, const er_medium_desc* m, erd::
     if (st != ER_OK) return st;
     P = t->P;
     P.brick = m->brick;
+    P.brickf = (float)m->brick;
     for (int i = 0; i < 3; i++) P.nb[i] = (P.res[i] + m->brick - 1) / m->brick;
     P.majorant = m->d_majorant;
     M.rho = m->d_density;

@@ -145,10 +145,10 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary(const WfView* __restri
             se1 = se0; se1.type = 1;
             /* the event normal (no RNG) is computed by the shade stage */
             if (FF == WF_DELTA || (FF == WF_MIXED && P.free_flight == 1)) sample_volume_delta<false>(P, R, rng, se0, ms.tau_u);
-            else sample_volume<false>(P, R, rng, se0);
+            else sample_volume<false, ER_K_PRIMARY>(P, R, rng, se0);
             int lslot = -1;
             LightHit lh;
-            intersect_lights_geom(P, R, se1, true, lslot, lh);
+            intersect_lights_geom(P, R, se1, true, lslot, lh, se0.valid ? event_end(se0.T) : FLT_MAX);
             SE = se0; SE.valid = false; SE.type = 0;
             float T = FLT_MAX;
             if (se0.valid && se0.T < T) { SE = se0; T = se0.T; }
@@ -188,150 +188,170 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary(const WfView* __restri
     }
 }
 
-/* persistent stages: a warp stops tracking to refill when fewer than
-   refill / 8 of the lanes that were tracking still are (a launch argument,
-   WavefrontBuffers::refill_eighths, 2 by default; measured in er_runtime.cu
-   refill_eighths) */
+/* Persistent lanes (delta tracking).  A warp alternates between three parts,
+   each made by as many of its lanes together as can be had:
+     crossing : lanes cross majorant bricks until cross / 8 of those that
+                were crossing still do;
+     collision: the lanes that are at a tentative collision look it up, and
+                go on to the brick's next one, until collide / 8 are left;
+     set-up   : when `gate` lanes have ended their rays (or no lane tracks),
+                those lanes finish their samples, take the window's next items
+                (consecutive ones, one atomic per warp) and set their rays up,
+                while the others keep theirs.
+   Each part is some 60 to 600 instructions long, so what bounds the stage is
+   the lanes that run them (with one loop of steps, in which colliding and
+   crossing lanes took turns, and each ended lane's set-up on its own, 7 to 8
+   lanes of the shadow stage were active and 17 of the primary stage). */
+ER_D bool few_left(unsigned m, int start, int cross) { return 8 * __popc(m) <= cross * start; }
 
-/* queue slot among the lanes that are here together (persistent stages,
-   where lanes reach their queue pushes at different loop trips) */
-ER_D uint32_t queue_slot_active(bool want, uint32_t* counter)
+ER_D uint32_t take_items(unsigned needy, uint32_t* fetch)
 {
-    const unsigned active = __activemask();
-    const unsigned mask = __ballot_sync(active, want);
     const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
+    const int leader = __ffs(needy) - 1;
     uint32_t base = 0;
-    if (mask && lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask));
-    base = __shfl_sync(active, base, leader < 0 ? (__ffs(active) - 1) : leader);
-    return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+    if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(needy));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    return base + (uint32_t)__popc(needy & ((1u << lane) - 1u));
 }
 
-/* ---- stage 1, persistent lanes (delta tracking) ----
+/* ---- stage 1, persistent lanes ----
 
-   The work of k_wf_primary with lanes tracking one tentative collision or
-   majorant brick per inner loop trip: when most of a warp's tracking lanes
-   have ended their rays, the warp finishes those samples and gives the
-   lanes the next items of the window (consecutive ones, one atomic per
-   warp), while the other lanes keep their rays.  The MetroSample values an event
-   record carries are drawn again from the sample's seed when the sample
-   finishes instead of being held through the tracking. */
+   The MetroSample values an event record carries are drawn again from the
+   sample's seed when the sample finishes instead of being held through the
+   tracking. */
 template <int MINB, bool ONE, bool OBJ>
 __global__ void __launch_bounds__(256, MINB) k_wf_primary_pt(const WfView* __restrict__ views, const WfSegment* __restrict__ segs,
                                                               int nseg, const WfView one, const WfSegment one_seg, uint32_t items,
                                                               float4* __restrict__ results, float4* __restrict__ events,
-                                                              uint32_t* __restrict__ n_events, uint32_t* __restrict__ fetch, int refill)
+                                                              uint32_t* __restrict__ n_events, uint32_t* __restrict__ fetch, int cross,
+                                                              int collide, int gate)
 {
-    const int lane = threadIdx.x & 31;
     uint32_t i = 0;
-    bool tracking = false, exhausted = false;
+    /* at: the ray is at a tentative collision; hit: at a real one */
+    bool have = false, exhausted = false, hit = false, at = false;
     int seg = 0;
     Rng rng;
     rng.s0 = 0u;
     rng.s1 = 0u;
     Ray R;
-    DeltaTracker k;
+    Tracker k;
     k.done = true;
-    k.hit = false;
     for (;;) {
-        /* lanes without a sample take the next items of the window together
-           (one atomic per warp), so a warp's new samples are neighbours */
-        const unsigned needy = __ballot_sync(0xffffffffu, !tracking && !exhausted);
-        if (needy) {
-            const int leader = __ffs(needy) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(needy));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (!tracking && !exhausted) {
-                i = base + (uint32_t)__popc(needy & ((1u << lane) - 1u));
-                exhausted = i >= items;
+        const unsigned idle = __ballot_sync(0xffffffffu, have ? k.done : !exhausted);
+        const unsigned busy = __ballot_sync(0xffffffffu, have && !k.done);
+        if (!(idle | busy)) break;
+        if (!busy || __popc(idle) >= gate) {
+            bool push = false;
+            Event SE;
+            WfSegment sg = one_seg;
+            if (have && k.done) {
+                /* the sample's nearest event: volume, visible lights, objects */
+                if (!ONE) sg = segs[seg];
+                const Params& P = view_of<ONE>(views, one, sg.view).P;
+                Event se1;
+                SE.type = 0; SE.valid = false; SE.T = 0.0f; SE.Le = C3(0, 0, 0);
+                SE.P = V3(0, 0, 0); SE.N = V3(0, 0, 0); SE.Wo = V3(0, 0, 0);
+                se1 = SE; se1.type = 1;
+                if (hit) {
+                    SE.valid = true;
+                    SE.T = k.t;
+                    SE.P = vadd(R.O, vscale(R.D, k.t));
+                    SE.N = V3(0.0f, 0.0f, 0.0f);
+                    SE.Wo = vneg(R.D);
+                }
+                const Event se0 = SE;
+                int lslot = -1;
+                LightHit lh;
+                intersect_lights_geom(P, R, se1, true, lslot, lh, se0.valid ? event_end(se0.T) : FLT_MAX);
+                SE.valid = false; SE.type = 0;
+                float T = FLT_MAX;
+                if (se0.valid && se0.T < T) { SE = se0; T = se0.T; }
+                if (se1.valid && se1.T < T) { SE = se1; T = se1.T; }
+                ObjHit ohit;
+                if (OBJ && P.object_count > 0) {
+                    Event se2;
+                    se2.type = 2; se2.valid = false; se2.T = 0.0f;
+                    intersect_objects(P, R, se2, ohit);
+                    if (se2.valid && se2.T < T) { SE = se2; T = se2.T; }
+                }
+                if (SE.valid && SE.type == 1) SE.Le = light_emission(P, P.lights[lslot], lh);
+                if (!SE.valid) {
+                    results[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                } else if (SE.type == 1) {
+                    const c3 Lv = cadd(C3(0, 0, 0), SE.Le);
+                    results[i] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
+                } else {
+                    push = true;
+                    if (OBJ && SE.type == 2) results[i] = make_float4(ohit.UV.x, ohit.UV.y, u2f((uint32_t)ohit.id), 0.0f);
+                }
+                have = false;
+            }
+            __syncwarp();
+            const uint32_t slot = queue_slot(push, n_events);
+            if (push) {
+                const WfView& V = view_of<ONE>(views, one, sg.view);
+                const Params& P = V.P;
+                const uint32_t local = i - sg.offset;
+                const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
+                Rng r0;
+                const uint32_t sidx = V.first + (uint32_t)(sg.s0 + (int)(local / npix));
+                const uint32_t pix = slot_pixel(P, local % npix);
+                er_seed_lanes(P.seed, V.view_id, pix, sidx, &r0.s0, &r0.s1);
+                Metro ms;
+                ms.large_step(r0);
+                ms.stratify(P, V.view_id, pix, sidx);
+                const bool obj = OBJ && SE.type == 2;
+                float4* e = events + (size_t)slot * 5;
+                e[0] = make_float4(u2f(i), u2f(rng.s0), u2f(rng.s1), ms.light_num);
+                e[1] = make_float4(SE.P.x, SE.P.y, SE.P.z, ms.brdf_component);
+                e[2] = obj ? make_float4(SE.N.x, SE.N.y, SE.N.z, ms.brdf_dir.x) : make_float4(0.0f, 0.0f, 0.0f, ms.brdf_dir.x);
+                e[3] = make_float4(SE.Wo.x, SE.Wo.y, SE.Wo.z, ms.brdf_dir.y);
+                e[4] = make_float4(ms.light_uvw.x, ms.light_uvw.y, ms.light_uvw.z, u2f((uint32_t)sg.view | (obj ? WF_OBJECT_EVENT : 0u)));
+            }
+            __syncwarp();
+            const unsigned needy = __ballot_sync(0xffffffffu, !have && !exhausted);
+            if (needy) {
+                const uint32_t next = take_items(needy, fetch);
+                if (!have && !exhausted) {
+                    i = next;
+                    exhausted = i >= items;
+                    if (!exhausted) {
+                        seg = ONE ? 0 : find_segment(segs, nseg, i);
+                        if (!ONE) sg = segs[seg];
+                        const WfView& V = view_of<ONE>(views, one, sg.view);
+                        const Params& P = V.P;
+                        const uint32_t local = i - sg.offset;
+                        const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
+                        const int s = sg.s0 + (int)(local / npix);
+                        const int pix = (int)slot_pixel(P, local % npix);
+                        er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, V.first + (uint32_t)s, &rng.s0, &rng.s1);
+                        Metro ms;
+                        ms.large_step(rng);
+                        ms.stratify(P, V.view_id, (uint32_t)pix, V.first + (uint32_t)s);
+                        R = sample_camera(P, pix % P.film[0], pix / P.film[0], ms.film_uv, ms.lens_uv);
+                        delta_begin(P, R, rng, k, ms.tau_u);
+                        hit = false;
+                        have = true;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        const Params& P = view_of<ONE>(views, one, ONE ? 0 : segs[seg].view).P;
+        int start = __popc(__ballot_sync(0xffffffffu, have && !k.done && !at));
+        for (;;) {
+            const bool crossing = have && !k.done && !at;
+            if (few_left(__ballot_sync(0xffffffffu, crossing), start, cross)) break;
+            if (crossing) at = track_cross(P, k);
+        }
+        start = __popc(__ballot_sync(0xffffffffu, at));
+        for (;;) {
+            if (few_left(__ballot_sync(0xffffffffu, at), start, collide)) break;
+            if (at) {
+                hit = delta_collide(P, R, rng, k);
+                at = !k.done && track_again(k);
             }
         }
-        if (!tracking && !exhausted) {
-            seg = ONE ? 0 : find_segment(segs, nseg, i);
-            const WfSegment sg = ONE ? one_seg : segs[seg];
-            const WfView& V = view_of<ONE>(views, one, sg.view);
-            const Params& P = V.P;
-            const uint32_t local = i - sg.offset;
-            const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
-            const int s = sg.s0 + (int)(local / npix);
-            const int pix = (int)slot_pixel(P, local % npix);
-            er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, V.first + (uint32_t)s, &rng.s0, &rng.s1);
-            Metro ms;
-            ms.large_step(rng);
-            ms.stratify(P, V.view_id, (uint32_t)pix, V.first + (uint32_t)s);
-            R = sample_camera(P, pix % P.film[0], pix / P.film[0], ms.film_uv, ms.lens_uv);
-            delta_begin(P, R, rng, k, ms.tau_u);
-            tracking = true;
-        }
-        if (!__any_sync(0xffffffffu, tracking)) break;
-        const WfSegment sg = ONE ? one_seg : segs[seg];
-        const WfView& V = view_of<ONE>(views, one, sg.view);
-        const Params& P = V.P;
-        /* track until most of the lanes that were tracking have ended */
-        const int n_work = __popc(__ballot_sync(0xffffffffu, tracking && !k.done));
-        while (tracking && !k.done) {
-            delta_step(P, R, rng, k);
-            if (k.done || 8 * __popc(__activemask()) < refill * n_work) break;
-        }
-        if (!tracking || !k.done) continue;
-        /* the sample's nearest event: volume, visible lights, objects */
-        Event SE, se1;
-        SE.type = 0; SE.valid = false; SE.T = 0.0f; SE.Le = C3(0, 0, 0);
-        SE.P = V3(0, 0, 0); SE.N = V3(0, 0, 0); SE.Wo = V3(0, 0, 0);
-        se1 = SE; se1.type = 1;
-        if (k.hit) {
-            SE.valid = true;
-            SE.T = k.t;
-            SE.P = vadd(R.O, vscale(R.D, k.t));
-            SE.N = V3(0.0f, 0.0f, 0.0f);
-            SE.Wo = vneg(R.D);
-        }
-        const Event se0 = SE;
-        int lslot = -1;
-        LightHit lh;
-        intersect_lights_geom(P, R, se1, true, lslot, lh);
-        SE.valid = false; SE.type = 0;
-        float T = FLT_MAX;
-        if (se0.valid && se0.T < T) { SE = se0; T = se0.T; }
-        if (se1.valid && se1.T < T) { SE = se1; T = se1.T; }
-        ObjHit hit;
-        if (OBJ && P.object_count > 0) {
-            Event se2;
-            se2.type = 2; se2.valid = false; se2.T = 0.0f;
-            intersect_objects(P, R, se2, hit);
-            if (se2.valid && se2.T < T) { SE = se2; T = se2.T; }
-        }
-        if (SE.valid && SE.type == 1) SE.Le = light_emission(P, P.lights[lslot], lh);
-        bool push = false;
-        if (!SE.valid) {
-            results[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else if (SE.type == 1) {
-            const c3 Lv = cadd(C3(0, 0, 0), SE.Le);
-            results[i] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
-        } else {
-            push = true;
-            if (OBJ && SE.type == 2) results[i] = make_float4(hit.UV.x, hit.UV.y, u2f((uint32_t)hit.id), 0.0f);
-        }
-        const uint32_t slot = queue_slot_active(push, n_events);
-        if (push) {
-            const uint32_t local = i - sg.offset;
-            const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
-            Rng r0;
-            const uint32_t sidx = V.first + (uint32_t)(sg.s0 + (int)(local / npix));
-            er_seed_lanes(P.seed, V.view_id, slot_pixel(P, local % npix), sidx, &r0.s0, &r0.s1);
-            Metro ms;
-            ms.large_step(r0);
-            ms.stratify(P, V.view_id, slot_pixel(P, local % npix), sidx);
-            const bool obj = OBJ && SE.type == 2;
-            float4* e = events + (size_t)slot * 5;
-            e[0] = make_float4(u2f(i), u2f(rng.s0), u2f(rng.s1), ms.light_num);
-            e[1] = make_float4(SE.P.x, SE.P.y, SE.P.z, ms.brdf_component);
-            e[2] = obj ? make_float4(SE.N.x, SE.N.y, SE.N.z, ms.brdf_dir.x) : make_float4(0.0f, 0.0f, 0.0f, ms.brdf_dir.x);
-            e[3] = make_float4(SE.Wo.x, SE.Wo.y, SE.Wo.z, ms.brdf_dir.y);
-            e[4] = make_float4(ms.light_uvw.x, ms.light_uvw.y, ms.light_uvw.z, u2f((uint32_t)sg.view | (obj ? WF_OBJECT_EVENT : 0u)));
-        }
-        tracking = false;
     }
 }
 
@@ -460,7 +480,7 @@ __global__ void __launch_bounds__(128, MINB) k_wf_shade(const WfView* __restrict
                         SE2.P = V3(0, 0, 0); SE2.N = V3(0, 0, 0); SE2.Wo = V3(0, 0, 0);
                         int hit = -1;
                         LightHit lh;
-                        intersect_lights_geom(P, R2, SE2, false, hit, lh);
+                        intersect_lights_geom<false>(P, R2, SE2, false, hit, lh);
                         if (SE2.valid && P.light_ids[hit] == P.light_ids[idx]) SE2.Le = light_emission(P, P.lights[hit], lh);
                         if (SE2.valid && P.light_ids[hit] == P.light_ids[idx] && !cblack(SE2.Le)) {
                             const float LightPdf = vlen2(vsub(SE.P, SE2.P)) / (vabsdot(SE2.N, vneg(Wb)) * L.area);
@@ -666,7 +686,7 @@ __global__ void __launch_bounds__(128, MINB) k_wf_shade_sorted(const WfView* __r
                         SE2.P = V3(0, 0, 0); SE2.N = V3(0, 0, 0); SE2.Wo = V3(0, 0, 0);
                         int hit = -1;
                         LightHit lh;
-                        intersect_lights_geom(P, R2, SE2, false, hit, lh);
+                        intersect_lights_geom<false>(P, R2, SE2, false, hit, lh);
                         if (SE2.valid && P.light_ids[hit] == P.light_ids[idx]) SE2.Le = light_emission(P, P.lights[hit], lh);
                         if (SE2.valid && P.light_ids[hit] == P.light_ids[idx] && !cblack(SE2.Le)) {
                             const float LightPdf = vlen2(vsub(SE.P, SE2.P)) / (vabsdot(SE2.N, vneg(Wb)) * L.area);
@@ -721,14 +741,14 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow(const WfView* __restric
         const c3 Le = C3(j2.w, j3.w, j4.w);
         c3 dl = C3(0, 0, 0);
         if (flags & WF_RAY1) {
-            const float Tr = visibility<OBJ, FF>(P, Pp, V3(j2.x, j2.y, j2.z), rng);
+            const float Tr = visibility<OBJ, FF, ER_K_SHADOW>(P, Pp, V3(j2.x, j2.y, j2.z), rng);
             if (Tr > 0.0f) {
                 const c3 c1 = C3(j3.x, j3.y, j3.z);
                 dl = ref_mode ? cadd(dl, c1) : cadd(dl, cscale(c1, Tr));
             }
         }
         if (flags & WF_RAY2) {
-            const float Tr = visibility<OBJ, FF>(P, Pp, V3(j4.x, j4.y, j4.z), rng);
+            const float Tr = visibility<OBJ, FF, ER_K_SHADOW>(P, Pp, V3(j4.x, j4.y, j4.z), rng);
             if (Tr > 0.0f) dl = cadd(dl, cscale(C3(j5.x, j5.y, j5.z), Tr));
         }
         const c3 Lv = cadd(C3(0, 0, 0), cscale(cadd(Le, dl), count));
@@ -738,23 +758,19 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow(const WfView* __restric
 
 /* ---- stage 3, persistent lanes (delta tracking: ratio-tracked shadows) ----
 
-   The same jobs and arithmetic as k_wf_shadow, with the work split
-   differently: lanes track one collision or majorant brick per inner loop
-   trip; when most of a warp's tracking lanes have ended their segments,
-   the warp starts their next segments or takes new jobs (consecutive ones,
-   one atomic per warp) and tracks on.  In k_wf_shadow a warp runs until its
-   longest segment ends while the other lanes idle (5.5 of 32 lanes active
-   per instruction on the c2 workload). */
+   The same jobs and arithmetic as k_wf_shadow.  A lane tracks its job's
+   segments one after the other (the second continues the first one's random
+   stream); both are set up in the warp's common set-up part. */
 template <int MINB, bool ONE, bool OBJ>
 __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __restrict__ views, const WfView one,
                                                              const float4* __restrict__ jobs, const uint32_t* __restrict__ n_jobs,
-                                                             float4* __restrict__ results, uint32_t* __restrict__ fetch, int refill)
+                                                             float4* __restrict__ results, uint32_t* __restrict__ fetch, int cross,
+                                                             int collide, int gate)
 {
     const uint32_t n = *n_jobs;
-    const int lane = threadIdx.x & 31;
     uint32_t j_i = 0;
-    bool exhausted = false;
-    /* phase 0: take a job; 1, 2: tracking shadow segment 1 or 2; 3: write the sample */
+    bool exhausted = false, at = false;
+    /* phase 0: no job; 1, 2: shadow segment 1 or 2 */
     int phase = 0;
     uint32_t flags = 0, v = 0;
     Rng rng;
@@ -762,81 +778,82 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __rest
     rng.s1 = 0u;
     c3 dl = C3(0, 0, 0);
     Ray R;
-    RatioTracker k;
+    Tracker k;
+    float Tr = 1.0f;
     k.done = true;
-    k.Tr = 1.0f;
     for (;;) {
-        /* lanes without a job take the next jobs together (one atomic per warp) */
-        const unsigned needy = __ballot_sync(0xffffffffu, phase == 0 && !exhausted);
-        if (needy) {
-            const int leader = __ffs(needy) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(needy));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (phase == 0 && !exhausted) {
-                j_i = base + (uint32_t)__popc(needy & ((1u << lane) - 1u));
-                exhausted = j_i >= n;
+        const unsigned idle = __ballot_sync(0xffffffffu, phase ? k.done : !exhausted);
+        const unsigned busy = __ballot_sync(0xffffffffu, phase && !k.done);
+        if (!(idle | busy)) break;
+        if (!busy || __popc(idle) >= gate) {
+            bool set_up = false;
+            if (phase && k.done) {
+                const float4* j = jobs + (size_t)j_i * 6;
+                if (Tr > 0.0f) {
+                    const float4 c = j[phase == 1 ? 3 : 5];
+                    dl = cadd(dl, cscale(C3(c.x, c.y, c.z), Tr));
+                }
+                if (phase == 1 && (flags & WF_RAY2)) {
+                    phase = 2;
+                    set_up = true;
+                } else {
+                    const float4 j0 = j[0], j1 = j[1], j2 = j[2], j3 = j[3], j4 = j[4];
+                    const c3 Le = C3(j2.w, j3.w, j4.w);
+                    const c3 Lv = cadd(C3(0, 0, 0), cscale(cadd(Le, dl), j1.w));
+                    results[f2u(j0.x)] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
+                    phase = 0;
+                }
             }
-        }
-        if (phase == 0 && !exhausted) {
-            const float4* j = jobs + (size_t)j_i * 6;
-            const float4 j0 = j[0];
-            rng.s0 = f2u(j0.y);
-            rng.s1 = f2u(j0.z);
-            flags = f2u(j0.w);
-            v = f2u(j[5].w);
-            dl = C3(0, 0, 0);
-            phase = (flags & WF_RAY1) ? 1 : ((flags & WF_RAY2) ? 2 : 3);
-            if (phase != 3) {
+            __syncwarp();
+            const unsigned needy = __ballot_sync(0xffffffffu, !phase && !exhausted);
+            if (needy) {
+                const uint32_t next = take_items(needy, fetch);
+                if (!phase && !exhausted) {
+                    j_i = next;
+                    exhausted = j_i >= n;
+                    if (!exhausted) {
+                        const float4* j = jobs + (size_t)j_i * 6;
+                        const float4 j0 = j[0];
+                        rng.s0 = f2u(j0.y);
+                        rng.s1 = f2u(j0.z);
+                        flags = f2u(j0.w);
+                        v = f2u(j[5].w);
+                        dl = C3(0, 0, 0);
+                        phase = (flags & WF_RAY1) ? 1 : 2;     /* a job has a segment */
+                        set_up = true;
+                    }
+                }
+            }
+            __syncwarp();
+            if (set_up) {
                 /* Visible (Source/transport.h:46-56) up to the tracking */
                 const Params& P = view_of<ONE>(views, one, v).P;
+                const float4* j = jobs + (size_t)j_i * 6;
                 const float4 j1 = j[1], js = j[phase == 1 ? 2 : 4];
                 k.done = true;
-                k.Tr = 1.0f;
+                Tr = 1.0f;
                 if (P.shadows) {
                     R = shadow_ray(P, V3(j1.x, j1.y, j1.z), V3(js.x, js.y, js.z));
-                    if (intersects_light(P, R) || (OBJ && P.object_count > 0 && intersects_object(P, R))) k.Tr = 0.0f;
+                    if (intersects_light(P, R) || (OBJ && P.object_count > 0 && intersects_object(P, R))) Tr = 0.0f;
                     else ratio_begin(P, R, rng, k);
                 }
             }
+            __syncwarp();
         }
-        if (!__any_sync(0xffffffffu, phase != 0)) break;
-        const bool seg_phase = phase == 1 || phase == 2;
         const Params& P = view_of<ONE>(views, one, v).P;
-        /* track until most of the lanes that were tracking have ended */
-        const int n_work = __popc(__ballot_sync(0xffffffffu, seg_phase && !k.done));
-        while (seg_phase && !k.done) {
-            ratio_step(P, R, rng, k);
-            if (k.done || 8 * __popc(__activemask()) < refill * n_work) break;
+        int start = __popc(__ballot_sync(0xffffffffu, phase && !k.done && !at));
+        for (;;) {
+            const bool crossing = phase && !k.done && !at;
+            if (few_left(__ballot_sync(0xffffffffu, crossing), start, cross)) break;
+            if (crossing) at = track_cross(P, k);
         }
-        if (seg_phase && k.done) {
-            const float4* j = jobs + (size_t)j_i * 6;
-            const float Tr = k.Tr;
-            if (Tr > 0.0f) {
-                const float4 c = j[phase == 1 ? 3 : 5];
-                dl = cadd(dl, cscale(C3(c.x, c.y, c.z), Tr));
+        start = __popc(__ballot_sync(0xffffffffu, at));
+        for (;;) {
+            if (few_left(__ballot_sync(0xffffffffu, at), start, collide)) break;
+            if (at) {
+                ratio_collide(P, R, rng, k, Tr);
+                at = !k.done && track_again(k);
             }
-            if (phase == 1 && (flags & WF_RAY2)) {
-                phase = 2;
-                const float4 j1 = j[1], js = j[4];
-                k.done = true;
-                k.Tr = 1.0f;
-                if (P.shadows) {
-                    R = shadow_ray(P, V3(j1.x, j1.y, j1.z), V3(js.x, js.y, js.z));
-                    if (intersects_light(P, R) || (OBJ && P.object_count > 0 && intersects_object(P, R))) k.Tr = 0.0f;
-                    else ratio_begin(P, R, rng, k);
-                }
-            } else {
-                phase = 3;
-            }
-        }
-        if (phase == 3) {
-            const float4* j = jobs + (size_t)j_i * 6;
-            const float4 j0 = j[0], j1 = j[1], j2 = j[2], j3 = j[3], j4 = j[4];
-            const c3 Le = C3(j2.w, j3.w, j4.w);
-            const c3 Lv = cadd(C3(0, 0, 0), cscale(cadd(Le, dl), j1.w));
-            results[f2u(j0.x)] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
-            phase = 0;
         }
     }
 }
@@ -1003,7 +1020,7 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         const uint32_t g1 = (items + 255) / 256 < (uint32_t)sm * 64 ? (items + 255) / 256 : (uint32_t)sm * 64;
         cudaEvent_t t0 = stage_begin(s);
 #define ER_PRIMARY(M, O, F) k_wf_primary<M, ONE, O, F><<<g1, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters)
-#define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2, B.refill_eighths)
+#define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2, B.cross_eighths, B.collide_eighths, B.gate_primary)
         if (B.pt_primary) {
             /* delta tracking: persistent lanes, one resident wave */
             if (B.objects) ER_PRIMARY_PT(4, true);
@@ -1064,7 +1081,7 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         stage_end(t0, 1, s);
         t0 = stage_begin(s);
 #define ER_SHADOW(M, O, F) k_wf_shadow<M, ONE, O, F><<<sm * 8, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results)
-#define ER_SHADOW_PT(M, O) k_wf_shadow_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.refill_eighths)
+#define ER_SHADOW_PT(M, O) k_wf_shadow_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.cross_eighths, B.collide_eighths, B.gate_shadow)
         if (B.pt_shadow) {
             /* ratio-tracked shadows: persistent lanes, one resident wave */
             if (B.objects) ER_SHADOW_PT(4, true);
