@@ -32,6 +32,7 @@ UNITS = {
     "er_post.cu": ["--fmad=false"],
     "er_volume.cu": ["--fmad=false"],
     "er_wavefront.cu": ["--fmad=false", "-Xptxas", "-v"],
+    "er_wavefront_batch.cu": ["--fmad=false", "-Xptxas", "-v"],
     "er_medium.cu": ["--fmad=false", "-Xptxas", "-v"],
     "er_runtime.cu": [],
     "er_cxx_api.cpp": [],
@@ -64,6 +65,7 @@ def _stale(obj: str, deps: list[str]) -> bool:
 def build(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OUT, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
+    headers.append(os.path.join(CSRC, "er_wavefront.cu"))      # er_wavefront_batch.cu includes it
     headers += [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))]
     jobs = {}
     with cf.ThreadPoolExecutor(max_workers=len(UNITS)) as ex:

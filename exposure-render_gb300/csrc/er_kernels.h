@@ -20,6 +20,8 @@ struct BilateralTables {
     float range[256];
 };
 
+/* er_seed_lanes(seed, 0, pixel, 0xffffffff) of n pixels: lane 0 block, lane 1 block */
+cudaError_t er_launch_init_lanes(uint32_t seed, uint32_t* lanes, uint32_t n, cudaStream_t s);
 cudaError_t er_launch_trace_frame(const erd::Params& P, uint32_t* lanes, float4* frame, cudaStream_t s);
 cudaError_t er_launch_trace_sum(const erd::Params& P, int spp, uint32_t view, uint32_t first, float4* sum, int accumulate,
                                 cudaStream_t s);
@@ -37,6 +39,13 @@ cudaError_t er_launch_tonemap(const float4* xyza, float scale, uchar4* rgba, int
 cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int W, int H, const BilateralTables& T,
                                 cudaStream_t s);
 cudaError_t er_launch_gradient_magnitude(const erd::Params& P, uint16_t* gm, unsigned int* max_bits, cudaStream_t s);
+/* the largest gradient magnitude alone (as er_launch_gradient_magnitude);
+   scratch: 3 words per 8^3 brick and 2 more; max_bits zero before */
+cudaError_t er_launch_gradient_max(const erd::Params& P, uint32_t* scratch, unsigned int* max_bits, cudaStream_t s);
+/* lo | hi << 16 of every B^3 brick's footprint, voxels b B .. (b + 1) B per axis (er_volume.cu) */
+cudaError_t er_launch_brick_minmax(const uint16_t* vox, const int res[3], int B, const int nb[3], uint32_t* minmax, cudaStream_t s);
+/* every step-th of n voxels into out */
+cudaError_t er_launch_sample_voxels(const uint16_t* vox, size_t n, int step, uint16_t* out, cudaStream_t s);
 cudaError_t er_launch_math_eval(int fn, int n, const float* x, const float* y, float* out, cudaStream_t s);
 cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, const int nb[3], const float* sigma, int n,
                                float* rmq, int levels, uint32_t* minmax, float density_scale, float* majorant, cudaStream_t s);

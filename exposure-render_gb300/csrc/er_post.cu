@@ -40,11 +40,22 @@ ER_D uchar4 tonemap_px(float4 R, float exposure)
     return make_uchar4(o[0], o[1], o[2], (unsigned char)(R.w * 255.0f));
 }
 
-/* Gauss2D(1, dx, dy) - Source/filterframeestimate.cuh:28-31 */
-ER_D float gauss_w(int dx, int dy) { return er_expf(-((float)(dx * dx + dy * dy) / (2 * 1.0f * 1.0f))); }
+/* Gauss2D(1, dx, dy) - Source/filterframeestimate.cuh:28-31 - of a 3x3
+   window takes three values, by dx^2 + dy^2; made once on the host (er_expf
+   has the same bits there) instead of nine exponentials a pixel */
+struct GaussW {
+    float w[3];
+};
+
+static GaussW gauss_weights()
+{
+    GaussW g;
+    for (int d = 0; d < 3; d++) g.w[d] = er_expf(-((float)d / (2 * 1.0f * 1.0f)));
+    return g;
+}
 
 template <bool FROM_SUM>
-ER_D float4 filtered_pixel(const float4* __restrict__ src, float inv_n_div, int x, int y, int W, int H, int filter)
+ER_D float4 filtered_pixel(const float4* __restrict__ src, float inv_n_div, int x, int y, int W, int H, int filter, const GaussW& G)
 {
     const size_t c = (size_t)y * W + x;
     if (!filter) {
@@ -57,9 +68,13 @@ ER_D float4 filtered_pixel(const float4* __restrict__ src, float inv_n_div, int 
     const int y0 = (y - 1) > 0 ? (y - 1) : 0;
     const int y1 = (y + 1) < (H - 1) ? (y + 1) : (H - 1);
     float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f, tot = 0.0f;
-    for (int yy = y0; yy <= y1; yy++) {
-        for (int xx = x0; xx <= x1; xx++) {
-            const float w = gauss_w(xx - x, yy - y);
+#pragma unroll
+    for (int dy = -1; dy <= 1; dy++) {
+#pragma unroll
+        for (int dx = -1; dx <= 1; dx++) {
+            const int xx = x + dx, yy = y + dy;
+            if (xx < x0 || xx > x1 || yy < y0 || yy > y1) continue;
+            const float w = G.w[dx * dx + dy * dy];
             float4 f = src[(size_t)yy * W + xx];
             if (FROM_SUM) f = make_float4(f.x / inv_n_div, f.y / inv_n_div, f.z / inv_n_div, f.w / inv_n_div);
             s0 += f.x * w; s1 += f.y * w; s2 += f.z * w; s3 += f.w * w;
@@ -74,13 +89,13 @@ ER_D float4 filtered_pixel(const float4* __restrict__ src, float inv_n_div, int 
 }
 
 __global__ void k_post_frame(const float4* __restrict__ frame, float4* __restrict__ running, uchar4* __restrict__ rgba, int W,
-                             int H, int no_iterations, float exposure, int filter)
+                             int H, int no_iterations, float exposure, int filter, const GaussW G)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
     const size_t c = (size_t)y * W + x;
-    const float4 F = filtered_pixel<false>(frame, 1.0f, x, y, W, H, filter);
+    const float4 F = filtered_pixel<false>(frame, 1.0f, x, y, W, H, filter, G);
     const float div = smax((float)no_iterations, 1.0f);
     const float4 A = running[c];
     const float4 R = make_float4(A.x + (F.x - A.x) / div, A.y + (F.y - A.y) / div, A.z + (F.z - A.z) / div, A.w + (F.w - A.w) / div);
@@ -89,20 +104,20 @@ __global__ void k_post_frame(const float4* __restrict__ frame, float4* __restric
 }
 
 __global__ void k_post_mean(const float4* __restrict__ sum, float n, float4* __restrict__ running, uchar4* __restrict__ rgba, int W,
-                            int H, float exposure, int filter)
+                            int H, float exposure, int filter, const GaussW G)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
     const size_t c = (size_t)y * W + x;
-    const float4 R = filtered_pixel<true>(sum, n, x, y, W, H, filter);
+    const float4 R = filtered_pixel<true>(sum, n, x, y, W, H, filter, G);
     running[c] = R;
     rgba[c] = tonemap_px(R, exposure);
 }
 
 /* k_post_mean for every view of a batch (blockIdx.z = view); an accumulating
    view's sum holds samples [0, first + spp) of its stream */
-__global__ void k_post_batch(const WfView* __restrict__ views)
+__global__ void k_post_batch(const WfView* __restrict__ views, const GaussW G)
 {
     const WfView& V = views[blockIdx.z];
     if (!V.display) return;
@@ -112,7 +127,7 @@ __global__ void k_post_batch(const WfView* __restrict__ views)
     if (x >= W || y >= H) return;
     const float n = V.accumulate ? (float)(V.first + (uint32_t)V.spp) : (float)V.spp;
     const size_t c = (size_t)y * W + x;
-    const float4 R = filtered_pixel<true>(V.sum, n, x, y, W, H, V.filter);
+    const float4 R = filtered_pixel<true>(V.sum, n, x, y, W, H, V.filter, G);
     V.running[c] = R;
     V.rgba[c] = tonemap_px(R, V.exposure);
 }
@@ -136,38 +151,75 @@ ER_D float lum255(uchar4 c)
     return L;
 }
 
+/* The window's pixels and their luminances are made once per block in shared
+   memory (a 4K film at radius 2: 161 us a pass before, when every tap read
+   its range weight from the constant bank at a lane's own index and computed
+   its luminance again).  The tile is BIL_N pixels along the pass's axis by
+   BIL_M across; the range weights sit in shared memory too. */
+#define BIL_N 64
+#define BIL_M 16
+
 template <bool HORIZONTAL>
-__global__ void k_bilateral(const uchar4* __restrict__ in, uchar4* __restrict__ out, int W, int H, BilateralTables T)
+__global__ void __launch_bounds__(256) k_bilateral(const uchar4* __restrict__ in, uchar4* __restrict__ out, int W, int H, BilateralTables T)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= W || y >= H) return;
+    extern __shared__ uint32_t tile[];          /* (BIL_N + 2 r) * BIL_M pixels, then as many luminances */
+    __shared__ float range[256];
     const int r = T.radius;
-    const int i = HORIZONTAL ? x : y;
-    const int lim = HORIZONTAL ? W : H;
-    const int r0 = (i - r) > 0 ? (i - r) : 0;
-    const int r1 = (i + r) < (lim - 1) ? (i + r) : (lim - 1);
-    const uchar4 ctr = in[(size_t)y * W + x];
-    const float lc = lum255(ctr);
-    float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, tot = 0.0f;
-    for (int k = r0; k < r1; k++) {     /* window end exclusive (Source/filterrunningestimate.cuh:88,157) */
-        const uchar4 c = HORIZONTAL ? in[(size_t)y * W + k] : in[(size_t)k * W + x];
-        int d = (int)fabsf(lum255(c) - lc);
-        d = d > 255 ? 255 : d;
-        const float w = T.spatial[r + k - i] * T.range[d];
-        tot += w;
-        s0 += (float)c.x * w; s1 += (float)c.y * w; s2 += (float)c.z * w;
+    const int span = BIL_N + 2 * r;
+    float* lum = (float*)(tile + span * BIL_M);
+    const int n0 = blockIdx.x * BIL_N, m0 = blockIdx.y * BIL_M;
+    const int N = HORIZONTAL ? W : H, M = HORIZONTAL ? H : W;
+    range[threadIdx.x] = T.range[threadIdx.x];
+    /* neighbouring threads read neighbouring pixels of the film's rows */
+    for (int i = threadIdx.x; i < span * BIL_M; i += 256) {
+        const int n = HORIZONTAL ? i % span : i / BIL_M, m = HORIZONTAL ? i / span : i % BIL_M;
+        int a = n0 - r + n, b = m0 + m;
+        a = a < 0 ? 0 : (a > N - 1 ? N - 1 : a);
+        b = b > M - 1 ? M - 1 : b;
+        const uchar4 c = HORIZONTAL ? in[(size_t)b * W + a] : in[(size_t)a * W + b];
+        tile[i] = (uint32_t)c.x | ((uint32_t)c.y << 8) | ((uint32_t)c.z << 16);
+        lum[i] = lum255(c);
     }
-    uchar4 o;
-    if (tot > 0.0f) {
-        o.x = (unsigned char)eclamp(s0 / tot, 0.0f, 255.0f);
-        o.y = (unsigned char)eclamp(s1 / tot, 0.0f, 255.0f);
-        o.z = (unsigned char)eclamp(s2 / tot, 0.0f, 255.0f);
-    } else {
-        o.x = 0; o.y = 0; o.z = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < BIL_N * BIL_M; i += 256) {
+        const int n = HORIZONTAL ? i % BIL_N : i / BIL_M, m = HORIZONTAL ? i / BIL_N : i % BIL_M;
+        const int p = n0 + n, q = m0 + m;
+        if (p >= N || q >= M) continue;
+        const int k0 = (p - r) > 0 ? (p - r) : 0;
+        const int k1 = (p + r) < (N - 1) ? (p + r) : (N - 1);
+        const int step = HORIZONTAL ? 1 : BIL_M;
+        const int row = HORIZONTAL ? m * span : m;
+        const float lc = lum[row + (n + r) * step];
+        float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, tot = 0.0f;
+        for (int k = k0; k < k1; k++) {     /* window end exclusive (Source/filterrunningestimate.cuh:88,157) */
+            const int t = row + (k - n0 + r) * step;
+            const uint32_t c = tile[t];
+            int d = (int)fabsf(lum[t] - lc);
+            d = d > 255 ? 255 : d;
+            const float w = T.spatial[r + k - p] * range[d];
+            tot += w;
+            s0 += (float)(c & 0xffu) * w; s1 += (float)((c >> 8) & 0xffu) * w; s2 += (float)(c >> 16) * w;
+        }
+        uchar4 o;
+        if (tot > 0.0f) {
+            o.x = (unsigned char)eclamp(s0 / tot, 0.0f, 255.0f);
+            o.y = (unsigned char)eclamp(s1 / tot, 0.0f, 255.0f);
+            o.z = (unsigned char)eclamp(s2 / tot, 0.0f, 255.0f);
+        } else {
+            o.x = 0; o.y = 0; o.z = 0;
+        }
+        o.w = 255;
+        out[HORIZONTAL ? (size_t)q * W + p : (size_t)p * W + q] = o;
     }
-    o.w = 255;
-    out[(size_t)y * W + x] = o;
+}
+
+ER_D float voxel_gradient_magnitude(const Params& P, int X, int Y, int Z)
+{
+    const float sx = 2.0f * P.half_size[0], sy = 2.0f * P.half_size[1], sz = 2.0f * P.half_size[2];
+    const v3 p = V3(P.minp[0] + sx * (((float)X + 0.5f) * (1.0f / (float)P.res[0])),
+                    P.minp[1] + sy * (((float)Y + 0.5f) * (1.0f / (float)P.res[1])),
+                    P.minp[2] + sz * (((float)Z + 0.5f) * (1.0f / (float)P.res[2])));
+    return gradient_magnitude(P, p);
 }
 
 /* per-voxel gradient magnitude at voxel centres + max; the magnitude volume
@@ -179,11 +231,7 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
     const int Z = blockIdx.z * blockDim.z + threadIdx.z;
     float g = 0.0f;
     if (X < P.res[0] && Y < P.res[1] && Z < P.res[2]) {
-        const float sx = 2.0f * P.half_size[0], sy = 2.0f * P.half_size[1], sz = 2.0f * P.half_size[2];
-        const v3 p = V3(P.minp[0] + sx * (((float)X + 0.5f) * (1.0f / (float)P.res[0])),
-                        P.minp[1] + sy * (((float)Y + 0.5f) * (1.0f / (float)P.res[1])),
-                        P.minp[2] + sz * (((float)Z + 0.5f) * (1.0f / (float)P.res[2])));
-        g = gradient_magnitude(P, p);
+        g = voxel_gradient_magnitude(P, X, Y, Z);
         if (gm) {
             const size_t idx = (size_t)Z * P.res[0] * P.res[1] + (size_t)Y * P.res[0] + X;
             gm[idx] = (uint16_t)(g < 65535.0f ? g : 65535.0f);
@@ -198,6 +246,86 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
         b = v > b ? v : b;
     }
     if ((threadIdx.x + threadIdx.y * blockDim.x + threadIdx.z * blockDim.x * blockDim.y) % 32 == 0) atomicMax(max_bits, b);
+}
+
+/* The largest gradient magnitude alone, for the shader switch: only the
+   bricks of 8^3 voxels that can hold it are evaluated.  A voxel's six lookups
+   blend voxels at most two away from it, inside the brick's and its
+   neighbours' footprints [8 b, 8 b + 8], and a blend is no larger than the
+   largest of them and at most three below the smallest (all zero: zero); the
+   magnitude's float operations are monotone in the three differences, so with
+   each at the range's width they bound every voxel's magnitude.  First the
+   bricks whose bound is within a tenth of the largest, then those whose bound
+   still exceeds what they found.  512^3 shells: 4.3 ms with all voxels. */
+__global__ void k_gm_bound(const Params P, const uint32_t* __restrict__ minmax, int nbx, int nby, int nbz, uint32_t* __restrict__ bound,
+                           uint32_t* __restrict__ top)
+{
+    const uint32_t total = (uint32_t)nbx * nby * nbz;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t bits = 0;
+    if (i < total) {
+        const int x = (int)(i % nbx), y = (int)((i / nbx) % nby), z = (int)(i / ((uint32_t)nbx * nby));
+        uint32_t lo = 65535u, hi = 0u;
+        for (int dz = -1; dz <= 1; dz++)
+            for (int dy = -1; dy <= 1; dy++)
+                for (int dx = -1; dx <= 1; dx++) {
+                    const int a = iclamp(x + dx, 0, nbx - 1), b = iclamp(y + dy, 0, nby - 1), c = iclamp(z + dz, 0, nbz - 1);
+                    const uint32_t m = __ldg(minmax + ((size_t)c * nby + b) * nbx + a);
+                    lo = min(lo, m & 0xffffu);
+                    hi = max(hi, m >> 16);
+                }
+        float g = 0.0f;
+        if (hi > 0) {
+            float sum = 0.0f;
+            for (int k = 0; k < 3; k++) {
+                float D = (float)(hi - (lo > 3 ? lo - 3 : 0));
+                D *= 0.5f / P.spacing[k];
+                sum += D * D;
+            }
+            g = sqrtf(sum);
+        }
+        bits = __float_as_uint(g);
+        bound[i] = bits;
+    }
+    for (int o = 16; o > 0; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
+    if ((threadIdx.x & 31) == 0 && bits) atomicMax(top, bits);
+}
+
+/* lists the bricks to evaluate (round 0: bound above 0.9 of the largest;
+   round 1: of the rest, those above the largest magnitude found) */
+__global__ void k_gm_select(const uint32_t* __restrict__ bound, uint32_t total, const uint32_t* __restrict__ top,
+                            const unsigned int* __restrict__ found, int round, uint32_t* __restrict__ list, uint32_t* __restrict__ count)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool take = false;
+    if (i < total) {
+        const uint32_t b = bound[i];
+        const bool first = __uint_as_float(b) > 0.9f * __uint_as_float(*top);
+        take = round == 0 ? first : (!first && b > *found);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (!m) return;
+    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (take) list[base + __popc(m & ((1u << lane) - 1u))] = i;
+}
+
+__global__ void __launch_bounds__(512) k_gm_bricks(const Params P, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
+                                                   const uint32_t* __restrict__ bound, int nbx, int nby, unsigned int* max_bits)
+{
+    const uint32_t n = *count;
+    for (uint32_t e = blockIdx.x; e < n; e += gridDim.x) {
+        const uint32_t i = list[e];
+        if (bound[i] <= *(volatile unsigned int*)max_bits) continue;     /* raised by another block since */
+        const int X = (int)(i % nbx) * 8 + (int)(threadIdx.x & 7), Y = (int)((i / nbx) % nby) * 8 + (int)((threadIdx.x >> 3) & 7),
+                  Z = (int)(i / ((uint32_t)nbx * nby)) * 8 + (int)(threadIdx.x >> 6);
+        unsigned int b = 0;
+        if (X < P.res[0] && Y < P.res[1] && Z < P.res[2]) b = __float_as_uint(voxel_gradient_magnitude(P, X, Y, Z));
+        for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(max_bits, b);
+    }
 }
 
 __global__ void k_math_eval(int fn, int n, const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out)
@@ -233,7 +361,7 @@ cudaError_t er_launch_post_frame(const float4* frame, float4* running, uchar4* r
                                  int filter, cudaStream_t s)
 {
     const dim3 b(16, 8), g((W + 15) / 16, (H + 7) / 8);
-    k_post_frame<<<g, b, 0, s>>>(frame, running, rgba, W, H, n_iter, exposure, filter);
+    k_post_frame<<<g, b, 0, s>>>(frame, running, rgba, W, H, n_iter, exposure, filter, gauss_weights());
     return cudaGetLastError();
 }
 
@@ -241,14 +369,14 @@ cudaError_t er_launch_post_mean(const float4* sum, float n, float4* running, uch
                                 cudaStream_t s)
 {
     const dim3 b(16, 8), g((W + 15) / 16, (H + 7) / 8);
-    k_post_mean<<<g, b, 0, s>>>(sum, n, running, rgba, W, H, exposure, filter);
+    k_post_mean<<<g, b, 0, s>>>(sum, n, running, rgba, W, H, exposure, filter, gauss_weights());
     return cudaGetLastError();
 }
 
 cudaError_t er_launch_post_batch(const WfView* d_views, int n_views, int max_w, int max_h, cudaStream_t s)
 {
     const dim3 b(16, 8), g((max_w + 15) / 16, (max_h + 7) / 8, n_views);
-    k_post_batch<<<g, b, 0, s>>>(d_views);
+    k_post_batch<<<g, b, 0, s>>>(d_views, gauss_weights());
     return cudaGetLastError();
 }
 
@@ -261,9 +389,11 @@ cudaError_t er_launch_tonemap(const float4* xyza, float scale, uchar4* rgba, int
 cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int W, int H, const BilateralTables& T,
                                 cudaStream_t s)
 {
-    const dim3 b(16, 8), g((W + 15) / 16, (H + 7) / 8);
-    k_bilateral<true><<<g, b, 0, s>>>(in, tmp, W, H, T);
-    k_bilateral<false><<<g, b, 0, s>>>(tmp, out, W, H, T);
+    /* radius <= 127: at most 318 * 16 * 8 B = 40.7 KB */
+    const size_t bytes = (size_t)(BIL_N + 2 * T.radius) * BIL_M * 8;
+    const dim3 gh((W + BIL_N - 1) / BIL_N, (H + BIL_M - 1) / BIL_M), gv((H + BIL_N - 1) / BIL_N, (W + BIL_M - 1) / BIL_M);
+    k_bilateral<true><<<gh, 256, bytes, s>>>(in, tmp, W, H, T);
+    k_bilateral<false><<<gv, 256, bytes, s>>>(tmp, out, W, H, T);
     return cudaGetLastError();
 }
 
@@ -272,5 +402,23 @@ cudaError_t er_launch_gradient_magnitude(const Params& P, uint16_t* gm, unsigned
     const dim3 b(8, 8, 8);
     const dim3 g((P.res[0] + 7) / 8, (P.res[1] + 7) / 8, (P.res[2] + 7) / 8);
     k_gradient_magnitude<<<g, b, 0, s>>>(P, gm, max_bits);
+    return cudaGetLastError();
+}
+
+cudaError_t er_launch_gradient_max(const Params& P, uint32_t* scratch, unsigned int* max_bits, cudaStream_t s)
+{
+    const int nb[3] = { (P.res[0] + 7) / 8, (P.res[1] + 7) / 8, (P.res[2] + 7) / 8 };
+    const uint32_t total = (uint32_t)((size_t)nb[0] * nb[1] * nb[2]);
+    uint32_t *minmax = scratch, *bound = scratch + total, *list = scratch + 2 * (size_t)total, *top = scratch + 3 * (size_t)total, *count = top + 1;
+    const unsigned grid = (total + 255) / 256;
+    cudaError_t e = er_launch_brick_minmax(P.vox, P.res, 8, nb, minmax, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(top, 0, 2 * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    k_gm_bound<<<grid, 256, 0, s>>>(P, minmax, nb[0], nb[1], nb[2], bound, top);
+    for (int round = 0; round < 2; round++) {
+        if (round && (e = cudaMemsetAsync(count, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
+        k_gm_select<<<grid, 256, 0, s>>>(bound, total, top, max_bits, round, list, count);
+        k_gm_bricks<<<152 * 4, 512, 0, s>>>(P, list, count, bound, nb[0], nb[1], max_bits);
+    }
     return cudaGetLastError();
 }

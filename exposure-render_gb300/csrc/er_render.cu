@@ -60,6 +60,14 @@ __global__ void k_sigma_table(const Plf* __restrict__ opacity, float density_sca
     table[i] = density_scale * plf_eval(*opacity, (float)i);
 }
 
+/* a tracer's per-pixel lanes: lane 0 of every pixel, then lane 1 (seeding a
+   1024^2 film on the host and copying it took 4 ms of every restart) */
+__global__ void k_init_lanes(uint32_t seed, uint32_t* __restrict__ lanes, uint32_t n)
+{
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride) er_seed_lanes(seed, 0u, p, 0xffffffffu, &lanes[p], &lanes[(size_t)n + p]);
+}
+
 /* the shading transfer functions at every integer intensity (shade_tf) */
 __global__ void k_shade_table(const Tfs* __restrict__ tfs, float4* __restrict__ tab, int n)
 {
@@ -115,6 +123,13 @@ __global__ void k_autofocus(const Params P, int u, int v, uint32_t lane0, uint32
 cudaError_t er_launch_autofocus(const Params& P, int u, int v, uint32_t lane0, uint32_t lane1, float* out, cudaStream_t s)
 {
     k_autofocus<<<1, 32, 0, s>>>(P, u, v, lane0, lane1, out);
+    return cudaGetLastError();
+}
+
+cudaError_t er_launch_init_lanes(uint32_t seed, uint32_t* lanes, uint32_t n, cudaStream_t s)
+{
+    const uint32_t blocks = (n + 255) / 256;
+    k_init_lanes<<<blocks < 2432 ? blocks : 2432, 256, 0, s>>>(seed, lanes, n);
     return cudaGetLastError();
 }
 

@@ -231,13 +231,23 @@ struct VolumeItem {
     float spacing[3];
     int normalize;
     uint16_t vmax = 0;
-    uint64_t signature = 0;        /* sampled content hash (tuning cache key) */
+    /* sampled content hash (tuning cache key), made when a key is asked for
+       (volume_signature): FNV-1a over the resolution, every 61st voxel as
+       bound and what later region edits add.  Until then the edits' bytes wait
+       in sig_log, and sig_base holds the bound voxels' samples from the first
+       edit on.  (Hashing at every bind took 4 of the 7 ms that binding a
+       384x384x256 volume and showing it took.) */
+    uint64_t signature = 0;
+    bool sig_pending = false;
+    std::vector<unsigned char> sig_log;
+    DevBuf<uint16_t> sig_base;
     uint64_t edits = 0;            /* region edits from device voxels (folded into the signature) */
     DevBuf<uint16_t> vox;
     DevBuf<uint2> quad;            /* corner quads (NULL when they do not fit in memory) */
     int qb_nbx = 0;                /* quads in 8^3 bricks: bricks along x (0: x fastest) */
     unsigned long long qb_slab = 0;
     DevBuf<unsigned int> gm_max_bits;
+    DevBuf<uint32_t> gm_scratch;   /* er_launch_gradient_max */
     DevBuf<unsigned int> box_max;  /* largest voxel of an uploaded box */
     float gm_max = -1.0f;          /* lazily computed maximum gradient magnitude */
 };
@@ -538,10 +548,8 @@ er_status check_settings(const er_tracer_desc& d)
 
 er_status init_lanes(TracerItem& t)
 {
-    const size_t n = (size_t)t.W * t.H;
-    std::vector<uint32_t> h(2 * n);
-    for (size_t p = 0; p < n; p++) er_seed_lanes(t.d.settings.seed, 0u, (uint32_t)p, 0xffffffffu, &h[p], &h[n + p]);
-    ER_CUDA(cudaMemcpyAsync(t.lanes.p, h.data(), 2 * n * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx().stream));
+    ER_CUDA(er_launch_init_lanes(t.d.settings.seed, t.lanes.p, (uint32_t)((size_t)t.W * t.H), ctx().stream));
+    /* the cleared buffers may be used from another stream next */
     ER_CUDA(cudaStreamSynchronize(ctx().stream));
     return ER_OK;
 }
@@ -1021,6 +1029,38 @@ std::string tune_cache_path()
     return std::string(home) + "/.cache/exposurerender_gb300/autotune.txt";
 }
 
+/* every 61st voxel of the volume into sig_base */
+er_status sample_voxels(VolumeItem& v, cudaStream_t s)
+{
+    const size_t n = (size_t)v.res[0] * v.res[1] * v.res[2];
+    ER_CUDA(v.sig_base.ensure((n + 60) / 61));
+    ER_CUDA(er_launch_sample_voxels(v.vox.p, n, 61, v.sig_base.p, s));
+    return ER_OK;
+}
+
+/* makes the volume's signature from what has waited for it */
+er_status volume_signature(VolumeItem& v)
+{
+    if (!v.sig_pending) return ER_OK;
+    cudaStream_t s = ctx().stream;
+    if (!v.sig_base.p) {
+        const er_status ss = sample_voxels(v, s);
+        if (ss != ER_OK) return ss;
+    }
+    std::vector<uint16_t> h(((size_t)v.res[0] * v.res[1] * v.res[2] + 60) / 61);
+    ER_CUDA(cudaMemcpyAsync(h.data(), v.sig_base.p, h.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost, s));
+    ER_CUDA(cudaStreamSynchronize(s));
+    const int32_t res[3] = { v.res[0], v.res[1], v.res[2] };
+    uint64_t sig = fnv1a(kFnvBasis, res, sizeof(res));
+    sig = fnv1a(sig, h.data(), h.size() * sizeof(uint16_t));
+    v.signature = fnv1a(sig, v.sig_log.data(), v.sig_log.size());
+    v.sig_pending = false;
+    v.sig_log.clear();
+    v.sig_log.shrink_to_fit();
+    v.sig_base.release();
+    return ER_OK;
+}
+
 /* device, volume content and every setting that changes the work of a sample */
 uint64_t tune_key(const TracerItem& t, const VolumeItem& v, int probe_spp)
 {
@@ -1310,10 +1350,9 @@ ER_API er_status er_bind_volume(const er_volume_desc* d, int32_t* id)
     for (int i = 0; i < 3; i++) { v->res[i] = d->resolution[i]; v->spacing[i] = d->spacing[i]; }
     v->normalize = d->normalize_size;
     v->gm_max = -1.0f;
-    /* content signature of the tuning cache: every 61st voxel */
-    uint64_t sig = fnv1a(kFnvBasis, d->resolution, sizeof(d->resolution));
-    for (size_t i = 0; i < n; i += 61) sig = fnv1a(sig, &d->voxels[i], sizeof(uint16_t));
-    v->signature = sig;
+    v->sig_pending = true;
+    v->sig_log.clear();
+    v->sig_base.release();
     const int lo[3] = { 0, 0, 0 };
     unsigned int vmax = 0;
     er_status us = upload_box(*v, lo, d->resolution, d->voxels, cudaMemcpyHostToDevice, C.stream, &vmax);
@@ -1340,6 +1379,10 @@ static er_status update_volume_region(int32_t id, const int32_t* offset, const i
     }
     /* the volume may be read by queued work: the edit follows it */
     ER_CUDA(cudaStreamSynchronize(C.stream));
+    if (v.sig_pending && !v.sig_base.p) {
+        const er_status ss = sample_voxels(v, s);
+        if (ss != ER_OK) return ss;
+    }
     unsigned int bmax = 0;
     er_status us = upload_box(v, offset, size, voxels, kind, s, &bmax);
     if (us != ER_OK) return us;
@@ -1348,15 +1391,21 @@ static er_status update_volume_region(int32_t id, const int32_t* offset, const i
     /* tuning-cache signature: the edit's box, its contents (every 61st of
        the host voxels, as er_bind_volume samples a whole volume) and, for
        device voxels the host cannot read, the volume's edit count */
-    v.signature = fnv1a(v.signature, offset, 3 * sizeof(int32_t));
-    v.signature = fnv1a(v.signature, size, 3 * sizeof(int32_t));
+    auto sign = [&](const void* p, size_t bytes) {
+        if (v.sig_pending) v.sig_log.insert(v.sig_log.end(), (const unsigned char*)p, (const unsigned char*)p + bytes);
+        else v.signature = fnv1a(v.signature, p, bytes);
+    };
+    sign(offset, 3 * sizeof(int32_t));
+    sign(size, 3 * sizeof(int32_t));
     const size_t n = (size_t)size[0] * size[1] * size[2];
     if (kind == cudaMemcpyHostToDevice) {
-        for (size_t i = 0; i < n; i += 61) v.signature = fnv1a(v.signature, &voxels[i], sizeof(uint16_t));
+        for (size_t i = 0; i < n; i += 61) sign(&voxels[i], sizeof(uint16_t));
     } else {
         v.edits++;
-        v.signature = fnv1a(v.signature, &v.edits, sizeof(v.edits));
+        sign(&v.edits, sizeof(v.edits));
     }
+    if (v.sig_log.size() > ((size_t)1 << 20)) us = volume_signature(v);
+    if (us != ER_OK) return us;
     C.version++;
     return ER_OK;
 }
@@ -1868,7 +1917,9 @@ ER_API er_status er_autotune_tracer(int32_t tracer_id, int32_t probe_spp, er_tun
     er_status st = build(*t);
     if (st != ER_OK) return st;
     Context& C = ctx();
-    const VolumeItem& v = *C.volumes.items.find(t->d.volume_id)->second;
+    VolumeItem& v = *C.volumes.items.find(t->d.volume_id)->second;
+    st = volume_signature(v);
+    if (st != ER_OK) return st;
     const uint64_t key = tune_key(*t, v, probe_spp);
     er_tune_result r;
     memset(&r, 0, sizeof(r));
@@ -2186,7 +2237,14 @@ ER_API er_status er_gradient_magnitude(int32_t volume_id, uint16_t* d_gm, float*
     ER_CUDA(v.gm_max_bits.ensure(1));
     cudaStream_t s = ctx().stream;
     ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, sizeof(unsigned int), s));
-    ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
+    const size_t bricks = (size_t)((P.res[0] + 7) / 8) * ((P.res[1] + 7) / 8) * ((P.res[2] + 7) / 8);
+    if (!d_gm && bricks < (1ull << 31) && v.gm_scratch.ensure(3 * bricks + 2) == cudaSuccess) {
+        /* the maximum alone: only bricks that can hold it */
+        ER_CUDA(er_launch_gradient_max(P, v.gm_scratch.p, v.gm_max_bits.p, s));
+    } else {
+        cudaGetLastError();
+        ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
+    }
     unsigned int bits = 0;
     ER_CUDA(cudaMemcpyAsync(&bits, v.gm_max_bits.p, sizeof(bits), cudaMemcpyDeviceToHost, s));
     ER_CUDA(cudaStreamSynchronize(s));

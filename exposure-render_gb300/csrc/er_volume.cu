@@ -181,6 +181,24 @@ static void launch_minmax(const uint16_t* vox, const int res[3], int B, const in
         k_brick_minmax<1><<<grid, BM_THREADS, 0, s>>>(vox, res[0], res[1], res[2], B, nb[0], nb[1], nb[2], xbricks, zbricks, xblocks, minmax);
 }
 
+cudaError_t er_launch_brick_minmax(const uint16_t* vox, const int res[3], int B, const int nb[3], uint32_t* minmax, cudaStream_t s)
+{
+    launch_minmax(vox, res, B, nb, minmax, s);
+    return cudaGetLastError();
+}
+
+__global__ void k_sample_voxels(const uint16_t* __restrict__ vox, size_t n, int step, uint16_t* __restrict__ out)
+{
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i * step < n; i += stride) out[i] = vox[i * step];
+}
+
+cudaError_t er_launch_sample_voxels(const uint16_t* vox, size_t n, int step, uint16_t* out, cudaStream_t s)
+{
+    k_sample_voxels<<<1216, 256, 0, s>>>(vox, n, step, out);
+    return cudaGetLastError();
+}
+
 cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, const int nb[3], const float* sigma, int n,
                                float* rmq, int levels, uint32_t* minmax, float density_scale, float* majorant, cudaStream_t s)
 {
@@ -252,9 +270,10 @@ cudaError_t er_launch_empty_skip(float* majorant, const int nb[3], uint8_t* tmp,
 /* The empty-space map of the fixed-step march: dist bytes of bricks of
    2^shift voxels a side (k_skip_pass<1>).  A brick is empty when sigma is
    exactly zero (of either sign) at every intensity a lookup in it can have,
-   lo - 1 .. hi as for the majorant: a step there adds nothing to the march's
-   sum, so the march may leave the lookup out.  A negative or NaN sigma counts
-   as not empty. */
+   lo - 3 .. hi (each of the blend's three truncated lerps can round to one
+   below its smaller end): a step there adds nothing to the march's sum, so
+   the march may leave the lookup out.  A negative or NaN sigma counts as not
+   empty. */
 __global__ void __launch_bounds__(1024) k_nonzero_prefix(const float* __restrict__ sigma, uint32_t* __restrict__ count, int n)
 {
     __shared__ uint32_t part[32];
@@ -284,7 +303,7 @@ __global__ void k_occupancy(const uint32_t* __restrict__ minmax, const uint32_t*
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const uint32_t mm = minmax[i];
-    int lo = (int)(mm & 0xffffu) - 1, hi = (int)(mm >> 16);
+    int lo = (int)(mm & 0xffffu) - 3, hi = (int)(mm >> 16);
     lo = lo < 0 ? 0 : (lo > n - 1 ? n - 1 : lo);
     hi = hi > n - 1 ? n - 1 : hi;
     const uint32_t below = lo > 0 ? count[lo - 1] : 0u;
@@ -313,37 +332,61 @@ cudaError_t er_launch_march_map(const uint16_t* vox, const int res[3], int shift
    kernel writes the quads of the voxels in the box [lo, lo + n) (a region
    edit changes the quads of the voxels one below it in x and y as well) and
    finds the largest voxel value in the box. */
-__global__ void k_box_quads_max(const uint16_t* __restrict__ vox, int rx, int ry, int x0, int y0, int z0, int nx, int ny, int nz,
-                                uint2* __restrict__ quad, int qb_nbx, unsigned long long qb_slab, unsigned int* __restrict__ vmax)
+/* A warp takes a row of the box at a time (no division per voxel: one 64-bit
+   remainder chain a voxel bounded the kernel before, 569 us at 512^3); a lane
+   makes VEC neighbouring quads: with VEC 2 (x fastest, even rows) it reads
+   three voxels of two rows as two words and stores both quads as 16 bytes. */
+template <int VEC>
+__global__ void __launch_bounds__(256) k_box_quads_max(const uint16_t* __restrict__ vox, int rx, int ry, int x0, int y0, int z0, int nx,
+                                                       int ny, int nz, uint2* __restrict__ quad, int qb_nbx,
+                                                       unsigned long long qb_slab, unsigned int* __restrict__ vmax)
 {
-    const size_t n = (size_t)nx * ny * nz;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const long long rows = (long long)ny * nz;
+    const long long stride = (long long)gridDim.x * (blockDim.x >> 5);
+    const int lane = threadIdx.x & 31;
     unsigned int m = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const int x = x0 + (int)(i % nx), y = y0 + (int)((i / nx) % ny), z = z0 + (int)(i / ((size_t)nx * ny));
-        const size_t zb = (size_t)z * rx * ry;
-        const int x1 = x + 1 < rx ? x + 1 : rx - 1, y1 = y + 1 < ry ? y + 1 : ry - 1;
-        const uint32_t v00 = vox[zb + (size_t)y * rx + x], v10 = vox[zb + (size_t)y * rx + x1];
-        const uint32_t v01 = vox[zb + (size_t)y1 * rx + x], v11 = vox[zb + (size_t)y1 * rx + x1];
-        if (quad) quad[erd::quad_index(x, y, z, rx, ry, qb_nbx, qb_slab)] = make_uint2(v00 | (v10 << 16), v01 | (v11 << 16));
-        m = v00 > m ? v00 : m;
+    for (long long r = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += stride) {
+        const int y = y0 + (int)(r % ny), z = z0 + (int)(r / ny);
+        const int y1 = y + 1 < ry ? y + 1 : ry - 1;
+        const uint16_t* a = vox + ((size_t)z * ry + y) * (size_t)rx;
+        const uint16_t* b = vox + ((size_t)z * ry + y1) * (size_t)rx;
+        if (VEC == 2) {
+#pragma unroll 2
+            for (int x = x0 + 2 * lane; x < x0 + nx; x += 64) {
+                const int x2 = x + 2 < rx ? x + 2 : rx - 1;
+                const uint32_t wa = *(const uint32_t*)(a + x), wb = *(const uint32_t*)(b + x);
+                const uint32_t na = a[x2], nb = b[x2];
+                const uint32_t a1 = wa >> 16, b1 = wb >> 16;
+                *(uint4*)(quad + ((size_t)z * ry + y) * (size_t)rx + x) = make_uint4(wa, wb, a1 | (na << 16), b1 | (nb << 16));
+                m = max(m, max(wa & 0xffffu, a1));
+            }
+        } else {
+            for (int x = x0 + lane; x < x0 + nx; x += 32) {
+                const int x1 = x + 1 < rx ? x + 1 : rx - 1;
+                const uint32_t v00 = a[x], v10 = a[x1], v01 = b[x], v11 = b[x1];
+                if (quad) quad[erd::quad_index(x, y, z, rx, ry, qb_nbx, qb_slab)] = make_uint2(v00 | (v10 << 16), v01 | (v11 << 16));
+                m = max(m, v00);
+            }
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned int t = __shfl_xor_sync(0xffffffffu, m, o);
-        m = t > m ? t : m;
-    }
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(vmax, m);
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0 && m) atomicMax(vmax, m);
 }
 
 cudaError_t er_launch_box_quads_max(const uint16_t* vox, const int res[3], const int lo[3], const int n[3], uint2* quad, int qb_nbx,
                                     unsigned long long qb_slab, unsigned int* vmax, cudaStream_t s)
 {
-    const size_t total = (size_t)n[0] * n[1] * n[2];
-    if (total == 0) return cudaSuccess;
-    size_t blocks = (total + 255) / 256;
-    if (blocks > 4096) blocks = 4096;
-    k_box_quads_max<<<(unsigned)blocks, 256, 0, s>>>(vox, res[0], res[1], lo[0], lo[1], lo[2], n[0], n[1], n[2], quad, qb_nbx, qb_slab,
-                                                     vmax);
+    const long long rows = (long long)n[1] * n[2];
+    if (rows == 0 || n[0] == 0) return cudaSuccess;
+    const long long want = (rows + 7) / 8;
+    const unsigned blocks = (unsigned)(want < 152 * 16 ? want : 152 * 16);
+    /* pairs: the rows' first voxels and quads aligned, the box's pairs whole */
+    const bool pairs = quad && qb_nbx == 0 && (res[0] & 1) == 0 && (lo[0] & 1) == 0 && (n[0] & 1) == 0 && ((uintptr_t)vox & 3u) == 0 &&
+                       ((uintptr_t)quad & 15u) == 0;
+    if (pairs)
+        k_box_quads_max<2><<<blocks, 256, 0, s>>>(vox, res[0], res[1], lo[0], lo[1], lo[2], n[0], n[1], n[2], quad, qb_nbx, qb_slab, vmax);
+    else
+        k_box_quads_max<1><<<blocks, 256, 0, s>>>(vox, res[0], res[1], lo[0], lo[1], lo[2], n[0], n[1], n[2], quad, qb_nbx, qb_slab, vmax);
     return cudaGetLastError();
 }
 

@@ -897,6 +897,11 @@ __global__ void k_wf_reduce(const WfView* __restrict__ views, const WfSegment* _
 
 /* ---- host side ---- */
 
+/* Two translation units compile this file (each its half of the kernels'
+   variants, in parallel): er_wavefront.cu the one-view launches and the plan
+   and profiler, er_wavefront_batch.cu (WF_BATCH_UNIT) the batch launches. */
+#ifndef WF_BATCH_UNIT
+
 void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, WavefrontPlan& plan)
 {
     plan.segs.clear();
@@ -932,8 +937,6 @@ void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t wind
     }
 }
 
-namespace {
-
 /* stage timing (er_profile_*): CUDA events around every stage launch on the
    launching stream, read back and accumulated by er_wavefront_profile_read */
 struct StageProfiler {
@@ -957,14 +960,14 @@ struct StageProfiler {
     }
 };
 
-StageProfiler& profiler()
+static StageProfiler& profiler()
 {
     static StageProfiler* p = new StageProfiler();
     return *p;
 }
 
 /* records the start of a stage; returns the event or nullptr when off */
-cudaEvent_t stage_begin(cudaStream_t s)
+cudaEvent_t wf_stage_begin(cudaStream_t s)
 {
     StageProfiler& P = profiler();
     std::lock_guard<std::mutex> lock(P.m);
@@ -977,7 +980,7 @@ cudaEvent_t stage_begin(cudaStream_t s)
     return a;
 }
 
-void stage_end(cudaEvent_t a, int stage, cudaStream_t s)
+void wf_stage_end(cudaEvent_t a, int stage, cudaStream_t s)
 {
     if (!a) return;
     StageProfiler& P = profiler();
@@ -986,6 +989,15 @@ void stage_end(cudaEvent_t a, int stage, cudaStream_t s)
     cudaEventRecord(b, s);
     P.pending.push_back({a, b, stage});
 }
+
+#else
+
+cudaEvent_t wf_stage_begin(cudaStream_t s);
+void wf_stage_end(cudaEvent_t a, int stage, cudaStream_t s);
+
+#endif
+
+namespace {
 
 int sm_count()
 {
@@ -1018,7 +1030,7 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         cudaError_t e = cudaMemsetAsync(B.counters, 0, 6 * sizeof(uint32_t), s);
         if (e != cudaSuccess) return e;
         const uint32_t g1 = (items + 255) / 256 < (uint32_t)sm * 64 ? (items + 255) / 256 : (uint32_t)sm * 64;
-        cudaEvent_t t0 = stage_begin(s);
+        cudaEvent_t t0 = wf_stage_begin(s);
 #define ER_PRIMARY(M, O, F) k_wf_primary<M, ONE, O, F><<<g1, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters)
 #define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2, B.cross_eighths, B.collide_eighths, B.gate_primary)
         if (B.pt_primary) {
@@ -1054,8 +1066,8 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         } else ER_PRIMARY(4, false, WF_MIXED);
 #undef ER_PRIMARY_PT
 #undef ER_PRIMARY
-        stage_end(t0, 0, s);
-        t0 = stage_begin(s);
+        wf_stage_end(t0, 0, s);
+        t0 = wf_stage_begin(s);
 #define ER_SHADE(M, O) k_wf_shade<ONE, M, O><<<sm * 16, 128, 0, s>>>(d_views, one, B.events, B.counters, B.results, B.jobs, B.counters + 1)
 #define ER_SORTED(M) k_wf_shade_sorted<ONE, M><<<sm * 16, 128, 0, s>>>(d_views, one, B.records, cap, B.counters + 4, B.results, B.jobs, \
                                                                     B.counters + 1)
@@ -1078,8 +1090,8 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         }
 #undef ER_SORTED
 #undef ER_SHADE
-        stage_end(t0, 1, s);
-        t0 = stage_begin(s);
+        wf_stage_end(t0, 1, s);
+        t0 = wf_stage_begin(s);
 #define ER_SHADOW(M, O, F) k_wf_shadow<M, ONE, O, F><<<sm * 8, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results)
 #define ER_SHADOW_PT(M, O) k_wf_shadow_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.cross_eighths, B.collide_eighths, B.gate_shadow)
         if (B.pt_shadow) {
@@ -1115,15 +1127,15 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
         } else ER_SHADOW(4, false, WF_MIXED);
 #undef ER_SHADOW_PT
 #undef ER_SHADOW
-        stage_end(t0, 2, s);
+        wf_stage_end(t0, 2, s);
         int max_npix = 0;
         for (int g = s0; g < s1; g++) {
             const int np = plan.view_npix[plan.segs[g].view];
             if (np > max_npix) max_npix = np;
         }
-        t0 = stage_begin(s);
+        t0 = wf_stage_begin(s);
         k_wf_reduce<ONE><<<dim3((max_npix + 255) / 256, ONE ? 1 : nseg), 256, 0, s>>>(d_views, dseg, one, one_seg, B.results, p_in, p_out);
-        stage_end(t0, 3, s);
+        wf_stage_end(t0, 3, s);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1132,17 +1144,11 @@ cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const
 
 }  // namespace
 
+#ifndef WF_BATCH_UNIT
+
 cudaError_t er_launch_wavefront_one(const WfView& view, const WavefrontPlan& plan, const WavefrontBuffers& B, cudaStream_t s)
 {
     return launch_windows<true>(nullptr, nullptr, view, plan, B, s);
-}
-
-cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfSegment* d_segs, const WavefrontPlan& plan,
-                                      const WavefrontBuffers& B, cudaStream_t s)
-{
-    WfView unused;
-    memset(&unused, 0, sizeof(unused));
-    return launch_windows<false>(d_views, d_segs, unused, plan, B, s);
 }
 
 void er_wavefront_profile_enable(bool on)
@@ -1176,3 +1182,15 @@ cudaError_t er_wavefront_profile_read(double* ms, int64_t* launches)
     }
     return err;
 }
+
+#else
+
+cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfSegment* d_segs, const WavefrontPlan& plan,
+                                      const WavefrontBuffers& B, cudaStream_t s)
+{
+    WfView unused;
+    memset(&unused, 0, sizeof(unused));
+    return launch_windows<false>(d_views, d_segs, unused, plan, B, s);
+}
+
+#endif
