@@ -39,11 +39,10 @@ cudaError_t er_launch_tonemap(const float4* xyza, float scale, uchar4* rgba, int
 cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int W, int H, const BilateralTables& T,
                                 cudaStream_t s);
 cudaError_t er_launch_gradient_magnitude(const erd::Params& P, uint16_t* gm, unsigned int* max_bits, cudaStream_t s);
-/* the largest gradient magnitude alone (as er_launch_gradient_magnitude);
-   scratch: 3 words per 8^3 brick and 2 more; max_bits zero before */
-cudaError_t er_launch_gradient_max(const erd::Params& P, uint32_t* scratch, unsigned int* max_bits, cudaStream_t s);
-/* lo | hi << 16 of every B^3 brick's footprint, voxels b B .. (b + 1) B per axis (er_volume.cu) */
-cudaError_t er_launch_brick_minmax(const uint16_t* vox, const int res[3], int B, const int nb[3], uint32_t* minmax, cudaStream_t s);
+/* the largest gradient magnitude alone (as er_launch_gradient_magnitude) of a
+   volume it applies to, whose largest voxel is vmax: bits[0]; two words, zero before */
+bool er_gradient_max_applies(const erd::Params& P);
+cudaError_t er_launch_gradient_max(const erd::Params& P, int vmax, unsigned int* bits, cudaStream_t s);
 /* every step-th of n voxels into out */
 cudaError_t er_launch_sample_voxels(const uint16_t* vox, size_t n, int step, uint16_t* out, cudaStream_t s);
 cudaError_t er_launch_math_eval(int fn, int n, const float* x, const float* y, float* out, cudaStream_t s);

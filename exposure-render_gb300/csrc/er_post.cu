@@ -248,84 +248,68 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
     if ((threadIdx.x + threadIdx.y * blockDim.x + threadIdx.z * blockDim.x * blockDim.y) % 32 == 0) atomicMax(max_bits, b);
 }
 
-/* The largest gradient magnitude alone, for the shader switch: only the
-   bricks of 8^3 voxels that can hold it are evaluated.  A voxel's six lookups
-   blend voxels at most two away from it, inside the brick's and its
-   neighbours' footprints [8 b, 8 b + 8], and a blend is no larger than the
-   largest of them and at most three below the smallest (all zero: zero); the
-   magnitude's float operations are monotone in the three differences, so with
-   each at the range's width they bound every voxel's magnitude.  First the
-   bricks whose bound is within a tenth of the largest, then those whose bound
-   still exceeds what they found.  512^3 shells: 4.3 ms with all voxels. */
-__global__ void k_gm_bound(const Params P, const uint32_t* __restrict__ minmax, int nbx, int nby, int nbz, uint32_t* __restrict__ bound,
-                           uint32_t* __restrict__ top)
+/* The largest gradient magnitude alone, for the shader switch, of a volume
+   with one spacing on all axes.  A voxel's six lookups lie (but for rounding)
+   at its neighbours' centres, where the blend is the mean of a cell's eight
+   voxels: integer sums give each magnitude to within a known error, and only
+   the voxels that may hold the maximum make their six lookups.  Two passes:
+   the largest lower bound, then the exact magnitudes of the voxels whose
+   upper bound reaches it.  tol: how far a lookup may be from its cell's mean
+   (three truncations, the weights' rounding).
+
+   A block walks GM_Z planes of a GM_X x GM_Y tile of cells (a ring of halo
+   around the voxels): a thread sums its cell's four voxels of a plane, adds
+   the plane before, and shares three planes of cell sums.  Bound by the read
+   of the volume.  Every voxel's six lookups took 1213 us at 384x384x256 and
+   4304 us at 512^3. */
+#define GM_X 32
+#define GM_Y 16
+#define GM_Z 32
+
+template <bool EXACT>
+__global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float tol, const unsigned int* low_in, unsigned int* out_bits)
 {
-    const uint32_t total = (uint32_t)nbx * nby * nbz;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t bits = 0;
-    if (i < total) {
-        const int x = (int)(i % nbx), y = (int)((i / nbx) % nby), z = (int)(i / ((uint32_t)nbx * nby));
-        uint32_t lo = 65535u, hi = 0u;
-        for (int dz = -1; dz <= 1; dz++)
-            for (int dy = -1; dy <= 1; dy++)
-                for (int dx = -1; dx <= 1; dx++) {
-                    const int a = iclamp(x + dx, 0, nbx - 1), b = iclamp(y + dy, 0, nby - 1), c = iclamp(z + dz, 0, nbz - 1);
-                    const uint32_t m = __ldg(minmax + ((size_t)c * nby + b) * nbx + a);
-                    lo = min(lo, m & 0xffffu);
-                    hi = max(hi, m >> 16);
-                }
-        float g = 0.0f;
-        if (hi > 0) {
-            float sum = 0.0f;
-            for (int k = 0; k < 3; k++) {
-                float D = (float)(hi - (lo > 3 ? lo - 3 : 0));
-                D *= 0.5f / P.spacing[k];
-                sum += D * D;
+    __shared__ int cells[3][GM_Y][GM_X];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int X = (int)blockIdx.x * (GM_X - 2) - 1 + tx, Y = (int)blockIdx.y * (GM_Y - 2) - 1 + ty;
+    const int z0 = (int)blockIdx.z * GM_Z, z1 = min(z0 + GM_Z, P.res[2]);
+    const size_t rx = (size_t)P.res[0], slice = rx * (size_t)P.res[1];
+    const size_t xa = (size_t)iclamp(X, 0, P.res[0] - 1), xb = (size_t)iclamp(X + 1, 0, P.res[0] - 1);
+    const size_t ya = (size_t)iclamp(Y, 0, P.res[1] - 1) * rx, yb = (size_t)iclamp(Y + 1, 0, P.res[1] - 1) * rx;
+    auto plane = [&](int z) -> int {
+        const uint16_t* v = P.vox + (size_t)iclamp(z, 0, P.res[2] - 1) * slice;
+        return (int)__ldg(v + ya + xa) + (int)__ldg(v + ya + xb) + (int)__ldg(v + yb + xa) + (int)__ldg(v + yb + xb);
+    };
+    const bool inner = tx > 0 && tx < GM_X - 1 && ty > 0 && ty < GM_Y - 1 && X < P.res[0] && Y < P.res[1];
+    const float h = 0.5f / P.spacing[0];
+    const float low = EXACT ? __uint_as_float(*low_in) : 0.0f;
+    unsigned int best = 0;
+    int prev = plane(z0 - 1);
+    /* cell z is in cells[(z + 3) % 3]; voxel z needs cells z - 1, z and z + 1 */
+    for (int z = z0 - 1; z <= z1; z++) {
+        const int next = plane(z + 1);
+        cells[(z + 3) % 3][ty][tx] = prev + next;
+        prev = next;
+        __syncthreads();
+        const int Z = z - 1;
+        if (Z >= z0 && inner) {
+            const int c = (Z + 3) % 3;
+            const float dx = fabsf((float)(cells[c][ty][tx - 1] - cells[c][ty][tx + 1])) * 0.125f;
+            const float dy = fabsf((float)(cells[c][ty - 1][tx] - cells[c][ty + 1][tx])) * 0.125f;
+            const float dz = fabsf((float)(cells[(Z + 2) % 3][ty][tx] - cells[(Z + 4) % 3][ty][tx])) * 0.125f;
+            if (EXACT) {
+                const float a = (dx + 2.0f * tol) * h, b = (dy + 2.0f * tol) * h, e = (dz + 2.0f * tol) * h;
+                if (sqrtf(a * a + b * b + e * e) * 1.00001f >= low) best = max(best, __float_as_uint(voxel_gradient_magnitude(P, X, Y, Z)));
+            } else {
+                const float a = fmaxf(dx - 2.0f * tol, 0.0f) * h, b = fmaxf(dy - 2.0f * tol, 0.0f) * h, e = fmaxf(dz - 2.0f * tol, 0.0f) * h;
+                best = max(best, __float_as_uint(sqrtf(a * a + b * b + e * e) * 0.99999f));
             }
-            g = sqrtf(sum);
         }
-        bits = __float_as_uint(g);
-        bound[i] = bits;
+        /* the next plane overwrites cell z - 2, which voxel z - 1 has read */
+        __syncthreads();
     }
-    for (int o = 16; o > 0; o >>= 1) bits = max(bits, __shfl_xor_sync(0xffffffffu, bits, o));
-    if ((threadIdx.x & 31) == 0 && bits) atomicMax(top, bits);
-}
-
-/* lists the bricks to evaluate (round 0: bound above 0.9 of the largest;
-   round 1: of the rest, those above the largest magnitude found) */
-__global__ void k_gm_select(const uint32_t* __restrict__ bound, uint32_t total, const uint32_t* __restrict__ top,
-                            const unsigned int* __restrict__ found, int round, uint32_t* __restrict__ list, uint32_t* __restrict__ count)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool take = false;
-    if (i < total) {
-        const uint32_t b = bound[i];
-        const bool first = __uint_as_float(b) > 0.9f * __uint_as_float(*top);
-        take = round == 0 ? first : (!first && b > *found);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, take);
-    if (!m) return;
-    const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-    uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(count, (uint32_t)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (take) list[base + __popc(m & ((1u << lane) - 1u))] = i;
-}
-
-__global__ void __launch_bounds__(512) k_gm_bricks(const Params P, const uint32_t* __restrict__ list, const uint32_t* __restrict__ count,
-                                                   const uint32_t* __restrict__ bound, int nbx, int nby, unsigned int* max_bits)
-{
-    const uint32_t n = *count;
-    for (uint32_t e = blockIdx.x; e < n; e += gridDim.x) {
-        const uint32_t i = list[e];
-        if (bound[i] <= *(volatile unsigned int*)max_bits) continue;     /* raised by another block since */
-        const int X = (int)(i % nbx) * 8 + (int)(threadIdx.x & 7), Y = (int)((i / nbx) % nby) * 8 + (int)((threadIdx.x >> 3) & 7),
-                  Z = (int)(i / ((uint32_t)nbx * nby)) * 8 + (int)(threadIdx.x >> 6);
-        unsigned int b = 0;
-        if (X < P.res[0] && Y < P.res[1] && Z < P.res[2]) b = __float_as_uint(voxel_gradient_magnitude(P, X, Y, Z));
-        for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-        if ((threadIdx.x & 31) == 0) atomicMax(max_bits, b);
-    }
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (tx == 0 && best) atomicMax(out_bits, best);
 }
 
 __global__ void k_math_eval(int fn, int n, const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out)
@@ -405,20 +389,21 @@ cudaError_t er_launch_gradient_magnitude(const Params& P, uint16_t* gm, unsigned
     return cudaGetLastError();
 }
 
-cudaError_t er_launch_gradient_max(const Params& P, uint32_t* scratch, unsigned int* max_bits, cudaStream_t s)
+bool er_gradient_max_applies(const Params& P)
 {
-    const int nb[3] = { (P.res[0] + 7) / 8, (P.res[1] + 7) / 8, (P.res[2] + 7) / 8 };
-    const uint32_t total = (uint32_t)((size_t)nb[0] * nb[1] * nb[2]);
-    uint32_t *minmax = scratch, *bound = scratch + total, *list = scratch + 2 * (size_t)total, *top = scratch + 3 * (size_t)total, *count = top + 1;
-    const unsigned grid = (total + 255) / 256;
-    cudaError_t e = er_launch_brick_minmax(P.vox, P.res, 8, nb, minmax, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(top, 0, 2 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    k_gm_bound<<<grid, 256, 0, s>>>(P, minmax, nb[0], nb[1], nb[2], bound, top);
-    for (int round = 0; round < 2; round++) {
-        if (round && (e = cudaMemsetAsync(count, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
-        k_gm_select<<<grid, 256, 0, s>>>(bound, total, top, max_bits, round, list, count);
-        k_gm_bricks<<<152 * 4, 512, 0, s>>>(P, list, count, bound, nb[0], nb[1], max_bits);
-    }
+    /* the mean's argument: one spacing, weights within a tenth of a half, and grids within the launch limits */
+    const int most = P.res[0] > P.res[1] ? (P.res[0] > P.res[2] ? P.res[0] : P.res[2]) : (P.res[1] > P.res[2] ? P.res[1] : P.res[2]);
+    return P.spacing[0] == P.spacing[1] && P.spacing[1] == P.spacing[2] && P.spacing[0] > 0.0f && most <= 50000;
+}
+
+cudaError_t er_launch_gradient_max(const Params& P, int vmax, unsigned int* bits, cudaStream_t s)
+{
+    int most = P.res[0];
+    for (int i = 1; i < 3; i++) most = P.res[i] > most ? P.res[i] : most;
+    /* a lookup's local coordinate is off by a few ulps of the volume's extent, 1e-6 of it at most */
+    const float tol = 3.5f + 3e-6f * (float)most * (float)vmax;
+    const dim3 b(GM_X, GM_Y), g((P.res[0] + GM_X - 3) / (GM_X - 2), (P.res[1] + GM_Y - 3) / (GM_Y - 2), (P.res[2] + GM_Z - 1) / GM_Z);
+    k_gm_cells<false><<<g, b, 0, s>>>(P, tol, nullptr, bits + 1);
+    k_gm_cells<true><<<g, b, 0, s>>>(P, tol, bits + 1, bits);
     return cudaGetLastError();
 }

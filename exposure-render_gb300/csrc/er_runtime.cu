@@ -247,7 +247,6 @@ struct VolumeItem {
     int qb_nbx = 0;                /* quads in 8^3 bricks: bricks along x (0: x fastest) */
     unsigned long long qb_slab = 0;
     DevBuf<unsigned int> gm_max_bits;
-    DevBuf<uint32_t> gm_scratch;   /* er_launch_gradient_max */
     DevBuf<unsigned int> box_max;  /* largest voxel of an uploaded box */
     float gm_max = -1.0f;          /* lazily computed maximum gradient magnitude */
 };
@@ -2234,17 +2233,11 @@ ER_API er_status er_gradient_magnitude(int32_t volume_id, uint16_t* d_gm, float*
     erd::Params P;
     memset(&P, 0, sizeof(P));
     volume_geometry(v, P);
-    ER_CUDA(v.gm_max_bits.ensure(1));
+    ER_CUDA(v.gm_max_bits.ensure(2));
     cudaStream_t s = ctx().stream;
-    ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, sizeof(unsigned int), s));
-    const size_t bricks = (size_t)((P.res[0] + 7) / 8) * ((P.res[1] + 7) / 8) * ((P.res[2] + 7) / 8);
-    if (!d_gm && bricks < (1ull << 31) && v.gm_scratch.ensure(3 * bricks + 2) == cudaSuccess) {
-        /* the maximum alone: only bricks that can hold it */
-        ER_CUDA(er_launch_gradient_max(P, v.gm_scratch.p, v.gm_max_bits.p, s));
-    } else {
-        cudaGetLastError();
-        ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
-    }
+    ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, 2 * sizeof(unsigned int), s));
+    if (!d_gm && er_gradient_max_applies(P)) ER_CUDA(er_launch_gradient_max(P, (int)v.vmax, v.gm_max_bits.p, s));
+    else ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
     unsigned int bits = 0;
     ER_CUDA(cudaMemcpyAsync(&bits, v.gm_max_bits.p, sizeof(bits), cudaMemcpyDeviceToHost, s));
     ER_CUDA(cudaStreamSynchronize(s));

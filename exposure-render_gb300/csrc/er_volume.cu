@@ -181,12 +181,6 @@ static void launch_minmax(const uint16_t* vox, const int res[3], int B, const in
         k_brick_minmax<1><<<grid, BM_THREADS, 0, s>>>(vox, res[0], res[1], res[2], B, nb[0], nb[1], nb[2], xbricks, zbricks, xblocks, minmax);
 }
 
-cudaError_t er_launch_brick_minmax(const uint16_t* vox, const int res[3], int B, const int nb[3], uint32_t* minmax, cudaStream_t s)
-{
-    launch_minmax(vox, res, B, nb, minmax, s);
-    return cudaGetLastError();
-}
-
 __global__ void k_sample_voxels(const uint16_t* __restrict__ vox, size_t n, int step, uint16_t* __restrict__ out)
 {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
