@@ -155,8 +155,9 @@ struct WavefrontBuffers {
 };
 
 /* cuts the items of views (npix[v] * spp[v] each) into windows of whole
-   sample rows of at most window_cap items (one row at least) */
-void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, WavefrontPlan& plan);
+   sample rows of at most window_cap items (one row at least); a view starts a
+   window of its own when the open one has `apart` items (0: never) */
+void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, size_t apart, WavefrontPlan& plan);
 
 /* stage timing of the wavefront launches: 0 primary, 1 shade, 2 shadow,
    3 reduce; read returns the accumulated milliseconds and launch counts since
@@ -168,8 +169,9 @@ cudaError_t er_wavefront_profile_read(double* ms, int64_t* launches);
 /* one view with its parameters passed by value (no device tables) */
 cudaError_t er_launch_wavefront_one(const WfView& view, const WavefrontPlan& plan, const WavefrontBuffers& B, cudaStream_t s);
 
-/* many views: d_views / d_segs are the plan's tables in device memory */
-cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfSegment* d_segs, const WavefrontPlan& plan,
+/* many views: d_views / d_segs are the plan's tables in device memory,
+   host_views what d_views holds (but for `first`) */
+cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfView* host_views, const WfSegment* d_segs, const WavefrontPlan& plan,
                                       const WavefrontBuffers& B, cudaStream_t s);
 
 #endif

@@ -104,6 +104,11 @@ uint64_t fnv1a(uint64_t h, const void* data, size_t n)
 /* items of one wavefront window: 8M samples, 1.5 GB of queues */
 constexpr size_t kWindowCap = (size_t)8 << 20;
 
+/* a batch's next view starts a window of its own behind this many samples: a
+   window of one view runs the one-view kernels (er_launch_wavefront_batch),
+   some tenth faster, and its extra launches and tails cost about 40 us */
+constexpr size_t kWindowApart = (size_t)1 << 20;
+
 /* bricks of the march's empty-space map: 2^2 = 4 voxels a side */
 constexpr int kMarchBrickShift = 2;
 
@@ -861,7 +866,7 @@ er_status trace_sum(TracerItem& t, int spp, uint32_t view, uint32_t first, float
     }
     const int npix = t.W * t.H;
     WavefrontPlan plan;
-    er_wavefront_plan(&npix, &spp, 1, kWindowCap, plan);
+    er_wavefront_plan(&npix, &spp, 1, kWindowCap, 0, plan);
     WavefrontBuffers B;
     ER_CUDA(t.wf.ensure(plan, B));
     B.tune_primary = t.d.settings.tune_primary > 0 ? t.d.settings.tune_primary : 4;
@@ -946,7 +951,7 @@ er_status batch_plan(BatchItem& b)
         for (int u = 0; u < v; u++)
             if (b.host_views[(size_t)v].sum == b.host_views[(size_t)u].sum)
                 return fail(ER_ERR_INVALID_ARGUMENT, "batch views %d and %d share a sum buffer", u, v);
-    er_wavefront_plan(npix.data(), spp.data(), n, b.window_cap, b.plan);
+    er_wavefront_plan(npix.data(), spp.data(), n, b.window_cap, kWindowApart, b.plan);
     ER_CUDA(b.wf.ensure(b.plan, b.B));
     ER_CUDA(b.d_views.ensure((size_t)n));
     ER_CUDA(b.d_segs.ensure(b.plan.segs.size()));
@@ -996,7 +1001,7 @@ er_status batch_plan(BatchItem& b)
 /* the launch sequence of a batch: wavefront windows, display pass, bilateral */
 er_status batch_enqueue(BatchItem& b, cudaStream_t s)
 {
-    ER_CUDA(er_launch_wavefront_batch(b.d_views.p, b.d_segs.p, b.plan, b.B, s));
+    ER_CUDA(er_launch_wavefront_batch(b.d_views.p, b.host_views.data(), b.d_segs.p, b.plan, b.B, s));
     if (b.any_display) {
         ER_CUDA(er_launch_post_batch(b.d_views.p, (int)b.views.size(), b.max_w, b.max_h, s));
         for (const er_batch_view& bv : b.views) {

@@ -66,6 +66,15 @@ ER_D const WfView& view_of(const WfView* __restrict__ views, const WfView& one, 
     return views[v];
 }
 
+/* stream index of the view's first sample: er_batch_advance moves it in the
+   table, also for a window of a batch that passes its one view by value
+   (views: that view's entry; NULL for a launch without a table) */
+template <bool ONE>
+ER_D uint32_t first_of(const WfView* __restrict__ views, const WfView& V)
+{
+    return ONE && views ? views->first : V.first;
+}
+
 /* the pixel of slot j of a sample row: row by row, or (tile_order) in
    tiles of 32 pixels, row by row of tiles, so that a warp's 32 lanes trace a
    block of neighbouring pixels (tile_order 1: 8x4, 2: 4x8, 3: 16x2); a
@@ -135,9 +144,9 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary(const WfView* __restri
             const int s = sg.s0 + (int)(local / npix);
             const int pix = (int)slot_pixel(P, local % npix);
             const int x = pix % P.film[0], y = pix / P.film[0];
-            er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, V.first + (uint32_t)s, &rng.s0, &rng.s1);
+            er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s, &rng.s0, &rng.s1);
             ms.large_step(rng);
-            ms.stratify(P, V.view_id, (uint32_t)pix, V.first + (uint32_t)s);
+            ms.stratify(P, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s);
             const Ray R = sample_camera(P, x, y, ms.film_uv, ms.lens_uv);
             Event se0, se1;
             se0.type = 0; se0.valid = false; se0.T = 0.0f; se0.Le = C3(0, 0, 0);
@@ -294,7 +303,7 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary_pt(const WfView* __res
                 const uint32_t local = i - sg.offset;
                 const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
                 Rng r0;
-                const uint32_t sidx = V.first + (uint32_t)(sg.s0 + (int)(local / npix));
+                const uint32_t sidx = first_of<ONE>(views, V) + (uint32_t)(sg.s0 + (int)(local / npix));
                 const uint32_t pix = slot_pixel(P, local % npix);
                 er_seed_lanes(P.seed, V.view_id, pix, sidx, &r0.s0, &r0.s1);
                 Metro ms;
@@ -324,10 +333,10 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary_pt(const WfView* __res
                         const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
                         const int s = sg.s0 + (int)(local / npix);
                         const int pix = (int)slot_pixel(P, local % npix);
-                        er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, V.first + (uint32_t)s, &rng.s0, &rng.s1);
+                        er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s, &rng.s0, &rng.s1);
                         Metro ms;
                         ms.large_step(rng);
-                        ms.stratify(P, V.view_id, (uint32_t)pix, V.first + (uint32_t)s);
+                        ms.stratify(P, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s);
                         R = sample_camera(P, pix % P.film[0], pix / P.film[0], ms.film_uv, ms.lens_uv);
                         delta_begin(P, R, rng, k, ms.tau_u);
                         hit = false;
@@ -902,7 +911,7 @@ __global__ void k_wf_reduce(const WfView* __restrict__ views, const WfSegment* _
    and profiler, er_wavefront_batch.cu (WF_BATCH_UNIT) the batch launches. */
 #ifndef WF_BATCH_UNIT
 
-void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, WavefrontPlan& plan)
+void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, size_t apart, WavefrontPlan& plan)
 {
     plan.segs.clear();
     plan.window_first.clear();
@@ -915,7 +924,7 @@ void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t wind
         if (npix[v] > plan.max_npix) plan.max_npix = npix[v];
         int s = 0;
         while (s < spp[v]) {
-            if (plan.window_first.empty() || used + (size_t)npix[v] > window_cap) {
+            if (plan.window_first.empty() || used + (size_t)npix[v] > window_cap || (s == 0 && apart && used >= apart)) {
                 plan.window_first.push_back((int)plan.segs.size());
                 plan.window_items.push_back(0);
                 used = 0;
@@ -1012,143 +1021,148 @@ int sm_count()
    values run 4) */
 int narrow_minb(int m) { return (m == 2 || m == 3 || m == 6) ? m : 4; }
 
+/* the stages of window w: segments [s0, s1) of the plan; ONE: a window of one
+   view, `one`, whose table entry (or NULL) is d_views */
 template <bool ONE>
-cudaError_t launch_windows(const WfView* d_views, const WfSegment* d_segs, const WfView& one, const WavefrontPlan& plan,
-                           const WavefrontBuffers& B, cudaStream_t s)
+cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const WfView& one, const WavefrontPlan& plan, int w, int s0, int s1,
+                          const WavefrontBuffers& B, cudaStream_t s)
 {
     const int sm = sm_count();
-    const int nw = (int)plan.window_first.size();
-    for (int w = 0; w < nw; w++) {
-        const int s0 = plan.window_first[w];
-        const int s1 = (w + 1 < nw) ? plan.window_first[w + 1] : (int)plan.segs.size();
-        const int nseg = s1 - s0;
-        const uint32_t items = plan.window_items[w];
-        const WfSegment* dseg = ONE ? nullptr : d_segs + s0;
-        const WfSegment one_seg = plan.segs[s0];
-        float4* p_in = B.partial + (size_t)((w + 1) & 1) * plan.max_npix;
-        float4* p_out = B.partial + (size_t)(w & 1) * plan.max_npix;
-        cudaError_t e = cudaMemsetAsync(B.counters, 0, 6 * sizeof(uint32_t), s);
-        if (e != cudaSuccess) return e;
-        const uint32_t g1 = (items + 255) / 256 < (uint32_t)sm * 64 ? (items + 255) / 256 : (uint32_t)sm * 64;
-        cudaEvent_t t0 = wf_stage_begin(s);
+    const int nseg = s1 - s0;
+    const uint32_t items = plan.window_items[w];
+    const WfSegment one_seg = plan.segs[s0];
+    float4* p_in = B.partial + (size_t)((w + 1) & 1) * plan.max_npix;
+    float4* p_out = B.partial + (size_t)(w & 1) * plan.max_npix;
+    cudaError_t e = cudaMemsetAsync(B.counters, 0, 6 * sizeof(uint32_t), s);
+    if (e != cudaSuccess) return e;
+    const uint32_t g1 = (items + 255) / 256 < (uint32_t)sm * 64 ? (items + 255) / 256 : (uint32_t)sm * 64;
+    cudaEvent_t t0 = wf_stage_begin(s);
 #define ER_PRIMARY(M, O, F) k_wf_primary<M, ONE, O, F><<<g1, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters)
 #define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2, B.cross_eighths, B.collide_eighths, B.gate_primary)
-        if (B.pt_primary) {
-            /* delta tracking: persistent lanes, one resident wave */
-            if (B.objects) ER_PRIMARY_PT(4, true);
-            else {
-                switch (narrow_minb(B.tune_primary)) {
-                case 2: ER_PRIMARY_PT(2, false); break;
-                case 3: ER_PRIMARY_PT(3, false); break;
-                case 6: ER_PRIMARY_PT(6, false); break;
-                default: ER_PRIMARY_PT(4, false); break;
-                }
-            }
-        } else if (B.objects) {
-            if (B.free_flight == WF_DELTA) ER_PRIMARY(4, true, WF_DELTA);
-            else if (B.free_flight == WF_MARCH) ER_PRIMARY(4, true, WF_MARCH);
-            else ER_PRIMARY(4, true, WF_MIXED);
-        } else if (B.free_flight == WF_DELTA) {
+    if (B.pt_primary) {
+        /* delta tracking: persistent lanes, one resident wave */
+        if (B.objects) ER_PRIMARY_PT(4, true);
+        else {
             switch (narrow_minb(B.tune_primary)) {
-            case 2: ER_PRIMARY(2, false, WF_DELTA); break;
-            case 3: ER_PRIMARY(3, false, WF_DELTA); break;
-            case 6: ER_PRIMARY(6, false, WF_DELTA); break;
-            default: ER_PRIMARY(4, false, WF_DELTA); break;
+            case 2: ER_PRIMARY_PT(2, false); break;
+            case 3: ER_PRIMARY_PT(3, false); break;
+            case 6: ER_PRIMARY_PT(6, false); break;
+            default: ER_PRIMARY_PT(4, false); break;
             }
-        } else if (B.free_flight == WF_MARCH) {
-            switch (B.tune_primary) {
-            case 2: ER_PRIMARY(2, false, WF_MARCH); break;
-            case 3: ER_PRIMARY(3, false, WF_MARCH); break;
-            case 6: ER_PRIMARY(6, false, WF_MARCH); break;
-            case 8: ER_PRIMARY(8, false, WF_MARCH); break;
-            default: ER_PRIMARY(4, false, WF_MARCH); break;
-            }
-        } else ER_PRIMARY(4, false, WF_MIXED);
+        }
+    } else if (B.objects) {
+        if (B.free_flight == WF_DELTA) ER_PRIMARY(4, true, WF_DELTA);
+        else if (B.free_flight == WF_MARCH) ER_PRIMARY(4, true, WF_MARCH);
+        else ER_PRIMARY(4, true, WF_MIXED);
+    } else if (B.free_flight == WF_DELTA) {
+        switch (narrow_minb(B.tune_primary)) {
+        case 2: ER_PRIMARY(2, false, WF_DELTA); break;
+        case 3: ER_PRIMARY(3, false, WF_DELTA); break;
+        case 6: ER_PRIMARY(6, false, WF_DELTA); break;
+        default: ER_PRIMARY(4, false, WF_DELTA); break;
+        }
+    } else if (B.free_flight == WF_MARCH) {
+        switch (B.tune_primary) {
+        case 2: ER_PRIMARY(2, false, WF_MARCH); break;
+        case 3: ER_PRIMARY(3, false, WF_MARCH); break;
+        case 6: ER_PRIMARY(6, false, WF_MARCH); break;
+        case 8: ER_PRIMARY(8, false, WF_MARCH); break;
+        default: ER_PRIMARY(4, false, WF_MARCH); break;
+        }
+    } else ER_PRIMARY(4, false, WF_MIXED);
 #undef ER_PRIMARY_PT
 #undef ER_PRIMARY
-        wf_stage_end(t0, 0, s);
-        t0 = wf_stage_begin(s);
+    wf_stage_end(t0, 0, s);
+    t0 = wf_stage_begin(s);
 #define ER_SHADE(M, O) k_wf_shade<ONE, M, O><<<sm * 16, 128, 0, s>>>(d_views, one, B.events, B.counters, B.results, B.jobs, B.counters + 1)
 #define ER_SORTED(M) k_wf_shade_sorted<ONE, M><<<sm * 16, 128, 0, s>>>(d_views, one, B.records, cap, B.counters + 4, B.results, B.jobs, \
-                                                                    B.counters + 1)
-        const uint32_t cap = (uint32_t)plan.max_items;
-        if (B.objects) ER_SHADE(2, true);
-        else if (B.sort_shade) {
-            /* shader switch mixing BRDF and phase events: classify, then shade by shader */
-            k_wf_classify<ONE><<<sm * 16, 128, 0, s>>>(d_views, one, B.events, B.counters, B.results, B.records, cap, B.counters + 4);
-            switch (B.tune_shade) {
-            case 3: ER_SORTED(3); break;
-            case 4: ER_SORTED(4); break;
-            case 6: ER_SORTED(6); break;
-            default: ER_SORTED(2); break;
-            }
-        } else switch (B.tune_shade) {
-        case 3: ER_SHADE(3, false); break;
-        case 4: ER_SHADE(4, false); break;
-        case 6: ER_SHADE(6, false); break;
-        default: ER_SHADE(2, false); break;
+                                                                B.counters + 1)
+    const uint32_t cap = (uint32_t)plan.max_items;
+    if (B.objects) ER_SHADE(2, true);
+    else if (B.sort_shade) {
+        /* shader switch mixing BRDF and phase events: classify, then shade by shader */
+        k_wf_classify<ONE><<<sm * 16, 128, 0, s>>>(d_views, one, B.events, B.counters, B.results, B.records, cap, B.counters + 4);
+        switch (B.tune_shade) {
+        case 3: ER_SORTED(3); break;
+        case 4: ER_SORTED(4); break;
+        case 6: ER_SORTED(6); break;
+        default: ER_SORTED(2); break;
         }
+    } else switch (B.tune_shade) {
+    case 3: ER_SHADE(3, false); break;
+    case 4: ER_SHADE(4, false); break;
+    case 6: ER_SHADE(6, false); break;
+    default: ER_SHADE(2, false); break;
+    }
 #undef ER_SORTED
 #undef ER_SHADE
-        wf_stage_end(t0, 1, s);
-        t0 = wf_stage_begin(s);
+    wf_stage_end(t0, 1, s);
+    t0 = wf_stage_begin(s);
 #define ER_SHADOW(M, O, F) k_wf_shadow<M, ONE, O, F><<<sm * 8, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results)
 #define ER_SHADOW_PT(M, O) k_wf_shadow_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.cross_eighths, B.collide_eighths, B.gate_shadow)
-        if (B.pt_shadow) {
-            /* ratio-tracked shadows: persistent lanes, one resident wave */
-            if (B.objects) ER_SHADOW_PT(4, true);
-            else {
-                switch (narrow_minb(B.tune_shadow)) {
-                case 2: ER_SHADOW_PT(2, false); break;
-                case 3: ER_SHADOW_PT(3, false); break;
-                case 6: ER_SHADOW_PT(6, false); break;
-                default: ER_SHADOW_PT(4, false); break;
-                }
-            }
-        } else if (B.objects) {
-            if (B.free_flight == WF_DELTA) ER_SHADOW(4, true, WF_DELTA);
-            else if (B.free_flight == WF_MARCH) ER_SHADOW(4, true, WF_MARCH);
-            else ER_SHADOW(4, true, WF_MIXED);
-        } else if (B.free_flight == WF_DELTA) {
+    if (B.pt_shadow) {
+        /* ratio-tracked shadows: persistent lanes, one resident wave */
+        if (B.objects) ER_SHADOW_PT(4, true);
+        else {
             switch (narrow_minb(B.tune_shadow)) {
-            case 2: ER_SHADOW(2, false, WF_DELTA); break;
-            case 3: ER_SHADOW(3, false, WF_DELTA); break;
-            case 6: ER_SHADOW(6, false, WF_DELTA); break;
-            default: ER_SHADOW(4, false, WF_DELTA); break;
+            case 2: ER_SHADOW_PT(2, false); break;
+            case 3: ER_SHADOW_PT(3, false); break;
+            case 6: ER_SHADOW_PT(6, false); break;
+            default: ER_SHADOW_PT(4, false); break;
             }
-        } else if (B.free_flight == WF_MARCH) {
-            switch (B.tune_shadow) {
-            case 2: ER_SHADOW(2, false, WF_MARCH); break;
-            case 3: ER_SHADOW(3, false, WF_MARCH); break;
-            case 6: ER_SHADOW(6, false, WF_MARCH); break;
-            case 8: ER_SHADOW(8, false, WF_MARCH); break;
-            default: ER_SHADOW(4, false, WF_MARCH); break;
-            }
-        } else ER_SHADOW(4, false, WF_MIXED);
+        }
+    } else if (B.objects) {
+        if (B.free_flight == WF_DELTA) ER_SHADOW(4, true, WF_DELTA);
+        else if (B.free_flight == WF_MARCH) ER_SHADOW(4, true, WF_MARCH);
+        else ER_SHADOW(4, true, WF_MIXED);
+    } else if (B.free_flight == WF_DELTA) {
+        switch (narrow_minb(B.tune_shadow)) {
+        case 2: ER_SHADOW(2, false, WF_DELTA); break;
+        case 3: ER_SHADOW(3, false, WF_DELTA); break;
+        case 6: ER_SHADOW(6, false, WF_DELTA); break;
+        default: ER_SHADOW(4, false, WF_DELTA); break;
+        }
+    } else if (B.free_flight == WF_MARCH) {
+        switch (B.tune_shadow) {
+        case 2: ER_SHADOW(2, false, WF_MARCH); break;
+        case 3: ER_SHADOW(3, false, WF_MARCH); break;
+        case 6: ER_SHADOW(6, false, WF_MARCH); break;
+        case 8: ER_SHADOW(8, false, WF_MARCH); break;
+        default: ER_SHADOW(4, false, WF_MARCH); break;
+        }
+    } else ER_SHADOW(4, false, WF_MIXED);
 #undef ER_SHADOW_PT
 #undef ER_SHADOW
-        wf_stage_end(t0, 2, s);
-        int max_npix = 0;
-        for (int g = s0; g < s1; g++) {
-            const int np = plan.view_npix[plan.segs[g].view];
-            if (np > max_npix) max_npix = np;
-        }
-        t0 = wf_stage_begin(s);
-        k_wf_reduce<ONE><<<dim3((max_npix + 255) / 256, ONE ? 1 : nseg), 256, 0, s>>>(d_views, dseg, one, one_seg, B.results, p_in, p_out);
-        wf_stage_end(t0, 3, s);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+    wf_stage_end(t0, 2, s);
+    int max_npix = 0;
+    for (int g = s0; g < s1; g++) {
+        const int np = plan.view_npix[plan.segs[g].view];
+        if (np > max_npix) max_npix = np;
     }
-    return cudaSuccess;
+    t0 = wf_stage_begin(s);
+    k_wf_reduce<ONE><<<dim3((max_npix + 255) / 256, ONE ? 1 : nseg), 256, 0, s>>>(d_views, dseg, one, one_seg, B.results, p_in, p_out);
+    wf_stage_end(t0, 3, s);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
 #ifndef WF_BATCH_UNIT
 
+/* one window of one view with its parameters by value */
+cudaError_t wf_launch_window_one(const WfView* d_view, const WfView& view, const WavefrontPlan& plan, int w, int seg,
+                                 const WavefrontBuffers& B, cudaStream_t s)
+{
+    return launch_window<true>(d_view, nullptr, view, plan, w, seg, seg + 1, B, s);
+}
+
 cudaError_t er_launch_wavefront_one(const WfView& view, const WavefrontPlan& plan, const WavefrontBuffers& B, cudaStream_t s)
 {
-    return launch_windows<true>(nullptr, nullptr, view, plan, B, s);
+    for (int w = 0; w < (int)plan.window_first.size(); w++) {
+        const cudaError_t e = wf_launch_window_one(nullptr, view, plan, w, plan.window_first[w], B, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 void er_wavefront_profile_enable(bool on)
@@ -1185,12 +1199,28 @@ cudaError_t er_wavefront_profile_read(double* ms, int64_t* launches)
 
 #else
 
-cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfSegment* d_segs, const WavefrontPlan& plan,
+cudaError_t wf_launch_window_one(const WfView* d_view, const WfView& view, const WavefrontPlan& plan, int w, int seg,
+                                 const WavefrontBuffers& B, cudaStream_t s);
+
+/* A window that holds one view runs the one-view kernels, whose parameters
+   come from the constant bank instead of loads from the table at every brick
+   and lookup: a batch of one view of the c3 volumes took 6.15 against 5.32 ms
+   (64x96x96) and 3.38 against 2.93 ms (256x384x384) in the primary stage. */
+cudaError_t er_launch_wavefront_batch(const WfView* d_views, const WfView* host_views, const WfSegment* d_segs, const WavefrontPlan& plan,
                                       const WavefrontBuffers& B, cudaStream_t s)
 {
     WfView unused;
     memset(&unused, 0, sizeof(unused));
-    return launch_windows<false>(d_views, d_segs, unused, plan, B, s);
+    const int nw = (int)plan.window_first.size();
+    for (int w = 0; w < nw; w++) {
+        const int s0 = plan.window_first[w];
+        const int s1 = (w + 1 < nw) ? plan.window_first[w + 1] : (int)plan.segs.size();
+        const int v = plan.segs[s0].view;
+        const cudaError_t e = s1 - s0 == 1 ? wf_launch_window_one(d_views + v, host_views[v], plan, w, s0, B, s)
+                                           : launch_window<false>(d_views, d_segs + s0, unused, plan, w, s0, s1, B, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 #endif
