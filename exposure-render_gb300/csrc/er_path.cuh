@@ -1289,7 +1289,7 @@ ER_D float dda_majorant(const Params& P, const Dda& d)
 
 /* Empty-space jump.  An empty brick of the tracker's majorant grid holds
    -k, k the Chebyshev distance in bricks to the nearest non-empty brick
-   (er_volume.cu k_skip_pass), so the cube of bricks within k-1 of it is
+   (er_volume.cu launch_skip), so the cube of bricks within k-1 of it is
    empty: nothing is drawn and tau is unchanged while the ray crosses it.
    dda_jump moves the DDA to the cube's exit in one step.  The exit face of
    each axis is k-1 bricks past its next face (time next + (k-1) * delta);

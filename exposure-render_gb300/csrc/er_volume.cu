@@ -10,7 +10,7 @@
  *   k_rmq          : sparse table of running maxima over the sigma table
  *                    (sigma[I] = DensityScale * Opacity(I)).
  *   k_majorant     : majorant[brick] = DensityScale * max sigma[lo..hi].
- *   k_skip_pass    : distances to the nearest non-empty brick.
+ *   k_skip_x, _yz  : distances to the nearest non-empty brick.
  *   k_occupancy    : the empty bricks of the fixed-step march.
  *
  * A lookup inside a brick is a truncated trilinear blend of voxels in
@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <cstdio>
+#include <type_traits>
 
 #include "er_capi.h"
 #include "er_kernels.h"
@@ -40,7 +41,7 @@
    range.  One warp per brick, which it replaces, put 5 voxels of a row on 32
    lanes at 4^3 bricks and took 3.79 ms at 512^3; an edit of the transfer
    function of that volume with a one-sample picture went from 5.8 to 1.9 ms
-   with this kernel, k_rmq and the outward k_skip_pass. */
+   with this kernel, k_rmq and outward distance passes. */
 #define BM_THREADS 160
 
 template <int VEC>
@@ -207,62 +208,102 @@ cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, con
    non-empty bricks q of max_a |b_a - q_a| (Chebyshev distance in bricks),
    capped at ER_SKIP_CAP; computed exactly by three 1D passes (x: nearest
    non-empty along the row; y and z: min over offsets of max(offset, previous
-   pass)).  A pass looks outwards from its brick and stops at the first
-   offset that is no smaller than the best distance so far, so its length is
-   the distance it finds, not the 63 bricks of the cap's window (94 us a pass
-   at 128^3 bricks of a half-filled volume).  For the delta trackers
-   (k_skip_pass<0>) a brick is empty where its majorant is not positive, and
-   the last pass writes -dist into the empty bricks of the majorant grid; for
-   the fixed-step march (k_skip_pass<1>) the x pass reads the occupancy bytes
-   of k_occupancy and the last pass writes dist (0: not empty) as bytes.  A
-   ray in a brick at distance dist knows every brick within dist-1 of it is
-   empty too (er_path.cuh dda_jump, march_skip). */
+   pass)).  A ray in a brick at distance dist knows every brick within dist-1
+   of it is empty too (er_path.cuh dda_jump, march_skip).
+
+   k_skip_x: a warp takes 32 bricks of a row; the occupancy of them and of the
+   32 on either side are three ballots, and the nearest set bits give the
+   distance (below 32, so the neighbours' words suffice).  k_skip_yz looks
+   outwards and stops at the first offset that is no smaller than the best
+   distance so far; four bricks of a row to a thread where the rows are whole
+   words.  Loops over the 63 bricks of the cap's window took 94 us a pass at
+   128^3 bricks, outward ones, a brick to a thread, 53 us. */
 #define ER_SKIP_CAP 32
 
+/* MARCH: `occ` holds k_occupancy's bytes (0: not empty); else a brick is empty
+   where its majorant is not positive */
 template <int MARCH>
-__global__ void k_skip_pass(const float* __restrict__ majorant, const uint8_t* __restrict__ in, uint8_t* __restrict__ out,
-                            float* __restrict__ majorant_out, int axis, int nbx, int nby, int nbz, long long total)
+__global__ void __launch_bounds__(256) k_skip_x(const float* __restrict__ majorant, const uint8_t* __restrict__ occ,
+                                                uint8_t* __restrict__ out, int nbx, long long rows)
 {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int n = axis == 0 ? nbx : (axis == 1 ? nby : nbz);
-        const long long step = axis == 0 ? 1 : (axis == 1 ? (long long)nbx : (long long)nbx * nby);
-        const int c = (int)((i / step) % n);
-        auto at = [&](long long j) -> int {
-            if (!MARCH && axis == 0) return majorant[j] > 0.0f ? 0 : ER_SKIP_CAP;
-            return (int)in[j];
+    const int lane = threadIdx.x & 31;
+    const int words = (nbx + 31) / 32;
+    const long long total = rows * words, stride = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total; w += stride) {
+        const long long row = (w / words) * nbx;
+        const int x = (int)(w % words) * 32 + lane;
+        auto full = [&](int c) -> bool {
+            if (c < 0 || c >= nbx) return false;
+            return MARCH ? occ[row + c] == 0 : majorant[row + c] > 0.0f;
         };
-        int best = at(i);
-        for (int o = 1; o < best; o++) {
-            if (c - o >= 0) {
-                const int v = at(i - o * step);
-                const int d = v > o ? v : o;
-                best = d < best ? d : best;
-            }
-            if (c + o < n) {
-                const int v = at(i + o * step);
-                const int d = v > o ? v : o;
-                best = d < best ? d : best;
-            }
-        }
-        if (MARCH || axis < 2) out[i] = (uint8_t)best;
-        else if (!(majorant_out[i] > 0.0f)) majorant_out[i] = -(float)best;
+        const unsigned l = __ballot_sync(0xffffffffu, full(x - 32)), m = __ballot_sync(0xffffffffu, full(x)),
+                       r = __ballot_sync(0xffffffffu, full(x + 32));
+        if (x >= nbx) continue;
+        /* bits of the bricks at and right of x (bit 0: x), and at and left of it (bit 31: x) */
+        const unsigned right = __funnelshift_r(m, r, lane), left = __funnelshift_l(l, m, 31 - lane);
+        const int dr = right ? __ffs(right) - 1 : ER_SKIP_CAP, dl = left ? __clz(left) : ER_SKIP_CAP;
+        out[row + x] = (uint8_t)(dr < dl ? dr : dl);
     }
+}
+
+/* VEC bricks of a row per thread; the last pass of the delta trackers writes
+   -dist into the empty bricks of the majorant grid, the march's its bytes */
+template <int VEC>
+__global__ void __launch_bounds__(256) k_skip_yz(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, float* __restrict__ majorant_out,
+                                                 int n, long long step, long long total)
+{
+    typedef typename std::conditional<VEC == 4, uint32_t, uint8_t>::type Word;
+    const long long stride = (long long)gridDim.x * blockDim.x * VEC;
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC; i < total; i += stride) {
+        const int c = (int)((i / step) % n);
+        uint32_t best = *(const Word*)(in + i);
+        /* largest of the VEC distances bounds the offsets to look at */
+        for (int o = 1;; o++) {
+            uint32_t most = best & 0xffu;
+            if (VEC == 4) most = max(max(most, (best >> 8) & 0xffu), max((best >> 16) & 0xffu, best >> 24));
+            if ((uint32_t)o >= most) break;
+            const uint32_t oo = (uint32_t)o * (VEC == 4 ? 0x01010101u : 1u);
+            if (c - o >= 0) best = __vminu4(best, __vmaxu4((uint32_t) * (const Word*)(in + i - o * step), oo));
+            if (c + o < n) best = __vminu4(best, __vmaxu4((uint32_t) * (const Word*)(in + i + o * step), oo));
+        }
+        if (!majorant_out) {
+            *(Word*)(out + i) = (Word)best;
+        } else {
+#pragma unroll
+            for (int k = 0; k < VEC; k++)
+                if (!(majorant_out[i + k] > 0.0f)) majorant_out[i + k] = -(float)((best >> (8 * k)) & 0xffu);
+        }
+    }
+}
+
+static cudaError_t launch_skip(int march, float* majorant, uint8_t* occ, const int nb[3], uint8_t* tmp, cudaStream_t s)
+{
+    const long long total = (long long)nb[0] * nb[1] * nb[2], rows = (long long)nb[1] * nb[2];
+    const long long words = rows * ((nb[0] + 31) / 32);
+    auto grid = [](long long threads) { const long long b = (threads + 255) / 256; return (unsigned)(b < 65536 ? b : 65536); };
+    uint8_t *px = tmp, *py = tmp + total;
+    /* whole words: rows of a multiple of four bricks, and aligned maps */
+    const bool vec = (nb[0] & 3) == 0 && (((uintptr_t)px | (uintptr_t)py | (uintptr_t)occ) & 3u) == 0;
+    if (march) k_skip_x<1><<<grid(words * 32), 256, 0, s>>>(nullptr, occ, px, nb[0], rows);
+    else k_skip_x<0><<<grid(words * 32), 256, 0, s>>>(majorant, nullptr, px, nb[0], rows);
+    float* mj = march ? nullptr : majorant;
+    if (vec) {
+        k_skip_yz<4><<<grid(total / 4), 256, 0, s>>>(px, py, nullptr, nb[1], nb[0], total);
+        k_skip_yz<4><<<grid(total / 4), 256, 0, s>>>(py, occ, mj, nb[2], rows / nb[2] * nb[0], total);
+    } else {
+        k_skip_yz<1><<<grid(total), 256, 0, s>>>(px, py, nullptr, nb[1], nb[0], total);
+        k_skip_yz<1><<<grid(total), 256, 0, s>>>(py, occ, mj, nb[2], rows / nb[2] * nb[0], total);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t er_launch_empty_skip(float* majorant, const int nb[3], uint8_t* tmp, cudaStream_t s)
 {
-    const long long total = (long long)nb[0] * nb[1] * nb[2];
-    const long long want = (total + 255) / 256;
-    const unsigned blocks = (unsigned)(want < 65536 ? want : 65536);
-    k_skip_pass<0><<<blocks, 256, 0, s>>>(majorant, nullptr, tmp, nullptr, 0, nb[0], nb[1], nb[2], total);
-    k_skip_pass<0><<<blocks, 256, 0, s>>>(nullptr, tmp, tmp + total, nullptr, 1, nb[0], nb[1], nb[2], total);
-    k_skip_pass<0><<<blocks, 256, 0, s>>>(nullptr, tmp + total, nullptr, majorant, 2, nb[0], nb[1], nb[2], total);
-    return cudaGetLastError();
+    return launch_skip(0, majorant, nullptr, nb, tmp, s);
 }
 
 /* The empty-space map of the fixed-step march: dist bytes of bricks of
-   2^shift voxels a side (k_skip_pass<1>).  A brick is empty when sigma is
+   2^shift voxels a side (launch_skip).  A brick is empty when sigma is
    exactly zero (of either sign) at every intensity a lookup in it can have,
    lo - 3 .. hi (each of the blend's three truncated lerps can round to one
    below its smaller end): a step there adds nothing to the march's sum, so
@@ -309,14 +350,10 @@ cudaError_t er_launch_march_map(const uint16_t* vox, const int res[3], int shift
 {
     const long long total = (long long)nb[0] * nb[1] * nb[2];
     const long long want = (total + 255) / 256;
-    const unsigned blocks = (unsigned)(want < 65536 ? want : 65536);
     launch_minmax(vox, res, 1 << shift, nb, minmax, s);
     k_nonzero_prefix<<<1, 1024, 0, s>>>(sigma, count, n);
     k_occupancy<<<(unsigned)want, 256, 0, s>>>(minmax, count, n, occ, total);
-    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, occ, tmp, nullptr, 0, nb[0], nb[1], nb[2], total);
-    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, tmp, tmp + total, nullptr, 1, nb[0], nb[1], nb[2], total);
-    k_skip_pass<1><<<blocks, 256, 0, s>>>(nullptr, tmp + total, occ, nullptr, 2, nb[0], nb[1], nb[2], total);
-    return cudaGetLastError();
+    return launch_skip(1, nullptr, occ, nb, tmp, s);
 }
 
 /* corner quads: for voxel (x, y, z) the intensities at (x, y), (x+1, y),
