@@ -16,12 +16,16 @@
 
 namespace erd {
 
-/* steps of the march in flight (march): in the one-kernel paths, whose
-   registers hold the whole path, 2 (the frame of the 512^3 shells at 1, 2, 4
-   and 8: 3.1, 2.5, 2.8, 3.8 ms); in the wavefront's stages 4 (primary and
-   shadow stage of the 128^3 blobs at 1, 2 and 4: 3.63 and 2.43, 3.37 and 2.21,
-   3.26 and 2.12 ms) */
+/* steps of the march in flight (march).  One-kernel paths, whose registers
+   hold the whole path: 2 where warps fill the SMs (the frame of the 512^3
+   shells at 1024^2 with 1, 2, 4 and 8: 3.1, 2.5, 2.8, 3.8 ms), 4 where a film
+   has too few pixels for that and a lane's own latency is the frame's (two
+   320x240 frames of the objects scene with 2, 3 and 4: 904, 870, 858 us; one of
+   359x404 of a 72x86x50 volume: 384, 360, 349).
+   The wavefront's stages: 4 (primary and shadow stage of the 128^3 blobs with
+   1, 2 and 4: 3.63 and 2.43, 3.37 and 2.21, 3.26 and 2.12 ms). */
 #define ER_K_ONE 2
+#define ER_K_FEW 4
 #define ER_K_PRIMARY 4
 #define ER_K_SHADOW 4
 
@@ -1693,6 +1697,7 @@ ER_COLD v3 sample_bsdf_dir(const Shader& sh, v3 Wo, const Metro& ms)
 /* EstimateDirectLight - Source/transport.h:58-113: the live light-sampling
    half (mis 0, march), or both halves with power-heuristic weights (mis 1),
    with the ratio-tracked transmittance under delta tracking */
+template <int K>
 ER_D c3 estimate_direct_light(const Params& P, const Light& L, int slot, const Metro& ms, const Event& SE, Rng& rng,
                               const Shader& sh)
 {
@@ -1705,7 +1710,7 @@ ER_D c3 estimate_direct_light(const Params& P, const Light& L, int slot, const M
     const bool delta = P.free_flight == 1;
     const float BsdfPdf = full ? mis_bsdf_pdf(sh, SE.Wo, Wi) : shader_pdf(sh, SE.Wo, Wi);
     if (!full && !delta) {
-        if (!cblack(Li) && !cblack(F) && BsdfPdf > 0.0f && visibility<true, WF_MIXED, ER_K_ONE>(P, SE.P, SS.P, rng) > 0.0f) {
+        if (!cblack(Li) && !cblack(F) && BsdfPdf > 0.0f && visibility<true, WF_MIXED, K>(P, SE.P, SS.P, rng) > 0.0f) {
             const float LightPdf = vlen2(vsub(SE.P, SS.P)) / (vabsdot(SS.N, vneg(Wi)) * L.area);
             const float Weight = power_heuristic(LightPdf, BsdfPdf);
             if (sh.type == 0) Ld = cadd(Ld, cscale(cmul(F, Li), vabsdot(Wi, SE.N) * Weight / LightPdf));
@@ -1714,7 +1719,7 @@ ER_D c3 estimate_direct_light(const Params& P, const Light& L, int slot, const M
         return Ld;
     }
     if (!cblack(Li) && !cblack(F) && BsdfPdf > 0.0f) {
-        const float Tr = visibility<true, WF_MIXED, ER_K_ONE>(P, SE.P, SS.P, rng);
+        const float Tr = visibility<true, WF_MIXED, K>(P, SE.P, SS.P, rng);
         if (Tr > 0.0f) {
             const float LightPdf = vlen2(vsub(SE.P, SS.P)) / (vabsdot(SS.N, vneg(Wi)) * L.area);
             c3 c;
@@ -1748,7 +1753,7 @@ ER_D c3 estimate_direct_light(const Params& P, const Light& L, int slot, const M
     if (!SE2.valid || P.light_ids[hit] != P.light_ids[slot]) return Ld;
     SE2.Le = light_emission(P, P.lights[hit], lh);
     if (cblack(SE2.Le)) return Ld;
-    const float Tr = visibility<true, WF_MIXED, ER_K_ONE>(P, SE.P, SE2.P, rng);
+    const float Tr = visibility<true, WF_MIXED, K>(P, SE.P, SE2.P, rng);
     if (Tr > 0.0f) {
         const float LightPdf = vlen2(vsub(SE.P, SE2.P)) / (vabsdot(SE2.N, vneg(Wb)) * L.area);
         const float w = power_heuristic(pb, LightPdf);
@@ -1775,6 +1780,7 @@ ER_D void object_shader(const Params& P, const Event& SE, const ObjHit& hit, Sha
 }
 
 /* UniformSampleOneLight - Source/transport.h:115-156 (volume and object events) */
+template <int K>
 ER_D c3 uniform_sample_one_light(const Params& P, const Event& SE, Rng& rng, const Metro& ms, const ObjHit& hit)
 {
     c3 Ld = C3(0, 0, 0);
@@ -1793,7 +1799,7 @@ ER_D c3 uniform_sample_one_light(const Params& P, const Event& SE, Rng& rng, con
         const int type = P.apply_shading_type ? select_shader_type(P, SE, I, rng) : 0;
         shader_init(sh, type, SE.N, SE.Wo, tf.Kd, tf.Ks, P.volume_ior, tf.exponent);
     }
-    Ld = cadd(Ld, estimate_direct_light(P, L, idx, ms, SE, rng, sh));
+    Ld = cadd(Ld, estimate_direct_light<K>(P, L, idx, ms, SE, rng, sh));
     return cscale(Ld, (float)P.light_count);
 }
 
@@ -1820,6 +1826,7 @@ ER_D Ray sample_camera(const Params& P, int u, int v, v2 film_uv, v2 lens_uv)
 /* SingleScattering - Source/singlescattering.h:76-102.  `sample` >= 0 marks
    sample `sample` of view `view` of a multi-sample render (stratified light
    samples when enabled); -1 a frame of the reference's pipeline. */
+template <int K>
 ER_D float4 single_scattering(const Params& P, int x, int y, Rng& rng, uint32_t view = 0, int64_t sample = -1)
 {
     c3 Lv = C3(0, 0, 0);
@@ -1836,7 +1843,7 @@ ER_D float4 single_scattering(const Params& P, int x, int y, Rng& rng, uint32_t 
     ObjHit hit;
     hit.UV.x = 0.0f; hit.UV.y = 0.0f; hit.id = 0;
     if (P.free_flight == 1) sample_volume_delta(P, R, rng, se0, ms.tau_u);
-    else sample_volume<true, ER_K_ONE>(P, R, rng, se0);
+    else sample_volume<true, K>(P, R, rng, se0);
     int lslot = -1;
     LightHit lh;
     intersect_lights_geom(P, R, se1, true, lslot, lh, se0.valid ? event_end(se0.T) : FLT_MAX);
@@ -1847,9 +1854,9 @@ ER_D float4 single_scattering(const Params& P, int x, int y, Rng& rng, uint32_t 
     if (se1.valid && se1.T < T) { SE = se1; T = se1.T; }
     if (se2.valid && se2.T < T) { SE = se2; T = se2.T; }
     if (SE.valid && SE.type == 1) SE.Le = light_emission(P, P.lights[lslot], lh);
-    if (SE.valid && SE.type == 0) Lv = cadd(Lv, uniform_sample_one_light(P, SE, rng, ms, hit));
+    if (SE.valid && SE.type == 0) Lv = cadd(Lv, uniform_sample_one_light<K>(P, SE, rng, ms, hit));
     if (SE.valid && SE.type == 1) Lv = cadd(Lv, SE.Le);
-    if (SE.valid && SE.type == 2) Lv = cadd(Lv, uniform_sample_one_light(P, SE, rng, ms, hit));
+    if (SE.valid && SE.type == 2) Lv = cadd(Lv, uniform_sample_one_light<K>(P, SE, rng, ms, hit));
     return make_float4(Lv.r, Lv.g, Lv.b, SE.valid ? 1.0f : 0.0f);
 }
 

@@ -14,6 +14,7 @@
 
 using namespace erd;
 
+template <int K>
 __global__ void __launch_bounds__(128) k_trace_frame(const Params P, uint32_t* __restrict__ lanes, float4* __restrict__ frame)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -25,7 +26,7 @@ __global__ void __launch_bounds__(128) k_trace_frame(const Params P, uint32_t* _
     Rng rng;
     rng.s0 = lanes[p];
     rng.s1 = lanes[n + p];
-    frame[p] = single_scattering(P, x, y, rng);
+    frame[p] = single_scattering<K>(P, x, y, rng);
     lanes[p] = rng.s0;
     lanes[n + p] = rng.s1;
 }
@@ -42,7 +43,7 @@ __global__ void __launch_bounds__(128) k_trace_sum(const Params P, int spp, uint
     for (int k = 0; k < spp; k++) {
         Rng rng;
         er_seed_lanes(P.seed, view, pix, first + (uint32_t)k, &rng.s0, &rng.s1);
-        const float4 o = single_scattering(P, x, y, rng, view, (int64_t)(first + (uint32_t)k));
+        const float4 o = single_scattering<ER_K_ONE>(P, x, y, rng, view, (int64_t)(first + (uint32_t)k));
         a0 += o.x; a1 += o.y; a2 += o.z; a3 += o.w;
     }
     float4 r = make_float4(a0, a1, a2, a3);
@@ -137,7 +138,9 @@ cudaError_t er_launch_trace_frame(const Params& P, uint32_t* lanes, float4* fram
 {
     const dim3 b(16, 8);
     const dim3 g((P.film[0] + 15) / 16, (P.film[1] + 7) / 8);
-    k_trace_frame<<<g, b, 0, s>>>(P, lanes, frame);
+    /* four resident blocks an SM (128 registers): fewer do not fill it */
+    if ((size_t)g.x * g.y < 152 * 8) k_trace_frame<ER_K_FEW><<<g, b, 0, s>>>(P, lanes, frame);
+    else k_trace_frame<ER_K_ONE><<<g, b, 0, s>>>(P, lanes, frame);
     return cudaGetLastError();
 }
 

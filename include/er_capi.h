@@ -219,7 +219,7 @@ typedef struct er_render_settings {
                                      2, 3, 4, 6 or 8 (0 or other values: 4) */
     int32_t tune_shadow;          /* wavefront: same for the shadow stage (0 or other values: 4) */
     int32_t tune_shade;           /* wavefront: resident 128-thread blocks per SM of the shade stage
-                                     (2, 3, 4 or 6; 0 or other values: 2) */
+                                     (2, 3, 4 or 6; 0: 6; other values: 2) */
     int32_t stratify;             /* 1: multi-sample renders (er_render_spp, er_trace_sum_device, batches) take
                                      each sample's point on the light, light choice, BSDF sample and first
                                      delta-tracking draw from per-pixel shifted rank-1 lattices over the
