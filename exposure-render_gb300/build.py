@@ -1,11 +1,14 @@
 """Builds libexposurerender.so for sm_103a (nvcc, no cmake).
 
 Translation units:
-  er_render.cu, er_post.cu  reference-order kernels, --fmad=false so that the
-                            GPU evaluates the same floating-point operations
-                            as the reference's host build;
+  er_render.cu, er_post.cu, er_volume.cu, er_medium.cu, er_wavefront.cu,
+  er_wavefront_batch.cu     kernels, --fmad=false so that the GPU evaluates the
+                            same floating-point operations as the reference's
+                            host build (the last compiles the second to last's
+                            batch variants);
   er_runtime.cu             host runtime behind the C ABI, -ffp-contract=off
-                            for the host arithmetic that feeds the kernels.
+                            for the host arithmetic that feeds the kernels;
+  er_cxx_api.cpp            the reference's C++ API over it.
 Each TU compiles in its own nvcc process (in parallel); objects and the
 shared library go to exposure-render_gb300/_build/.
 """

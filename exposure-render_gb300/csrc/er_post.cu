@@ -19,6 +19,8 @@
  *                   (Source/gradientmagnitude.cuh:28-44 design,
  *                   Source/volumes.h:93-114 arithmetic) with a max reduction.
  */
+#include <string.h>
+
 #include "er_kernels.h"
 #include "er_path.cuh"
 
@@ -255,7 +257,10 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    the voxels that may hold the maximum make their six lookups.  Two passes:
    the largest lower bound, then the exact magnitudes of the voxels whose
    upper bound reaches it.  tol: how far a lookup may be from its cell's mean
-   (three truncations, the weights' rounding).
+   (three truncations, the weights' rounding).  Where the largest lower bound
+   is not well above that error (flat volumes, labels) most voxels would need
+   their lookups, and the exact pass leaves the volume to
+   k_gradient_magnitude (gm_bounds_tell).
 
    A block walks GM_Z planes of a GM_X x GM_Y tile of cells (a ring of halo
    around the voxels): a thread sums its cell's four voxels of a plane, adds
@@ -265,6 +270,11 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
 #define GM_X 32
 #define GM_Y 16
 #define GM_Z 32
+
+/* whether the bounds rule voxels out: the largest lower bound is over three
+   times what tol alone adds to an upper one (at eight times, the 384x384x256
+   blobs went the long way) */
+__host__ __device__ inline bool gm_bounds_tell(float low, float tol, float h) { return low > 3.0f * 2.0f * 1.7320508f * tol * h; }
 
 template <bool EXACT>
 __global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float tol, const unsigned int* low_in, unsigned int* out_bits)
@@ -283,6 +293,7 @@ __global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float 
     const bool inner = tx > 0 && tx < GM_X - 1 && ty > 0 && ty < GM_Y - 1 && X < P.res[0] && Y < P.res[1];
     const float h = 0.5f / P.spacing[0];
     const float low = EXACT ? __uint_as_float(*low_in) : 0.0f;
+    if (EXACT && !gm_bounds_tell(low, tol, h)) return;
     unsigned int best = 0;
     int prev = plane(z0 - 1);
     /* cell z is in cells[(z + 3) % 3]; voxel z needs cells z - 1, z and z + 1 */
@@ -396,12 +407,24 @@ bool er_gradient_max_applies(const Params& P)
     return P.spacing[0] == P.spacing[1] && P.spacing[1] == P.spacing[2] && P.spacing[0] > 0.0f && most <= 50000;
 }
 
-cudaError_t er_launch_gradient_max(const Params& P, int vmax, unsigned int* bits, cudaStream_t s)
+static float gradient_max_tol(const Params& P, int vmax)
 {
     int most = P.res[0];
     for (int i = 1; i < 3; i++) most = P.res[i] > most ? P.res[i] : most;
     /* a lookup's local coordinate is off by a few ulps of the volume's extent, 1e-6 of it at most */
-    const float tol = 3.5f + 3e-6f * (float)most * (float)vmax;
+    return 3.5f + 3e-6f * (float)most * (float)vmax;
+}
+
+bool er_gradient_max_found(const Params& P, int vmax, unsigned int low_bits)
+{
+    float low;
+    memcpy(&low, &low_bits, sizeof(low));
+    return gm_bounds_tell(low, gradient_max_tol(P, vmax), 0.5f / P.spacing[0]);
+}
+
+cudaError_t er_launch_gradient_max(const Params& P, int vmax, unsigned int* bits, cudaStream_t s)
+{
+    const float tol = gradient_max_tol(P, vmax);
     const dim3 b(GM_X, GM_Y), g((P.res[0] + GM_X - 3) / (GM_X - 2), (P.res[1] + GM_Y - 3) / (GM_Y - 2), (P.res[2] + GM_Z - 1) / GM_Z);
     k_gm_cells<false><<<g, b, 0, s>>>(P, tol, nullptr, bits + 1);
     k_gm_cells<true><<<g, b, 0, s>>>(P, tol, bits + 1, bits);

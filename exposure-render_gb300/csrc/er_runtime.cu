@@ -297,6 +297,7 @@ struct TracerItem {
     erd::Params P;
     uint64_t built_version = 0;
     uint64_t build_serial = 0;     /* distinct for every build of any tracer */
+    uint64_t map_serial = 0;       /* the build whose march map is made (or needs none) */
     bool built = false;
 };
 
@@ -588,12 +589,41 @@ er_status reset_tracer_buffers(TracerItem& t)
     return init_lanes(t);
 }
 
-/* Assembles the kernel parameters of a tracer; uploads the dependent blocks
-   when any bound item changed since the last build. */
-er_status build(TracerItem& t)
+/* the march's empty-space map of a built tracer, made when one of its renders
+   marches (the differentiable medium has no use for it); without room for it
+   the march makes every lookup */
+er_status build_march_map(TracerItem& t)
 {
     Context& C = ctx();
-    if (t.built && t.built_version == C.version) return ER_OK;
+    if (t.map_serial == t.build_serial) return ER_OK;
+    t.map_serial = t.build_serial;
+    VolumeItem& v = *C.volumes.items.find(t.d.volume_id)->second;
+    if (t.P.free_flight == ER_FREE_FLIGHT_DELTA || !v.normalize) return ER_OK;
+    const int shift = kMarchBrickShift, n = t.P.sigma_n;
+    int nb[3];
+    for (int i = 0; i < 3; i++) nb[i] = (v.res[i] + (1 << shift) - 1) >> shift;
+    const size_t total = (size_t)nb[0] * nb[1] * nb[2];
+    if (t.occ.ensure(total) != cudaSuccess || t.minmax.ensure(total) != cudaSuccess || t.skip_tmp.ensure(2 * total) != cudaSuccess ||
+        t.nonzero.ensure((size_t)n) != cudaSuccess) {
+        cudaGetLastError();
+        return ER_OK;
+    }
+    ER_CUDA(er_launch_march_map(v.vox.p, v.res, shift, nb, t.sigma.p, n, t.nonzero.p, t.minmax.p, t.skip_tmp.p, t.occ.p, C.stream));
+    /* renders may come on other streams */
+    ER_CUDA(cudaStreamSynchronize(C.stream));
+    t.P.occ = t.occ.p;
+    t.P.occ_shift = shift;
+    for (int i = 0; i < 3; i++) t.P.occ_nb[i] = nb[i];
+    return ER_OK;
+}
+
+/* Assembles the kernel parameters of a tracer; uploads the dependent blocks
+   when any bound item changed since the last build.  rays: for a render of
+   the tracer itself (its march's map too). */
+er_status build(TracerItem& t, bool rays = true)
+{
+    Context& C = ctx();
+    if (t.built && t.built_version == C.version) return rays ? build_march_map(t) : ER_OK;
     const er_tracer_desc& d = t.d;
     auto vit = C.volumes.items.find(d.volume_id);
     if (vit == C.volumes.items.end()) return fail(ER_ERR_INVALID_ID, "tracer references volume ID:%d which does not exist", d.volume_id);
@@ -681,21 +711,6 @@ er_status build(TracerItem& t)
         P.brickf = (float)brick;
         for (int i = 0; i < 3; i++) P.nb[i] = nb[i];
         P.majorant = t.majorant.p;
-    } else if (v.normalize) {
-        /* the march's empty-space map; without room for it the march makes every lookup */
-        const int shift = kMarchBrickShift;
-        int nb[3];
-        for (int i = 0; i < 3; i++) nb[i] = (v.res[i] + (1 << shift) - 1) >> shift;
-        const size_t total = (size_t)nb[0] * nb[1] * nb[2];
-        if (t.occ.ensure(total) == cudaSuccess && t.minmax.ensure(total) == cudaSuccess && t.skip_tmp.ensure(2 * total) == cudaSuccess &&
-            t.nonzero.ensure((size_t)n) == cudaSuccess) {
-            ER_CUDA(er_launch_march_map(v.vox.p, v.res, shift, nb, t.sigma.p, n, t.nonzero.p, t.minmax.p, t.skip_tmp.p, t.occ.p, st));
-            P.occ = t.occ.p;
-            P.occ_shift = shift;
-            for (int i = 0; i < 3; i++) P.occ_nb[i] = nb[i];
-        } else {
-            cudaGetLastError();
-        }
     }
     /* lights in LightIDs order */
     const int lc = d.light_count;
@@ -826,7 +841,7 @@ er_status build(TracerItem& t)
     t.built_version = C.version;
     static uint64_t serial = 0;
     t.build_serial = ++serial;
-    return ER_OK;
+    return rays ? build_march_map(t) : ER_OK;
 }
 
 er_status check_device_error(TracerItem& t)
@@ -2050,7 +2065,7 @@ static er_status medium_params(int32_t tracer_id, const er_medium_desc* m, erd::
     if (!(m->nee_probability > 0.0f && m->nee_probability <= 1.0f))
         return fail(ER_ERR_INVALID_ARGUMENT, "nee_probability must lie in (0, 1]");
     if (!(m->scale > 0.0f) || !std::isfinite(m->scale)) return fail(ER_ERR_INVALID_ARGUMENT, "scale must be finite and positive");
-    er_status st = build(*t);
+    er_status st = build(*t, false);
     if (st != ER_OK) return st;
     P = t->P;
     P.brick = m->brick;
@@ -2246,13 +2261,22 @@ ER_API er_status er_gradient_magnitude(int32_t volume_id, uint16_t* d_gm, float*
     ER_CUDA(v.gm_max_bits.ensure(2));
     cudaStream_t s = ctx().stream;
     ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, 2 * sizeof(unsigned int), s));
-    if (!d_gm && er_gradient_max_applies(P)) ER_CUDA(er_launch_gradient_max(P, (int)v.vmax, v.gm_max_bits.p, s));
-    else ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
-    unsigned int bits = 0;
-    ER_CUDA(cudaMemcpyAsync(&bits, v.gm_max_bits.p, sizeof(bits), cudaMemcpyDeviceToHost, s));
-    ER_CUDA(cudaStreamSynchronize(s));
+    unsigned int bits[2] = { 0u, 0u };
+    auto read = [&]() -> cudaError_t {
+        const cudaError_t e = cudaMemcpyAsync(bits, v.gm_max_bits.p, sizeof(bits), cudaMemcpyDeviceToHost, s);
+        return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+    };
+    const bool bounds = !d_gm && er_gradient_max_applies(P);
+    if (bounds) {
+        ER_CUDA(er_launch_gradient_max(P, (int)v.vmax, v.gm_max_bits.p, s));
+        ER_CUDA(read());
+    }
+    if (!bounds || !er_gradient_max_found(P, (int)v.vmax, bits[1])) {
+        ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
+        ER_CUDA(read());
+    }
     float m;
-    memcpy(&m, &bits, sizeof(m));
+    memcpy(&m, &bits[0], sizeof(m));
     v.gm_max = m;
     if (max_gm) *max_gm = m;
     ctx().version++;

@@ -211,6 +211,8 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary(const WfView* __restri
    the lanes that run them (with one loop of steps, in which colliding and
    crossing lanes took turns, and each ended lane's set-up on its own, 7 to 8
    lanes of the shadow stage were active and 17 of the primary stage). */
+#define GATE_TAIL 4
+
 ER_D bool few_left(unsigned m, int start, int cross) { return 8 * __popc(m) <= cross * start; }
 
 ER_D uint32_t take_items(unsigned needy, uint32_t* fetch)
@@ -790,6 +792,9 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __rest
     Tracker k;
     float Tr = 1.0f;
     k.done = true;
+    /* once there are no jobs to take (from the start, when they are fewer than
+       the launch's lanes), waiting only delays the jobs' second segments */
+    if (n <= gridDim.x * blockDim.x) gate = GATE_TAIL;
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, phase ? k.done : !exhausted);
         const unsigned busy = __ballot_sync(0xffffffffu, phase && !k.done);
@@ -817,6 +822,8 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __rest
             const unsigned needy = __ballot_sync(0xffffffffu, !phase && !exhausted);
             if (needy) {
                 const uint32_t next = take_items(needy, fetch);
+                if (next >= n) gate = GATE_TAIL;
+                gate = __reduce_min_sync(0xffffffffu, gate);
                 if (!phase && !exhausted) {
                     j_i = next;
                     exhausted = j_i >= n;
