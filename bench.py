@@ -1239,10 +1239,10 @@ def run_medium(args, rank, world, local_rank):
         "loss": loss, "grad_norm": {"density": float(state["g"][0].norm()), "opacity": float(state["g"][1].norm())},
         "cpu_baseline": cpu,
         "clocks": clk.summary(),
-        # per window of 2^21 items: forward count, jobs, shadow, gather (+ one reduce per step);
-        # adjoint primary replay and shadow replay (one window: against the forward's kept jobs;
-        # several: count, jobs and shadow again per window)
-        "gpu_launches": args.steps * ((6 if spp * film[0] * film[1] <= (1 << 21) else 9)
+        # per window of 2^21 items: forward count, jobs, shade, shadow, gather (+ one reduce per
+        # step); adjoint primary, shade and shadow replay (one window: against the forward's kept
+        # jobs; several: count, jobs, shade and shadow again per window)
+        "gpu_launches": args.steps * ((8 if spp * film[0] * film[1] <= (1 << 21) else 12)
                                       * (-(-spp // max(1, (1 << 21) // (film[0] * film[1])))) + 1),
     }
     print(json.dumps(line), flush=True)
