@@ -149,6 +149,8 @@ struct Params {
     const uint8_t* occ;
     int occ_shift;
     int occ_nb[3];
+    float short_a, short_b;  /* rays up to short_a + short_b * (largest coordinate of the origin) long
+                                take the exact light and object tests (ray_has_length) */
     float gm_inv_max;        /* 1 / max gradient magnitude (hybrid switch) */
     /* camera (Source/camera.h:98-116) */
     int film[2];

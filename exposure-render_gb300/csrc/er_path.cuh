@@ -562,6 +562,17 @@ ER_D v2 sphere_uv(v3 p)
     return uv;
 }
 
+/* Whether shape_missed may be asked about a ray.  The exact test makes its
+   local ray from the transformed origin and end: of rays so long that the end
+   loses its direction, and of rays so short that it rounds to the origin
+   (0 / 0: the flat shapes' comparisons then all pass, a hit), only the exact
+   test itself tells.  short_a, short_b: er_runtime.cu shape_short. */
+ER_D bool ray_has_length(const Params& P, const Ray& R)
+{
+    const float big = fmaxf(fabsf(R.O.x), fmaxf(fabsf(R.O.y), fabsf(R.O.z)));
+    return R.MaxT <= 1e8f && fabsf(R.MaxT) > P.short_a + P.short_b * big;
+}
+
 /* Whether the ray up to parameter t_end certainly misses a light or object,
    so that the exact test (some hundred and fifty operations) can be left
    out.  t_end: the ray's end, or the parameter of an event that wins over any
@@ -579,8 +590,6 @@ ER_D v2 sphere_uv(v3 p)
      the segment nor anything a tenth of the radius beyond its ends. */
 ER_D bool shape_missed(const Light& L, const Ray& R, float t_end)
 {
-    /* rays so long that the exact test's own end point loses its direction */
-    if (!(R.MaxT <= 1e8f)) return false;
     const v3 E = vadd(R.O, vscale(R.D, t_end));
     if (L.ball_r2 >= 0.0f) {
         const v3 c = vload(L.ball_c);
@@ -1117,11 +1126,12 @@ ER_D void intersect_lights_geom(const Params& P, const Ray& R, Event& RS, bool r
 {
     float T = FLT_MAX;
     const float end = t_end < R.MaxT ? t_end : R.MaxT;
+    const bool long_enough = MISS && ray_has_length(P, R);
     for (int i = 0; i < P.light_count; i++) {
         if (!P.light_valid[i]) continue;
         const Light& L = P.lights[i];
         if (respect_visibility && !L.visible) continue;
-        if (MISS && shape_missed(L, R, end)) continue;
+        if (long_enough && shape_missed(L, R, end)) continue;
         const Ray Rt = xform_ray(L.inv_tm, R);
         Isect Int; Int.invalid();
         intersect_shape(L, Rt, Int);
@@ -1163,10 +1173,11 @@ ER_D c3 light_emission(const Params& P, const Light& L, const LightHit& lh)
 /* IntersectsLight - Source/lights.h:115-131 */
 ER_D bool intersects_light(const Params& P, const Ray& R)
 {
+    const bool long_enough = ray_has_length(P, R);
     for (int i = 0; i < P.light_count; i++) {
         if (!P.light_valid[i]) continue;
         const Light& L = P.lights[i];
-        if (shape_missed(L, R, R.MaxT)) continue;
+        if (long_enough && shape_missed(L, R, R.MaxT)) continue;
         const Ray Rt = xform_ray(L.inv_tm, R);
         Isect Int; Int.invalid();
         intersect_shape(L, Rt, Int);
@@ -1180,9 +1191,10 @@ ER_D bool intersects_light(const Params& P, const Ray& R)
 ER_D void intersect_objects(const Params& P, const Ray& R, Event& RS, ObjHit& hit)
 {
     float T = FLT_MAX;
+    const bool long_enough = ray_has_length(P, R);
     for (int i = 0; i < P.object_count; i++) {
         const Object& O = P.objects[i];
-        if (shape_missed(O.shape, R, R.MaxT)) continue;
+        if (long_enough && shape_missed(O.shape, R, R.MaxT)) continue;
         const Ray Rt = xform_ray(O.shape.inv_tm, R);
         Isect Int; Int.invalid();
         intersect_shape(O.shape, Rt, Int);
@@ -1202,9 +1214,10 @@ ER_D void intersect_objects(const Params& P, const Ray& R, Event& RS, ObjHit& hi
 /* IntersectsObject - Source/objects.h:64-80 */
 ER_D bool intersects_object(const Params& P, const Ray& R)
 {
+    const bool long_enough = ray_has_length(P, R);
     for (int i = 0; i < P.object_count; i++) {
         const Object& O = P.objects[i];
-        if (shape_missed(O.shape, R, R.MaxT)) continue;
+        if (long_enough && shape_missed(O.shape, R, R.MaxT)) continue;
         const Ray Rt = xform_ray(O.shape.inv_tm, R);
         Isect Int; Int.invalid();
         intersect_shape(O.shape, Rt, Int);

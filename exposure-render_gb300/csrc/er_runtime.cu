@@ -456,6 +456,30 @@ void shape_balls(erd::Light& l)
     if (l.type == ER_SHAPE_SPHERE) l.inner_r2 = (float)(0.81 * radius * radius);
 }
 
+/* Params::short_a, short_b: the length below which the exact test's local ray
+   (origin and end under A x + t) may lose its direction.  The difference of
+   the two points is off by at most 1e-6 (|A| (|O| + length) + |t|) from the
+   roundings of ten operations, and as long as the length times A's smallest
+   singular value (at least 2 |det A| / |A|^2); the limit is ten times that,
+   and above the lengths whose square underflows. */
+void shape_short(const erd::Light& l, erd::Params& P)
+{
+    double f2 = 0.0, t2 = 0.0;
+    const auto& m = l.inv_tm;
+    for (int r = 0; r < 3; r++) {
+        for (int c = 0; c < 3; c++) f2 += (double)m[r][c] * m[r][c];
+        t2 += (double)m[r][3] * m[r][3];
+    }
+    const double det = (double)m[0][0] * ((double)m[1][1] * m[2][2] - (double)m[1][2] * m[2][1]) -
+                       (double)m[0][1] * ((double)m[1][0] * m[2][2] - (double)m[1][2] * m[2][0]) +
+                       (double)m[0][2] * ((double)m[1][0] * m[2][1] - (double)m[1][1] * m[2][0]);
+    const double least = 2.0 * std::fabs(det) / f2, f = std::sqrt(f2);
+    double a = (1e-5 * std::sqrt(t2) + 1e-15) / least, b = 1.8e-5 * f / least;
+    if (!(b < 0.5) || !std::isfinite(a)) a = HUGE_VAL;
+    P.short_a = std::max(P.short_a, (float)a);
+    P.short_b = std::max(P.short_b, (float)std::min(b, 1.0));
+}
+
 void to_light(erd::Light& o, const er_light_desc& s)
 {
     to_shape(o, s.shape);
@@ -725,7 +749,7 @@ er_status build(TracerItem& t, bool rays = true)
         valid[i] = 1;
     }
     for (int i = 0; i < lc; i++)
-        if (valid[i]) shape_balls(L[i]);
+        if (valid[i]) { shape_balls(L[i]); shape_short(L[i], P); }
         else L[i].inner_r2 = L[i].ball_r2 = -1.0f;
     /* lights whose texture is uniform (or unbound: black) get its value here,
        as EvaluateTexture computes it: colour * OutputLevel in float
@@ -769,6 +793,7 @@ er_status build(TracerItem& t, bool rays = true)
         memset(&o, 0, sizeof(o));
         to_shape(o.shape, kv.second->shape);
         shape_balls(o.shape);
+        shape_short(o.shape, P);
         o.diffuse_texture_id = kv.second->diffuse_texture_id;
         o.specular_texture_id = kv.second->specular_texture_id;
         o.glossiness_texture_id = kv.second->glossiness_texture_id;

@@ -99,6 +99,40 @@ def test_lights_with_extreme_rays(env, oracle, clip_far, aperture):
     check_sum(env, oracle, sc)
 
 
+def light_of(shape, pos, **kw):
+    L = C.er_light_desc()
+    L.visible = 1
+    L.shape = S.make_shape(shape, S.look_at_tm(pos, (0.0, 0.0, 0.0), (0.0, 1.0, 0.0)), **kw)
+    L.texture_id = 0
+    L.multiplier = 4.0
+    return L
+
+
+LIGHTS = {"plane": (C.SHAPE_PLANE, (0.3, 1.1, 0.9), dict(size=(0.6, 0.4, 0.0))), "disk": (C.SHAPE_DISK, (-0.9, 0.5, 0.8), dict(outer=0.3)),
+          "ring": (C.SHAPE_RING, (0.2, -0.9, 1.0), dict(inner=0.1, outer=0.3)), "sphere": (C.SHAPE_SPHERE, (0.8, 0.8, -0.6), dict(outer=0.2)),
+          "around": (C.SHAPE_SPHERE, (0.0, 0.0, 1.0), dict(outer=5.0))}
+
+
+@pytest.mark.parametrize("kind", list(LIGHTS))
+@pytest.mark.parametrize("shadow,far,mult", [(0.0, None, 1), (1e-9, None, 1), (1e-7, None, 1), (1e-5, None, 1), (-1e-8, None, 1), (None, 0.0, 1),
+                                             (None, 1e-9, 1), (0.0, None, 100)])
+def test_lights_with_rays_of_no_length(env, oracle, kind, shadow, far, mult):
+    """rays so short that their end rounds to their origin: the exact light and
+    object tests divide zero by zero there and count flat shapes as hit"""
+    shape, pos, kw = LIGHTS[kind]
+    sc = S.scene_objects(res=20, film=(24, 20))
+    sc.lights = [light_of(shape, tuple(mult * v for v in pos), **kw)]
+    t = sc.tracer
+    t.light_count, t.light_ids[0] = 1, 0
+    if shadow is not None:
+        t.settings.max_shadow_distance = shadow
+    if far is not None:
+        t.camera.clip_near, t.camera.clip_far = 0.0, far
+    for delta in (0, 1):
+        t.settings.free_flight = t.settings.mis = delta
+        check_sum(env, oracle, sc)
+
+
 @pytest.mark.parametrize("shape,spacing", [((1, 1, 1), (1, 1, 1)), ((2, 3, 1), (1, 1, 1)), ((31, 15, 29), (1, 1, 1)), ((33, 14, 30), (1, 1, 1)),
                                            ((64, 30, 61), (0.7, 0.7, 0.7)), ((20, 21, 22), (1.0, 2.0, 0.5))])
 @pytest.mark.parametrize("kind", ["noise", "flat", "spike"])
