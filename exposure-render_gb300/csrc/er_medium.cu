@@ -1391,8 +1391,14 @@ struct DmWorkspace {
     uint64_t key = 0;
     cudaStream_t key_stream = nullptr;
     uint32_t kept_jobs = 0;    /* the kept walk's job count */
+    /* behind the last call's work: the calls of a device share the arrays and
+       the counters that the walks take items from, so a call starts when the
+       one before it, on whatever stream, has left them */
+    cudaEvent_t done = nullptr;
+    bool used = false;
     ~DmWorkspace()
     {
+        if (done) cudaEventDestroy(done);
         cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id); cudaFree(rng); cudaFree(off); cudaFree(cnt); cudaFree(total); cudaFree(E);
         if (host_total) cudaFreeHost(host_total);
     }
@@ -1430,6 +1436,31 @@ struct DmWorkspace {
     }
 };
 
+static bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
+}
+
+/* a call's turn on the workspace, given back on every way out of the call.
+   Under capture (only an adjoint that replays kept jobs can be captured) the
+   event would join the captured graph: the caller orders the graph's launches. */
+struct DmTurn {
+    DmWorkspace& ws;
+    cudaStream_t s;
+    cudaError_t status = cudaSuccess;
+    DmTurn(DmWorkspace& w, cudaStream_t stream) : ws(w), s(stream)
+    {
+        if (!ws.done) status = cudaEventCreateWithFlags(&ws.done, cudaEventDisableTiming);
+        if (status == cudaSuccess && ws.used && !capturing(s)) status = cudaStreamWaitEvent(s, ws.done, 0);
+    }
+    ~DmTurn()
+    {
+        if (!ws.done || capturing(s)) return;
+        ws.used = cudaEventRecord(ws.done, s) == cudaSuccess || ws.used;
+    }
+};
+
 /* one workspace per device (callers hold the library lock) */
 static DmWorkspace& dm_workspace()
 {
@@ -1453,6 +1484,8 @@ static cudaError_t dm_windows(const Params& P, const DmParams& M, int spp, uint3
                               const float* dimg, float* g_rho, float* g_tf, uint64_t key, cudaStream_t s)
 {
     DmWorkspace& ws = dm_workspace();
+    const DmTurn turn(ws, s);
+    if (turn.status != cudaSuccess) return turn.status;
     const uint32_t npix = (uint32_t)P.film[0] * (uint32_t)P.film[1];
     uint32_t rows = (uint32_t)((1u << 21) / (npix ? npix : 1));
     if (rows < 1) rows = 1;

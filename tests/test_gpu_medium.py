@@ -167,3 +167,35 @@ def test_c4_adjoint_matches_finite_differences(torch, lib, pkg):
         print(f"worst relative error over 32 parameters: {worst:.2e}")
     finally:
         r.close()
+
+
+def test_two_streams_share_the_device(torch, lib, pkg):
+    """renders and adjoints of two media queued on two streams without waiting
+    in between give what they give alone (the calls share one workspace)"""
+    spp = 16
+    media = [make(torch, lib, pkg, (40, 36, 44), 16, (120, 100), 40.0, 8, seed=s, blobs=6) for s in (3, 5)]
+    g = torch.Generator(device="cuda").manual_seed(1)
+    slope = torch.randn((100, 120, 3), device="cuda", generator=g)
+
+    def both(streams):
+        out = []
+        for rep in range(3):
+            for (sc, r, m, rho, tf), st in zip(media, streams):
+                with torch.cuda.stream(st):
+                    smp, s = m.render_samples(rho, tf, spp, view=rep)
+                    out.append((smp, s, *m.adjoint(rho, tf, spp, slope, smp if rep % 2 else None, view=rep)))
+        torch.cuda.synchronize()
+        return out
+
+    try:
+        alone = both([torch.cuda.current_stream()] * 2)
+        for _ in range(3):
+            apart = both([torch.cuda.Stream(), torch.cuda.Stream()])
+            for a, b in zip(alone, apart):
+                assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+                # atomic sums in another order
+                for x, y in zip(a[2:], b[2:]):
+                    assert torch.allclose(x, y, rtol=1e-5, atol=1e-5 * float(x.abs().max()))
+    finally:
+        for sc, r, *_ in media:
+            r.close()

@@ -1,0 +1,88 @@
+"""The library's host code on a machine without a GPU: its objects linked
+against fake_cudart.cpp, which makes copies on the host and lists launches,
+copies and waits by stream."""
+import ctypes
+import importlib
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle_lib as OL
+
+C = OL.C
+S = OL.PKG.scenes
+BUILD = importlib.import_module("exposure-render_gb300.build")
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    BUILD.build()
+    out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    objs = [os.path.join(BUILD.OUT, os.path.splitext(u)[0] + ".o") for u in BUILD.UNITS]
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(BUILD.nvcc()))), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic,--no-undefined", "-I" + cuda,
+                    os.path.join(HERE, "fake_cudart.cpp"), *objs, "-o", out], check=True)
+    return out
+
+
+@pytest.fixture()
+def lib(fake_path, monkeypatch, tmp_path):
+    monkeypatch.setenv("ER_TUNE_CACHE", str(tmp_path / "autotune.txt"))
+    L = C.load_library(fake_path)
+    L.fake_log.restype = ctypes.c_char_p
+    L.fake_bad_read.argtypes = [ctypes.c_size_t]
+    L.fake_no_memory(0)
+    L.fake_bad_read(0)
+    L.fake_clear()
+    yield L
+    L.fake_no_memory(0)
+    L.fake_bad_read(0)
+    L.er_reset()
+
+
+def log(lib):
+    """(what, stream, kernel or event) of every call since the last look"""
+    out = [tuple(line.split(" ", 2)) for line in lib.fake_log().decode().splitlines()]
+    lib.fake_clear()
+    return out
+
+
+def renderer(lib, sc):
+    return importlib.import_module("exposure-render_gb300.runtime").Renderer(sc, lib)
+
+
+STREAM_A, STREAM_B = 0x1000, 0x2000
+
+
+@pytest.mark.parametrize("back", [False, True], ids=["forward", "adjoint"])
+def test_medium_calls_on_two_streams_take_turns(lib, back):
+    """the walks of one device share their job and item arrays: a call on
+    another stream starts behind the work of the call before it"""
+    sc = S.medium_scene(res=(8, 8, 8), film=(8, 8))
+    r = renderer(lib, sc)
+    buf = np.zeros(1 << 16, np.float32)
+    p = buf.ctypes.data
+    m = C.er_medium_desc()
+    m.d_density, m.d_opacity, m.n_opacity, m.scale, m.nee_probability = p, p, 16, 1.0, 0.5
+    m.d_majorant, m.brick, m.model = p, 8, C.ER_MEDIUM_SPLINE
+
+    def call(stream):
+        if back:
+            C.check(lib.er_medium_adjoint(r.tracer_id, ctypes.byref(m), 2, 0, 0, p, None, p, p, stream))
+        else:
+            C.check(lib.er_medium_render(r.tracer_id, ctypes.byref(m), 2, 0, 0, p, p, stream))
+
+    call(STREAM_A)
+    first = log(lib)
+    call(STREAM_B)
+    second = log(lib)
+    r.close()
+    a, b = f"{STREAM_A:x}", f"{STREAM_B:x}"
+    work = [i for i, e in enumerate(first) if e[0] in ("launch", "set") and e[1] == a and "k_dm_reduce" not in e[2]]
+    marks = [(i, e[2]) for i, e in enumerate(first) if e[0] == "record" and e[1] == a]
+    assert marks and marks[-1][0] > work[-1]
+    begin = next(i for i, e in enumerate(second) if e[0] in ("launch", "set") and e[1] == b)
+    assert ("wait", b, marks[-1][1]) in second[:begin]
