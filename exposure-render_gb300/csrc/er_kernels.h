@@ -157,9 +157,8 @@ struct WavefrontBuffers {
 };
 
 /* cuts the items of views (npix[v] * spp[v] each) into windows of whole
-   sample rows of at most window_cap items (one row at least); a view starts a
-   window of its own when the open one has `apart` items (0: never) */
-void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, size_t apart, WavefrontPlan& plan);
+   sample rows of at most window_cap items (one row at least) */
+void er_wavefront_plan(const int* npix, const int* spp, int n_views, size_t window_cap, WavefrontPlan& plan);
 
 /* stage timing of the wavefront launches: 0 primary, 1 shade, 2 shadow,
    3 reduce; read returns the accumulated milliseconds and launch counts since

@@ -104,11 +104,6 @@ uint64_t fnv1a(uint64_t h, const void* data, size_t n)
 /* items of one wavefront window: 8M samples, 1.5 GB of queues */
 constexpr size_t kWindowCap = (size_t)8 << 20;
 
-/* a batch's next view starts a window of its own behind this many samples: a
-   window of one view runs the one-view kernels (er_launch_wavefront_batch),
-   some tenth faster, and its extra launches and tails cost about 40 us */
-constexpr size_t kWindowApart = (size_t)1 << 20;
-
 /* resident blocks of the shade stage when the settings name none: 6 (80
    registers) hides its dependent loads better than 2 (c3 views 11.6 against
    12.5 ms, c5 views 6.6 against 7.0, c2 shells 3.7 against 3.8) */
@@ -911,7 +906,7 @@ er_status trace_sum(TracerItem& t, int spp, uint32_t view, uint32_t first, float
     }
     const int npix = t.W * t.H;
     WavefrontPlan plan;
-    er_wavefront_plan(&npix, &spp, 1, kWindowCap, 0, plan);
+    er_wavefront_plan(&npix, &spp, 1, kWindowCap, plan);
     WavefrontBuffers B;
     ER_CUDA(t.wf.ensure(plan, B));
     B.tune_primary = t.d.settings.tune_primary > 0 ? t.d.settings.tune_primary : 4;
@@ -996,7 +991,7 @@ er_status batch_plan(BatchItem& b)
         for (int u = 0; u < v; u++)
             if (b.host_views[(size_t)v].sum == b.host_views[(size_t)u].sum)
                 return fail(ER_ERR_INVALID_ARGUMENT, "batch views %d and %d share a sum buffer", u, v);
-    er_wavefront_plan(npix.data(), spp.data(), n, b.window_cap, kWindowApart, b.plan);
+    er_wavefront_plan(npix.data(), spp.data(), n, b.window_cap, b.plan);
     ER_CUDA(b.wf.ensure(b.plan, b.B));
     ER_CUDA(b.d_views.ensure((size_t)n));
     ER_CUDA(b.d_segs.ensure(b.plan.segs.size()));

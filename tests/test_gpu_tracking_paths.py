@@ -224,3 +224,40 @@ def test_batch_windows_of_one_view(env, stages, flags):
         b.close()
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("stages", [0, 1])
+@pytest.mark.parametrize("flags", [0, C.ER_BATCH_GRAPH])
+def test_batch_of_full_windows(env, stages, flags):
+    """two views that fill more than a window between them: each in windows of
+    its own, its parameters by value, its first sample from the table"""
+    torch, lib, runtime = env
+    sc = S.scene_tiny(res=24, film=(24, 20), seed=4)
+    s = sc.tracer.settings
+    s.free_flight = s.mis = s.stratify = 1
+    s.tune_stages, s.majorant_brick = stages, 2
+    r = runtime.Renderer(sc, lib)
+    rng = np.random.default_rng(5)
+    try:
+        cams = [S.orbit_camera(rng, (1025, 1024)) for _ in range(2)]
+        sums = [torch.zeros((1024, 1025, 4), device="cuda") for _ in cams]
+        b = runtime.Batch([(r.tracer_id, 5, d.data_ptr(), cam) for d, cam in zip(sums, cams)], flags=flags)
+        assert b.info()["windows"] == b.info()["segments"] == 2
+        for first in (0, 5):
+            if first:
+                b.advance(first)
+            b.launch()
+            torch.cuda.synchronize()
+            for i, cam in enumerate(cams):
+                t = C.er_tracer_desc.from_buffer_copy(r.tracer_desc)
+                t.camera = cam
+                tid = ctypes.c_int32(-1)
+                C.check(lib.er_bind_tracer(ctypes.byref(t), ctypes.byref(tid)))
+                d = torch.zeros((1024, 1025, 4), device="cuda")
+                C.check(lib.er_trace_sum_device(tid.value, 5, i, first, d.data_ptr(), 0, None))
+                torch.cuda.synchronize()
+                lib.er_unbind_tracer(tid.value)
+                assert torch.equal(d.view(torch.int32), sums[i].view(torch.int32)), (i, first)
+        b.close()
+    finally:
+        r.close()

@@ -86,3 +86,38 @@ def test_medium_calls_on_two_streams_take_turns(lib, back):
     assert marks and marks[-1][0] > work[-1]
     begin = next(i for i, e in enumerate(second) if e[0] in ("launch", "set") and e[1] == b)
     assert ("wait", b, marks[-1][1]) in second[:begin]
+
+
+def batch_info(lib, r, sizes, cap=0):
+    """(windows, segments) of a batch of (width, height, samples) views"""
+    runtime = importlib.import_module("exposure-render_gb300.runtime")
+    rng = np.random.default_rng(1)
+    views = [(r.tracer_id, spp, 0x100000 * (i + 1), S.orbit_camera(rng, (w, h))) for i, (w, h, spp) in enumerate(sizes)]
+    b = runtime.Batch(views, flags=0, window_items=cap, lib=lib)
+    info = b.info()
+    b.close()
+    return info["windows"], info["segments"]
+
+
+@pytest.mark.parametrize("sizes,cap,want", [
+    ([(200, 200, 16)] * 8, 0, (1, 8)),                              # 5.1 M samples: one window, however many views
+    ([(1024, 1024, 1)] * 8, 0, (1, 8)),
+    ([(1920, 1080, 1)] * 4, 0, (1, 4)),
+    ([(1024, 1024, 5)] * 2, 0, (2, 2)),                             # two windows in any case: one view each
+    ([(30, 20, 3), (30, 20, 3), (30, 20, 4)], 6000, (1, 3)),
+    ([(30, 20, 6), (30, 20, 6), (30, 20, 6)], 6000, (2, 4)),        # 10800 samples: the second view in both
+    ([(30, 20, 10), (30, 20, 10)], 6000, (2, 2)),
+    ([(30, 20, 9), (30, 20, 2), (30, 20, 10)], 6000, (3, 3)),
+    ([(30, 20, 25)], 6000, (3, 3)),
+    ([(1100, 1000, 1), (20, 20, 1)], 0, (2, 2)),                    # the reduce stage's grid is the larger film's
+])
+def test_windows_are_as_few_as_can_be(lib, sizes, cap, want):
+    """each window ends with its longest rays alone on the chip, so a view gets
+    a window of its own only where that adds none"""
+    sc = S.scene_tiny(res=8, film=(8, 8))
+    sc.tracer.settings.free_flight = C.FREE_FLIGHT_DELTA
+    r = renderer(lib, sc)
+    try:
+        assert batch_info(lib, r, sizes, cap) == want
+    finally:
+        r.close()
