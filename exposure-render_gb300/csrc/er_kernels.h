@@ -148,10 +148,9 @@ struct WavefrontBuffers {
     int pt_primary;      /* the persistent-lane primary stage runs (every view delta-tracks) */
     int pt_shadow;       /* the persistent-lane shadow stage runs (every view delta-tracks) */
     int free_flight;     /* WF_MARCH, WF_DELTA (every view uses that estimator) or WF_MIXED */
-    int cross_eighths;   /* persistent stages: lanes cross bricks together until this many eighths of them still do */
+    int cross_eighths;   /* persistent shadow stage of large windows: lanes cross bricks together until this many eighths of them still do */
     int collide_eighths; /* and collide together until this many eighths of the colliding ones still do */
-    int gate_primary;    /* and set rays up when this many lanes of a warp have ended theirs */
-    int gate_shadow;
+    int gate_shadow;     /* and set segments up when this many lanes of a warp have ended theirs */
     int sort_shade;      /* a view's shader switch mixes BRDF and phase events: the shade stage runs as
                             k_wf_classify + k_wf_shade_sorted (records must be allocated) */
 };

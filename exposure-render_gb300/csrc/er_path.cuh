@@ -178,11 +178,11 @@ ER_D void shade_tf(const Params& P, float I, ShadeTF& s)
 
 /* er_logf(u) for a draw u: 0 or a normal number below 1 (Rng::get1 and
    er_lattice_unit give no other).  er_logf's operations on those, without
-   its tests for other arguments. */
+   its tests for other arguments, and 0 by a select: a branch in every step's
+   chain (64 x 64 samples of 96^3 blobs in 8^3 bricks 1600 -> 1557 us). */
 ER_D float log_unit(float u)
 {
     const uint32_t b = __float_as_uint(u);
-    if (b == 0u) return -ER_F_INF;
     float fe = (float)((int)(b >> 23) - 127);
     float m = __uint_as_float((b & 0x007fffffu) | 0x3f800000u);
     if (m > 1.41421356f) { m = m * 0.5f; fe = fe + 1.0f; }
@@ -192,7 +192,8 @@ ER_D float log_unit(float u)
     const float R = z * (0.666666667f + z * (0.4f + z * (0.285714286f + z * 0.222222222f)));
     const float hfsq = 0.5f * f * f;
     const float lm = f - (hfsq - s * (hfsq + R));
-    return fe * ER_LN2_HI + (lm + fe * ER_LN2_LO);
+    const float r = fe * ER_LN2_HI + (lm + fe * ER_LN2_LO);
+    return b == 0u ? -ER_F_INF : r;
 }
 
 /* ---- gradients: Source/volumes.h:31-114 ---- */
@@ -1473,6 +1474,39 @@ ER_D bool track_cross(const Params& P, Tracker& k)
     dda_advance(P, k.d, k.e);
     k.done = k.d.done;
     return false;
+}
+
+/* one step of a lane on its own: crosses a brick (or jumps), or moves to the
+   next tentative collision of the brick and makes it.  track_cross and the
+   collision in one: written as the two, the chain of a step is longer (16384
+   samples of 24^3 blobs in 8^3 bricks 5405 against 5268 us). */
+template <typename Collide>
+ER_D void track_step(const Params& P, Tracker& k, Collide collide)
+{
+    if (!k.in_brick) {
+        k.e = dda_exit(k.d);
+        k.mu = dda_majorant(P, k.d);
+        k.t = k.d.t;
+        k.in_brick = true;
+    }
+    if (k.mu > 0.0f) {
+        const float dt = k.tau / k.mu;
+        if (k.t + dt < k.e) {
+            k.t = k.t + dt;
+            collide();
+            return;
+        }
+        k.tau = k.tau - k.mu * (k.e - k.t);
+        if (k.tau < 0.0f) k.tau = 0.0f;
+    } else if (k.mu <= -2.0f) {
+        dda_jump(P, k.d, (int)(-k.mu));
+        k.in_brick = false;
+        if (k.d.done) k.done = true;
+        return;
+    }
+    dda_advance(P, k.d, k.e);
+    k.in_brick = false;
+    if (k.d.done) k.done = true;
 }
 
 /* after a collision: whether the next one lies in the same brick (then at k.t);

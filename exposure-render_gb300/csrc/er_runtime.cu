@@ -112,22 +112,14 @@ constexpr int kShadeBlocks = 6;
 /* bricks of the march's empty-space map: 2^2 = 4 voxels a side */
 constexpr int kMarchBrickShift = 2;
 
-/* the persistent stages' lanes (er_wavefront.cu): a warp's crossing ends when
-   5 eighths of its crossing lanes still cross (ER_PT_REFILL=0..7 for
-   measurements), its collisions when 7 eighths of the colliding ones still
-   collide; the primary stage sets rays up when the whole warp has ended (its
-   set-up and finish, some 1500 instructions, cost more than the lanes that
-   wait), the shadow stage when 14 lanes have.  Measured, ms:
-   - gates of 8, 16, 24 and 32 lanes, primary stage of the c2 shells 16.7,
-     13.1, 11.5, 9.4, of the c3 views 56.1, 48.9, 45.7, 43.9, of the c5 views
-     42.4, 35.6, 32.0, 28.1; 8, 12, 16 and 24 lanes, shadow stage of the c5
-     views 10.9, 10.6, 10.7, 11.2;
-   - crossing / collision eighths (6 c3 views with 8^3, 2^3 bricks; shadow
-     stage of c5): 3 / one pass 59.9, 17.8, 10.4; 7 / 7 56.7, 17.5, 11.6;
-     5 / 7 55.4, 17.3, 10.6; 5 / 5 60.6, 17.2, 10.8.  Large bricks hold many
-     collisions each, so a warp that waits for its last colliding lanes is
-     the worse there. */
-constexpr int kGatePrimary = 32, kGateShadow = 14, kCollideEighths = 7;
+/* the persistent shadow stage's lanes in large windows (er_wavefront.cu): a
+   warp's crossing ends when 5 eighths of its crossing lanes still cross
+   (ER_PT_REFILL=0..7 for measurements), its collisions when 7 eighths of the
+   colliding ones still collide, and it sets segments up when 14 lanes have
+   ended theirs.  Measured, ms, shadow stage of the c5 views: gates of 8, 12, 16
+   and 24 lanes 10.9, 10.6, 10.7, 11.2; crossing / collision eighths 3 / one
+   pass 10.4, 7 / 7 11.6, 5 / 7 10.6, 5 / 5 10.8. */
+constexpr int kGateShadow = 14, kCollideEighths = 7;
 int cross_eighths()
 {
     static int v = -1;
@@ -174,7 +166,6 @@ struct WfQueues {
         B.sort_shade = 0;
         B.cross_eighths = cross_eighths();
         B.collide_eighths = kCollideEighths;
-        B.gate_primary = kGatePrimary;
         B.gate_shadow = kGateShadow;
         B.counters = counters.p;
         B.tune_primary = 4;

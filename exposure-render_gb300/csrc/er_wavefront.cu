@@ -197,20 +197,30 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary(const WfView* __restri
     }
 }
 
-/* Persistent lanes (delta tracking).  A warp alternates between three parts,
-   each made by as many of its lanes together as can be had:
-     crossing : lanes cross majorant bricks until cross / 8 of those that
-                were crossing still do;
+/* Persistent lanes (delta tracking): a lane whose ray has ended takes the next
+   item of the window, while the others keep theirs.  What bounds the stages is
+   the lanes that run each part and, where a window has few items for each
+   lane, the time of the longest chain of steps.
+
+   Steps: a lane crosses a brick or makes a collision at a time, with the
+   others; when under a quarter of the lanes that were tracking still are, the
+   warp finishes the ended samples and sets the next rays up.  The shadow stage
+   of large windows splits this in three parts instead, each made by as many
+   lanes together as can be had:
+     crossing : lanes cross bricks until cross / 8 of those that were
+                crossing still do;
      collision: the lanes that are at a tentative collision look it up, and
                 go on to the brick's next one, until collide / 8 are left;
-     set-up   : when `gate` lanes have ended their rays (or no lane tracks),
-                those lanes finish their samples, take the window's next items
-                (consecutive ones, one atomic per warp) and set their rays up,
-                while the others keep theirs.
-   Each part is some 60 to 600 instructions long, so what bounds the stage is
-   the lanes that run them (with one loop of steps, in which colliding and
-   crossing lanes took turns, and each ended lane's set-up on its own, 7 to 8
-   lanes of the shadow stage were active and 17 of the primary stage). */
+     set-up   : when `gate` lanes have ended their segments (or none tracks).
+   The parts make a large window's shadow stage faster and a small one's
+   slower (lanes wait for each other, and each step costs more ballots): c2
+   shells at 512^3, 0.26, 1.05, 2.1, 4.2 and 8.4 M samples, parts 197, 296,
+   453, 738, 1315 us, steps 171, 282, 445, 778, 1422; blobs at 96^3 in 2^3
+   bricks 443, 448, 568, 644, 886 against 424, 414, 484, 615, 875.  The free
+   flight in parts was slower on everything but sparse shells (64 x 64 samples
+   of the blobs in 8^3 bricks 1394 us in steps, 1648 in parts; 4.2 M samples
+   8.5 against 9.8 ms; 16 c3 views 37.0 against 38.2; shells of 200^3 at 4.2 M
+   1.69 against 1.58). */
 #define GATE_TAIL 4
 
 ER_D bool few_left(unsigned m, int start, int cross) { return 8 * __popc(m) <= cross * start; }
@@ -234,12 +244,10 @@ template <int MINB, bool ONE, bool OBJ>
 __global__ void __launch_bounds__(256, MINB) k_wf_primary_pt(const WfView* __restrict__ views, const WfSegment* __restrict__ segs,
                                                               int nseg, const WfView one, const WfSegment one_seg, uint32_t items,
                                                               float4* __restrict__ results, float4* __restrict__ events,
-                                                              uint32_t* __restrict__ n_events, uint32_t* __restrict__ fetch, int cross,
-                                                              int collide, int gate)
+                                                              uint32_t* __restrict__ n_events, uint32_t* __restrict__ fetch)
 {
     uint32_t i = 0;
-    /* at: the ray is at a tentative collision; hit: at a real one */
-    bool have = false, exhausted = false, hit = false, at = false;
+    bool have = false, exhausted = false, hit = false;
     int seg = 0;
     Rng rng;
     rng.s0 = 0u;
@@ -248,121 +256,106 @@ __global__ void __launch_bounds__(256, MINB) k_wf_primary_pt(const WfView* __res
     Tracker k;
     k.done = true;
     for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, have ? k.done : !exhausted);
-        const unsigned busy = __ballot_sync(0xffffffffu, have && !k.done);
-        if (!(idle | busy)) break;
-        if (!busy || __popc(idle) >= gate) {
-            bool push = false;
-            Event SE;
-            WfSegment sg = one_seg;
-            if (have && k.done) {
-                /* the sample's nearest event: volume, visible lights, objects */
-                if (!ONE) sg = segs[seg];
-                const Params& P = view_of<ONE>(views, one, sg.view).P;
-                Event se1;
-                SE.type = 0; SE.valid = false; SE.T = 0.0f; SE.Le = C3(0, 0, 0);
-                SE.P = V3(0, 0, 0); SE.N = V3(0, 0, 0); SE.Wo = V3(0, 0, 0);
-                se1 = SE; se1.type = 1;
-                if (hit) {
-                    SE.valid = true;
-                    SE.T = k.t;
-                    SE.P = vadd(R.O, vscale(R.D, k.t));
-                    SE.N = V3(0.0f, 0.0f, 0.0f);
-                    SE.Wo = vneg(R.D);
+        const unsigned needy = __ballot_sync(0xffffffffu, !have && !exhausted);
+        if (needy) {
+            const uint32_t next = take_items(needy, fetch);
+            if (!have && !exhausted) {
+                i = next;
+                exhausted = i >= items;
+                if (!exhausted) {
+                    seg = ONE ? 0 : find_segment(segs, nseg, i);
+                    const WfSegment sg = ONE ? one_seg : segs[seg];
+                    const WfView& V = view_of<ONE>(views, one, sg.view);
+                    const Params& P = V.P;
+                    const uint32_t local = i - sg.offset;
+                    const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
+                    const int s = sg.s0 + (int)(local / npix);
+                    const int pix = (int)slot_pixel(P, local % npix);
+                    er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s, &rng.s0, &rng.s1);
+                    Metro ms;
+                    ms.large_step(rng);
+                    ms.stratify(P, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s);
+                    R = sample_camera(P, pix % P.film[0], pix / P.film[0], ms.film_uv, ms.lens_uv);
+                    delta_begin(P, R, rng, k, ms.tau_u);
+                    hit = false;
+                    have = true;
                 }
-                const Event se0 = SE;
-                int lslot = -1;
-                LightHit lh;
-                intersect_lights_geom(P, R, se1, true, lslot, lh, se0.valid ? event_end(se0.T) : FLT_MAX);
-                SE.valid = false; SE.type = 0;
-                float T = FLT_MAX;
-                if (se0.valid && se0.T < T) { SE = se0; T = se0.T; }
-                if (se1.valid && se1.T < T) { SE = se1; T = se1.T; }
-                ObjHit ohit;
-                if (OBJ && P.object_count > 0) {
-                    Event se2;
-                    se2.type = 2; se2.valid = false; se2.T = 0.0f;
-                    intersect_objects(P, R, se2, ohit);
-                    if (se2.valid && se2.T < T) { SE = se2; T = se2.T; }
-                }
-                if (SE.valid && SE.type == 1) SE.Le = light_emission(P, P.lights[lslot], lh);
-                if (!SE.valid) {
-                    results[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                } else if (SE.type == 1) {
-                    const c3 Lv = cadd(C3(0, 0, 0), SE.Le);
-                    results[i] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
-                } else {
-                    push = true;
-                    if (OBJ && SE.type == 2) results[i] = make_float4(ohit.UV.x, ohit.UV.y, u2f((uint32_t)ohit.id), 0.0f);
-                }
-                have = false;
-            }
-            __syncwarp();
-            const uint32_t slot = queue_slot(push, n_events);
-            if (push) {
-                const WfView& V = view_of<ONE>(views, one, sg.view);
-                const Params& P = V.P;
-                const uint32_t local = i - sg.offset;
-                const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
-                Rng r0;
-                const uint32_t sidx = first_of<ONE>(views, V) + (uint32_t)(sg.s0 + (int)(local / npix));
-                const uint32_t pix = slot_pixel(P, local % npix);
-                er_seed_lanes(P.seed, V.view_id, pix, sidx, &r0.s0, &r0.s1);
-                Metro ms;
-                ms.large_step(r0);
-                ms.stratify(P, V.view_id, pix, sidx);
-                const bool obj = OBJ && SE.type == 2;
-                float4* e = events + (size_t)slot * 5;
-                e[0] = make_float4(u2f(i), u2f(rng.s0), u2f(rng.s1), ms.light_num);
-                e[1] = make_float4(SE.P.x, SE.P.y, SE.P.z, ms.brdf_component);
-                e[2] = obj ? make_float4(SE.N.x, SE.N.y, SE.N.z, ms.brdf_dir.x) : make_float4(0.0f, 0.0f, 0.0f, ms.brdf_dir.x);
-                e[3] = make_float4(SE.Wo.x, SE.Wo.y, SE.Wo.z, ms.brdf_dir.y);
-                e[4] = make_float4(ms.light_uvw.x, ms.light_uvw.y, ms.light_uvw.z, u2f((uint32_t)sg.view | (obj ? WF_OBJECT_EVENT : 0u)));
-            }
-            __syncwarp();
-            const unsigned needy = __ballot_sync(0xffffffffu, !have && !exhausted);
-            if (needy) {
-                const uint32_t next = take_items(needy, fetch);
-                if (!have && !exhausted) {
-                    i = next;
-                    exhausted = i >= items;
-                    if (!exhausted) {
-                        seg = ONE ? 0 : find_segment(segs, nseg, i);
-                        if (!ONE) sg = segs[seg];
-                        const WfView& V = view_of<ONE>(views, one, sg.view);
-                        const Params& P = V.P;
-                        const uint32_t local = i - sg.offset;
-                        const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
-                        const int s = sg.s0 + (int)(local / npix);
-                        const int pix = (int)slot_pixel(P, local % npix);
-                        er_seed_lanes(P.seed, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s, &rng.s0, &rng.s1);
-                        Metro ms;
-                        ms.large_step(rng);
-                        ms.stratify(P, V.view_id, (uint32_t)pix, first_of<ONE>(views, V) + (uint32_t)s);
-                        R = sample_camera(P, pix % P.film[0], pix / P.film[0], ms.film_uv, ms.lens_uv);
-                        delta_begin(P, R, rng, k, ms.tau_u);
-                        hit = false;
-                        have = true;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-        const Params& P = view_of<ONE>(views, one, ONE ? 0 : segs[seg].view).P;
-        int start = __popc(__ballot_sync(0xffffffffu, have && !k.done && !at));
-        for (;;) {
-            const bool crossing = have && !k.done && !at;
-            if (few_left(__ballot_sync(0xffffffffu, crossing), start, cross)) break;
-            if (crossing) at = track_cross(P, k);
-        }
-        start = __popc(__ballot_sync(0xffffffffu, at));
-        for (;;) {
-            if (few_left(__ballot_sync(0xffffffffu, at), start, collide)) break;
-            if (at) {
-                hit = delta_collide(P, R, rng, k);
-                at = !k.done && track_again(k);
             }
         }
+        if (!__any_sync(0xffffffffu, have)) break;
+        const WfSegment sg = ONE ? one_seg : segs[seg];
+        const WfView& V = view_of<ONE>(views, one, sg.view);
+        const Params& P = V.P;
+        const int start = __popc(__ballot_sync(0xffffffffu, have && !k.done));
+        while (have && !k.done) {
+            track_step(P, k, [&]() { hit = delta_collide(P, R, rng, k); });
+            /* ended lanes leave first, so the others count those that go on */
+            if (k.done || 4 * __popc(__activemask()) < start) break;
+        }
+        __syncwarp();
+        bool push = false;
+        Event SE;
+        if (have && k.done) {
+            /* the sample's nearest event: volume, visible lights, objects */
+            Event se1;
+            SE.type = 0; SE.valid = false; SE.T = 0.0f; SE.Le = C3(0, 0, 0);
+            SE.P = V3(0, 0, 0); SE.N = V3(0, 0, 0); SE.Wo = V3(0, 0, 0);
+            se1 = SE; se1.type = 1;
+            if (hit) {
+                SE.valid = true;
+                SE.T = k.t;
+                SE.P = vadd(R.O, vscale(R.D, k.t));
+                SE.N = V3(0.0f, 0.0f, 0.0f);
+                SE.Wo = vneg(R.D);
+            }
+            const Event se0 = SE;
+            int lslot = -1;
+            LightHit lh;
+            intersect_lights_geom(P, R, se1, true, lslot, lh, se0.valid ? event_end(se0.T) : FLT_MAX);
+            SE.valid = false; SE.type = 0;
+            float T = FLT_MAX;
+            if (se0.valid && se0.T < T) { SE = se0; T = se0.T; }
+            if (se1.valid && se1.T < T) { SE = se1; T = se1.T; }
+            ObjHit ohit;
+            if (OBJ && P.object_count > 0) {
+                Event se2;
+                se2.type = 2; se2.valid = false; se2.T = 0.0f;
+                intersect_objects(P, R, se2, ohit);
+                if (se2.valid && se2.T < T) { SE = se2; T = se2.T; }
+            }
+            if (SE.valid && SE.type == 1) SE.Le = light_emission(P, P.lights[lslot], lh);
+            if (!SE.valid) {
+                results[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            } else if (SE.type == 1) {
+                const c3 Lv = cadd(C3(0, 0, 0), SE.Le);
+                results[i] = make_float4(Lv.r, Lv.g, Lv.b, 1.0f);
+            } else {
+                push = true;
+                if (OBJ && SE.type == 2) results[i] = make_float4(ohit.UV.x, ohit.UV.y, u2f((uint32_t)ohit.id), 0.0f);
+            }
+            have = false;
+        }
+        __syncwarp();
+        const uint32_t slot = queue_slot(push, n_events);
+        if (push) {
+            const uint32_t local = i - sg.offset;
+            const uint32_t npix = (uint32_t)(P.film[0] * P.film[1]);
+            Rng r0;
+            const uint32_t sidx = first_of<ONE>(views, V) + (uint32_t)(sg.s0 + (int)(local / npix));
+            const uint32_t pix = slot_pixel(P, local % npix);
+            er_seed_lanes(P.seed, V.view_id, pix, sidx, &r0.s0, &r0.s1);
+            Metro ms;
+            ms.large_step(r0);
+            ms.stratify(P, V.view_id, pix, sidx);
+            const bool obj = OBJ && SE.type == 2;
+            float4* e = events + (size_t)slot * 5;
+            e[0] = make_float4(u2f(i), u2f(rng.s0), u2f(rng.s1), ms.light_num);
+            e[1] = make_float4(SE.P.x, SE.P.y, SE.P.z, ms.brdf_component);
+            e[2] = obj ? make_float4(SE.N.x, SE.N.y, SE.N.z, ms.brdf_dir.x) : make_float4(0.0f, 0.0f, 0.0f, ms.brdf_dir.x);
+            e[3] = make_float4(SE.Wo.x, SE.Wo.y, SE.Wo.z, ms.brdf_dir.y);
+            e[4] = make_float4(ms.light_uvw.x, ms.light_uvw.y, ms.light_uvw.z, u2f((uint32_t)sg.view | (obj ? WF_OBJECT_EVENT : 0u)));
+        }
+        __syncwarp();
     }
 }
 
@@ -771,8 +764,9 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow(const WfView* __restric
 
    The same jobs and arithmetic as k_wf_shadow.  A lane tracks its job's
    segments one after the other (the second continues the first one's random
-   stream); both are set up in the warp's common set-up part. */
-template <int MINB, bool ONE, bool OBJ>
+   stream); both are set up in the warp's common set-up part.  STEPS: in steps
+   instead of parts, see above. */
+template <int MINB, bool ONE, bool OBJ, bool STEPS>
 __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __restrict__ views, const WfView one,
                                                              const float4* __restrict__ jobs, const uint32_t* __restrict__ n_jobs,
                                                              float4* __restrict__ results, uint32_t* __restrict__ fetch, int cross,
@@ -799,7 +793,7 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __rest
         const unsigned idle = __ballot_sync(0xffffffffu, phase ? k.done : !exhausted);
         const unsigned busy = __ballot_sync(0xffffffffu, phase && !k.done);
         if (!(idle | busy)) break;
-        if (!busy || __popc(idle) >= gate) {
+        if (!busy || (STEPS ? idle != 0u : __popc(idle) >= gate)) {
             bool set_up = false;
             if (phase && k.done) {
                 const float4* j = jobs + (size_t)j_i * 6;
@@ -858,6 +852,14 @@ __global__ void __launch_bounds__(256, MINB) k_wf_shadow_pt(const WfView* __rest
         }
         const Params& P = view_of<ONE>(views, one, v).P;
         int start = __popc(__ballot_sync(0xffffffffu, phase && !k.done && !at));
+        if (STEPS) {
+            while (phase && !k.done) {
+                track_step(P, k, [&]() { ratio_collide(P, R, rng, k, Tr); });
+                if (k.done || 4 * __popc(__activemask()) < start) break;
+            }
+            __syncwarp();
+            continue;
+        }
         for (;;) {
             const bool crossing = phase && !k.done && !at;
             if (few_left(__ballot_sync(0xffffffffu, crossing), start, cross)) break;
@@ -1057,7 +1059,7 @@ cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const Wf
     const uint32_t g1 = (items + 255) / 256 < (uint32_t)sm * 64 ? (items + 255) / 256 : (uint32_t)sm * 64;
     cudaEvent_t t0 = wf_stage_begin(s);
 #define ER_PRIMARY(M, O, F) k_wf_primary<M, ONE, O, F><<<g1, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters)
-#define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2, B.cross_eighths, B.collide_eighths, B.gate_primary)
+#define ER_PRIMARY_PT(M, O) k_wf_primary_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, dseg, nseg, one, one_seg, items, B.results, B.events, B.counters, B.counters + 2)
     if (B.pt_primary) {
         /* delta tracking: persistent lanes, one resident wave */
         if (B.objects) ER_PRIMARY_PT(4, true);
@@ -1118,17 +1120,19 @@ cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const Wf
     wf_stage_end(t0, 1, s);
     t0 = wf_stage_begin(s);
 #define ER_SHADOW(M, O, F) k_wf_shadow<M, ONE, O, F><<<sm * 8, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results)
-#define ER_SHADOW_PT(M, O) k_wf_shadow_pt<M, ONE, O><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.cross_eighths, B.collide_eighths, B.gate_shadow)
+#define ER_SHADOW_PT(M, O) do { \
+        if (steps) k_wf_shadow_pt<M, ONE, O, true><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, 0, 0, 0); \
+        else k_wf_shadow_pt<M, ONE, O, false><<<sm * M, 256, 0, s>>>(d_views, one, B.jobs, B.counters + 1, B.results, B.counters + 3, B.cross_eighths, B.collide_eighths, B.gate_shadow); \
+    } while (0)
     if (B.pt_shadow) {
-        /* ratio-tracked shadows: persistent lanes, one resident wave */
-        if (B.objects) ER_SHADOW_PT(4, true);
-        else {
-            switch (narrow_minb(B.tune_shadow)) {
-            case 2: ER_SHADOW_PT(2, false); break;
-            case 3: ER_SHADOW_PT(3, false); break;
-            case 6: ER_SHADOW_PT(6, false); break;
-            default: ER_SHADOW_PT(4, false); break;
-            }
+        /* ratio-tracked shadows: persistent lanes, one resident wave; in steps
+           up to 16 samples for each of the wave's lanes (figures at k_wf_primary_pt) */
+        const bool steps = items <= 16u * 1024u * (uint32_t)sm;
+        switch (B.objects ? 4 : narrow_minb(B.tune_shadow)) {
+        case 2: ER_SHADOW_PT(2, false); break;
+        case 3: ER_SHADOW_PT(3, false); break;
+        case 6: ER_SHADOW_PT(6, false); break;
+        default: if (B.objects) ER_SHADOW_PT(4, true); else ER_SHADOW_PT(4, false); break;
         }
     } else if (B.objects) {
         if (B.free_flight == WF_DELTA) ER_SHADOW(4, true, WF_DELTA);

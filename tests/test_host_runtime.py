@@ -121,3 +121,17 @@ def test_windows_are_as_few_as_can_be(lib, sizes, cap, want):
         assert batch_info(lib, r, sizes, cap) == want
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("side,spp,steps", [(64, 1, True), (512, 9, True), (1024, 2, True), (512, 10, False), (1024, 8, False)])
+def test_shadow_stage_of_a_small_window_runs_in_steps(lib, side, spp, steps):
+    """up to 16 samples for each lane of the resident wave (152 SMs of 1024)"""
+    sc = S.scene_tiny(res=8, film=(side, side))
+    sc.tracer.settings.free_flight = C.FREE_FLIGHT_DELTA
+    r = renderer(lib, sc)
+    d = np.zeros((side, side, 4), np.float32)
+    log(lib)
+    r.trace_sum_device(d.ctypes.data, spp)
+    names = [e[2] for e in log(lib) if "k_wf_shadow_pt" in e[2]]
+    r.close()
+    assert len(names) == 1 and ("Lb1ELb0ELb1E" if steps else "Lb1ELb0ELb0E") in names[0]
