@@ -230,13 +230,15 @@ struct VolumeItem {
     /* sampled content hash (tuning cache key), made when a key is asked for
        (volume_signature): FNV-1a over the resolution, every 61st voxel as
        bound and what later region edits add.  Until then the edits' bytes wait
-       in sig_log, and sig_base holds the bound voxels' samples from the first
-       edit on.  (Hashing at every bind took 4 of the 7 ms that binding a
-       384x384x256 volume and showing it took.) */
+       in sig_log, and sig_base (sig_host, where the device has no room for it)
+       holds the bound voxels' samples from the first edit on.  (Hashing at
+       every bind took 4 of the 7 ms that binding a 384x384x256 volume and
+       showing it took.) */
     uint64_t signature = 0;
     bool sig_pending = false;
     std::vector<unsigned char> sig_log;
     DevBuf<uint16_t> sig_base;
+    std::vector<uint16_t> sig_host;
     uint64_t edits = 0;            /* region edits from device voxels (folded into the signature) */
     DevBuf<uint16_t> vox;
     DevBuf<uint2> quad;            /* corner quads (NULL when they do not fit in memory) */
@@ -1064,12 +1066,26 @@ std::string tune_cache_path()
     return std::string(home) + "/.cache/exposurerender_gb300/autotune.txt";
 }
 
-/* every 61st voxel of the volume into sig_base */
+/* every 61st voxel of the volume, before its first edit: into sig_base, or
+   without room for that into sig_host, from the volume read in pieces */
 er_status sample_voxels(VolumeItem& v, cudaStream_t s)
 {
+    if (v.sig_base.p || !v.sig_host.empty()) return ER_OK;
     const size_t n = (size_t)v.res[0] * v.res[1] * v.res[2];
-    ER_CUDA(v.sig_base.ensure((n + 60) / 61));
-    ER_CUDA(er_launch_sample_voxels(v.vox.p, n, 61, v.sig_base.p, s));
+    if (v.sig_base.ensure((n + 60) / 61) == cudaSuccess) {
+        ER_CUDA(er_launch_sample_voxels(v.vox.p, n, 61, v.sig_base.p, s));
+        return ER_OK;
+    }
+    cudaGetLastError();
+    std::vector<uint16_t> piece((size_t)61 << 15), all;
+    all.reserve((n + 60) / 61);
+    for (size_t i0 = 0; i0 < n; i0 += piece.size()) {
+        const size_t m = std::min(piece.size(), n - i0);
+        ER_CUDA(cudaMemcpyAsync(piece.data(), v.vox.p + i0, m * sizeof(uint16_t), cudaMemcpyDeviceToHost, s));
+        ER_CUDA(cudaStreamSynchronize(s));
+        for (size_t i = 0; i < m; i += 61) all.push_back(piece[i]);
+    }
+    v.sig_host = std::move(all);
     return ER_OK;
 }
 
@@ -1078,13 +1094,14 @@ er_status volume_signature(VolumeItem& v)
 {
     if (!v.sig_pending) return ER_OK;
     cudaStream_t s = ctx().stream;
-    if (!v.sig_base.p) {
-        const er_status ss = sample_voxels(v, s);
-        if (ss != ER_OK) return ss;
+    const er_status ss = sample_voxels(v, s);
+    if (ss != ER_OK) return ss;
+    std::vector<uint16_t> h = v.sig_host;
+    if (h.empty()) {
+        h.resize(((size_t)v.res[0] * v.res[1] * v.res[2] + 60) / 61);
+        ER_CUDA(cudaMemcpyAsync(h.data(), v.sig_base.p, h.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost, s));
+        ER_CUDA(cudaStreamSynchronize(s));
     }
-    std::vector<uint16_t> h(((size_t)v.res[0] * v.res[1] * v.res[2] + 60) / 61);
-    ER_CUDA(cudaMemcpyAsync(h.data(), v.sig_base.p, h.size() * sizeof(uint16_t), cudaMemcpyDeviceToHost, s));
-    ER_CUDA(cudaStreamSynchronize(s));
     const int32_t res[3] = { v.res[0], v.res[1], v.res[2] };
     uint64_t sig = fnv1a(kFnvBasis, res, sizeof(res));
     sig = fnv1a(sig, h.data(), h.size() * sizeof(uint16_t));
@@ -1093,6 +1110,8 @@ er_status volume_signature(VolumeItem& v)
     v.sig_log.clear();
     v.sig_log.shrink_to_fit();
     v.sig_base.release();
+    v.sig_host.clear();
+    v.sig_host.shrink_to_fit();
     return ER_OK;
 }
 
@@ -1388,6 +1407,7 @@ ER_API er_status er_bind_volume(const er_volume_desc* d, int32_t* id)
     v->sig_pending = true;
     v->sig_log.clear();
     v->sig_base.release();
+    v->sig_host.clear();
     const int lo[3] = { 0, 0, 0 };
     unsigned int vmax = 0;
     er_status us = upload_box(*v, lo, d->resolution, d->voxels, cudaMemcpyHostToDevice, C.stream, &vmax);
@@ -1414,7 +1434,7 @@ static er_status update_volume_region(int32_t id, const int32_t* offset, const i
     }
     /* the volume may be read by queued work: the edit follows it */
     ER_CUDA(cudaStreamSynchronize(C.stream));
-    if (v.sig_pending && !v.sig_base.p) {
+    if (v.sig_pending) {
         const er_status ss = sample_voxels(v, s);
         if (ss != ER_OK) return ss;
     }
@@ -1439,9 +1459,9 @@ static er_status update_volume_region(int32_t id, const int32_t* offset, const i
         v.edits++;
         sign(&v.edits, sizeof(v.edits));
     }
-    if (v.sig_log.size() > ((size_t)1 << 20)) us = volume_signature(v);
-    if (us != ER_OK) return us;
     C.version++;
+    /* the edit stands whether or not the key can be made now: it waits on */
+    if (v.sig_log.size() > ((size_t)1 << 20)) volume_signature(v);
     return ER_OK;
 }
 

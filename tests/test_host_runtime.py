@@ -135,3 +135,58 @@ def test_shadow_stage_of_a_small_window_runs_in_steps(lib, side, spp, steps):
     names = [e[2] for e in log(lib) if "k_wf_shadow_pt" in e[2]]
     r.close()
     assert len(names) == 1 and ("Lb1ELb0ELb1E" if steps else "Lb1ELb0ELb0E") in names[0]
+
+
+def edit(lib, r, box, value):
+    off, size = (ctypes.c_int32 * 3)(*box[0]), (ctypes.c_int32 * 3)(*box[1])
+    v = np.full(box[1][::-1], value, np.uint16)
+    return lib.er_update_volume_region(r.volume_id, off, size, v.ctypes.data)
+
+
+def tune_key(lib, r, path):
+    """the key under which the autotuner stores its choice"""
+    r.autotune(1)
+    with open(path) as f:
+        return f.read().split()[-7]
+
+
+BOXES = [((0, 0, 0), (30, 4, 4)), ((5, 6, 7), (20, 11, 3)), ((3, 6, 7), (20, 11, 9))]
+
+
+@pytest.mark.parametrize("memory", [True, False], ids=["room", "no-room"])
+def test_tuning_key_made_late_equals_one_made_at_once(lib, monkeypatch, tmp_path, memory):
+    """a bind and its edits give the key that they give when the key is made
+    after the bind, also when the device has no room for what the key needs"""
+    keys = []
+    for late in (False, True):
+        path = tmp_path / f"{late}.txt"
+        monkeypatch.setenv("ER_TUNE_CACHE", str(path))
+        sc = S.scene_tiny(res=32, film=(8, 8), seed=5)
+        r = renderer(lib, sc)
+        if not late:
+            tune_key(lib, r, path)
+        lib.fake_no_memory(0 if memory else 1)
+        for i, box in enumerate(BOXES):
+            C.check(edit(lib, r, box, 100 + i))
+        lib.fake_no_memory(0)
+        keys.append(tune_key(lib, r, path))
+        r.close()
+    assert keys[0] == keys[1]
+
+
+def test_an_edit_stands_when_its_key_cannot_be_made(lib):
+    """edits whose log is over a megabyte make the key: a failure there leaves
+    the edit made, and the next render with its tables"""
+    n = 256
+    sc = S.scene_tiny(res=8, film=(8, 8))
+    sc.volume = np.zeros((n, n, n), np.uint16)
+    r = renderer(lib, sc)
+    d = np.zeros((8, 8, 4), np.float32)
+    r.trace_sum_device(d.ctypes.data, 1)
+    lib.fake_bad_read((n ** 3 + 60) // 61 * 2)
+    for i in range(2):
+        assert edit(lib, r, ((0, 0, 0), (n, n, n)), i) == C.ER_OK
+        log(lib)
+        r.trace_sum_device(d.ctypes.data, 1)
+        assert any("k_sigma_table" in e[2] for e in log(lib) if e[0] == "launch")
+    r.close()
