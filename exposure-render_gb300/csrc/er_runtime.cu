@@ -1115,7 +1115,12 @@ er_status volume_signature(VolumeItem& v)
     return ER_OK;
 }
 
-/* device, volume content and every setting that changes the work of a sample */
+/* what the tracking and shade stages are: another number whenever a change to
+   them can change which choice is the fastest, so that choices timed on other
+   kernels are not taken from the cache */
+constexpr uint32_t kTuneKernels = 2;
+
+/* kernels, device, volume content and every setting that changes the work of a sample */
 uint64_t tune_key(const TracerItem& t, const VolumeItem& v, int probe_spp)
 {
     cudaDeviceProp prop;
@@ -1123,7 +1128,8 @@ uint64_t tune_key(const TracerItem& t, const VolumeItem& v, int probe_spp)
     int dev = 0;
     cudaGetDevice(&dev);
     cudaGetDeviceProperties(&prop, dev);
-    uint64_t h = fnv1a(kFnvBasis, prop.name, strnlen(prop.name, sizeof(prop.name)));
+    uint64_t h = fnv1a(kFnvBasis, &kTuneKernels, sizeof(kTuneKernels));
+    h = fnv1a(h, prop.name, strnlen(prop.name, sizeof(prop.name)));
     h = fnv1a(h, &prop.multiProcessorCount, sizeof(int));
     h = fnv1a(h, &v.signature, sizeof(v.signature));
     h = fnv1a(h, v.spacing, sizeof(v.spacing));

@@ -190,3 +190,29 @@ def test_an_edit_stands_when_its_key_cannot_be_made(lib):
         r.trace_sum_device(d.ctypes.data, 1)
         assert any("k_sigma_table" in e[2] for e in log(lib) if e[0] == "launch")
     r.close()
+
+
+def fnv1a(h, b):
+    for x in bytes(b):
+        h = ((h ^ x) * 1099511628211) % (1 << 64)
+    return h
+
+
+def test_choices_timed_on_other_kernels_are_not_taken(lib, tmp_path):
+    """a cache line under the key without the kernels' number (device, volume,
+    settings) is not applied"""
+    sc = S.scene_tiny(res=16, film=(8, 8), seed=5)
+    r = renderer(lib, sc)
+    t = r.tracer_desc
+    s = C.er_render_settings.from_buffer_copy(t.settings)
+    for f in ("majorant_brick", "tune_primary", "tune_shadow", "tune_shade", "tune_stages", "seed", "bilateral", "bilateral_radius", "frame_filter"):
+        setattr(s, f, 0)
+    s.bilateral_sigma_d = s.bilateral_sigma_r = 0.0
+    i32 = lambda *v: np.array(v, np.int32).tobytes()
+    volume = fnv1a(fnv1a(14695981039346656037, i32(16, 16, 16)), sc.volume.ravel()[::61].astype(np.uint16).tobytes())
+    h = fnv1a(14695981039346656037, b"no GPU" + i32(152) + volume.to_bytes(8, "little") + np.array(sc.spacing, np.float32).tobytes())
+    h = fnv1a(h, bytes(s) + bytes(t.opacity) + bytes(t.glossiness) + i32(t.camera.film_size[0], t.camera.film_size[1], t.light_count, 1))
+    (tmp_path / "autotune.txt").write_text(f"{h:016x} 8 2 2 2 1.000 0\n")
+    assert not r.autotune(1)["from_cache"]
+    assert r.autotune(1)["from_cache"]
+    r.close()
