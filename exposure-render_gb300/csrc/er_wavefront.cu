@@ -1071,26 +1071,33 @@ cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const Wf
             default: ER_PRIMARY_PT(4, false); break;
             }
         }
-    } else if (B.objects) {
-        if (B.free_flight == WF_DELTA) ER_PRIMARY(4, true, WF_DELTA);
-        else if (B.free_flight == WF_MARCH) ER_PRIMARY(4, true, WF_MARCH);
-        else ER_PRIMARY(4, true, WF_MIXED);
     } else if (B.free_flight == WF_DELTA) {
-        switch (narrow_minb(B.tune_primary)) {
+        if (B.objects) ER_PRIMARY(4, true, WF_DELTA);
+        else switch (narrow_minb(B.tune_primary)) {
         case 2: ER_PRIMARY(2, false, WF_DELTA); break;
         case 3: ER_PRIMARY(3, false, WF_DELTA); break;
         case 6: ER_PRIMARY(6, false, WF_DELTA); break;
         default: ER_PRIMARY(4, false, WF_DELTA); break;
         }
-    } else if (B.free_flight == WF_MARCH) {
-        switch (B.tune_primary) {
+    } else if (ONE || B.free_flight == WF_MARCH) {
+        if (B.objects) ER_PRIMARY(4, true, WF_MARCH);
+        else switch (B.tune_primary) {
         case 2: ER_PRIMARY(2, false, WF_MARCH); break;
         case 3: ER_PRIMARY(3, false, WF_MARCH); break;
         case 6: ER_PRIMARY(6, false, WF_MARCH); break;
         case 8: ER_PRIMARY(8, false, WF_MARCH); break;
         default: ER_PRIMARY(4, false, WF_MARCH); break;
         }
-    } else ER_PRIMARY(4, false, WF_MIXED);
+    } else if constexpr (!ONE) {
+        if (B.objects) ER_PRIMARY(4, true, WF_MIXED);
+        else switch (B.tune_primary) {
+        case 2: ER_PRIMARY(2, false, WF_MIXED); break;
+        case 3: ER_PRIMARY(3, false, WF_MIXED); break;
+        case 6: ER_PRIMARY(6, false, WF_MIXED); break;
+        case 8: ER_PRIMARY(8, false, WF_MIXED); break;
+        default: ER_PRIMARY(4, false, WF_MIXED); break;
+        }
+    }
 #undef ER_PRIMARY_PT
 #undef ER_PRIMARY
     wf_stage_end(t0, 0, s);
@@ -1134,26 +1141,33 @@ cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const Wf
         case 6: ER_SHADOW_PT(6, false); break;
         default: if (B.objects) ER_SHADOW_PT(4, true); else ER_SHADOW_PT(4, false); break;
         }
-    } else if (B.objects) {
-        if (B.free_flight == WF_DELTA) ER_SHADOW(4, true, WF_DELTA);
-        else if (B.free_flight == WF_MARCH) ER_SHADOW(4, true, WF_MARCH);
-        else ER_SHADOW(4, true, WF_MIXED);
     } else if (B.free_flight == WF_DELTA) {
-        switch (narrow_minb(B.tune_shadow)) {
+        if (B.objects) ER_SHADOW(4, true, WF_DELTA);
+        else switch (narrow_minb(B.tune_shadow)) {
         case 2: ER_SHADOW(2, false, WF_DELTA); break;
         case 3: ER_SHADOW(3, false, WF_DELTA); break;
         case 6: ER_SHADOW(6, false, WF_DELTA); break;
         default: ER_SHADOW(4, false, WF_DELTA); break;
         }
-    } else if (B.free_flight == WF_MARCH) {
-        switch (B.tune_shadow) {
+    } else if (ONE || B.free_flight == WF_MARCH) {
+        if (B.objects) ER_SHADOW(4, true, WF_MARCH);
+        else switch (B.tune_shadow) {
         case 2: ER_SHADOW(2, false, WF_MARCH); break;
         case 3: ER_SHADOW(3, false, WF_MARCH); break;
         case 6: ER_SHADOW(6, false, WF_MARCH); break;
         case 8: ER_SHADOW(8, false, WF_MARCH); break;
         default: ER_SHADOW(4, false, WF_MARCH); break;
         }
-    } else ER_SHADOW(4, false, WF_MIXED);
+    } else if constexpr (!ONE) {
+        if (B.objects) ER_SHADOW(4, true, WF_MIXED);
+        else switch (B.tune_shadow) {
+        case 2: ER_SHADOW(2, false, WF_MIXED); break;
+        case 3: ER_SHADOW(3, false, WF_MIXED); break;
+        case 6: ER_SHADOW(6, false, WF_MIXED); break;
+        case 8: ER_SHADOW(8, false, WF_MIXED); break;
+        default: ER_SHADOW(4, false, WF_MIXED); break;
+        }
+    }
 #undef ER_SHADOW_PT
 #undef ER_SHADOW
     wf_stage_end(t0, 2, s);
@@ -1172,10 +1186,12 @@ cudaError_t launch_window(const WfView* d_views, const WfSegment* dseg, const Wf
 
 #ifndef WF_BATCH_UNIT
 
-/* one window of one view with its parameters by value */
+/* one window of one view with its parameters by value; a window of a batch
+   that mixes estimators has its view's own */
 cudaError_t wf_launch_window_one(const WfView* d_view, const WfView& view, const WavefrontPlan& plan, int w, int seg,
-                                 const WavefrontBuffers& B, cudaStream_t s)
+                                 WavefrontBuffers B, cudaStream_t s)
 {
+    B.free_flight = view.P.free_flight == 1 ? WF_DELTA : WF_MARCH;
     return launch_window<true>(d_view, nullptr, view, plan, w, seg, seg + 1, B, s);
 }
 
@@ -1223,7 +1239,7 @@ cudaError_t er_wavefront_profile_read(double* ms, int64_t* launches)
 #else
 
 cudaError_t wf_launch_window_one(const WfView* d_view, const WfView& view, const WavefrontPlan& plan, int w, int seg,
-                                 const WavefrontBuffers& B, cudaStream_t s);
+                                 WavefrontBuffers B, cudaStream_t s);
 
 /* A window that holds one view runs the one-view kernels, whose parameters
    come from the constant bank instead of loads from the table at every brick

@@ -151,6 +151,33 @@ def test_batch_tuning_variants_equal(torch, lib, pair):
     C.check(lib.er_batch_destroy(bid))
 
 
+@pytest.mark.parametrize("delta", [0, 1], ids=["march", "delta"])
+@pytest.mark.parametrize("stages", [C.PERSISTENT_SHADOW, C.PERSISTENT_BOTH, C.PERSISTENT_NONE])
+def test_batch_tuning_variants_of_one_estimator(torch, lib, runtime, delta, stages):
+    """views of tracers that all march or all track: the occupancy variants of
+    their own kernels, and of the mixed ones above, give the same sums"""
+    rs = []
+    for seed in (3, 4):
+        sc = S.scene_tiny(res=24, film=(40, 32), seed=seed)
+        sc.tracer.settings.free_flight = sc.tracer.settings.mis = delta
+        rs.append(runtime.Renderer(sc, lib))
+    table = view_table(*rs)
+    ref = expected(torch, lib, table)
+    bid, outs = make_batch(torch, lib, table, 0, 2000)
+    C.check(lib.er_batch_set_stages(bid, stages))
+    for p, s in [(2, 8), (3, 6), (6, 3), (8, 2), (4, 4)]:
+        C.check(lib.er_batch_set_tuning(bid, p, s))
+        for d in outs:
+            d.zero_()
+        C.check(lib.er_batch_launch(bid, None))
+        torch.cuda.synchronize()
+        for k, d in enumerate(outs):
+            assert np.array_equal(bits(d.cpu().numpy()), bits(ref[k])), f"tuning {p}/{s} view {k}"
+    C.check(lib.er_batch_destroy(bid))
+    for r in rs:
+        r.close()
+
+
 def test_batch_progressive_accumulation(torch, lib, pair):
     """launch, advance by spp, launch == two accumulating one-view calls"""
     ra, rb = pair

@@ -216,3 +216,29 @@ def test_choices_timed_on_other_kernels_are_not_taken(lib, tmp_path):
     assert not r.autotune(1)["from_cache"]
     assert r.autotune(1)["from_cache"]
     r.close()
+
+
+@pytest.mark.parametrize("tune", [2, 3, 4, 6, 8])
+@pytest.mark.parametrize("mix", ["march", "delta", "both"])
+def test_batch_tuning_picks_the_kernels(lib, mix, tune):
+    """er_batch_set_tuning names the occupancy of the tracking stages in every
+    batch; 8 is a variant of the batches that march"""
+    runtime = importlib.import_module("exposure-render_gb300.runtime")
+    kinds = {"march": (0, 0), "delta": (1, 1), "both": (0, 1)}[mix]
+    rs = []
+    for k in kinds:
+        sc = S.scene_tiny(res=8, film=(8, 8))
+        sc.tracer.settings.free_flight = k
+        sc.tracer.settings.tune_stages = C.PERSISTENT_NONE
+        rs.append(renderer(lib, sc))
+    b = runtime.Batch([(r.tracer_id, 2, 0x100000 * (i + 1), None) for i, r in enumerate(rs)], flags=0, lib=lib)
+    b.set_tuning(tune, tune)
+    log(lib)
+    b.launch()
+    names = [e[2] for e in log(lib) if e[0] == "launch"]
+    want = 4 if mix == "delta" and tune == 8 else tune
+    for stage in ("k_wf_primary", "k_wf_shadow"):
+        assert [n.split("ILi")[1].split("E")[0] for n in names if stage + "I" in n] == [str(want)], names
+    b.close()
+    for r in rs:
+        r.close()
