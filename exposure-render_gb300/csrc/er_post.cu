@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(256) k_bilateral(const uchar4* __restrict__ in
     const int r = T.radius;
     const int span = BIL_N + 2 * r;
     float* lum = (float*)(tile + span * BIL_M);
-    const int n0 = blockIdx.x * BIL_N, m0 = blockIdx.y * BIL_M;
+    /* the grid's x is the film's, of any width; its y the film's rows */
+    const int n0 = (HORIZONTAL ? blockIdx.x : blockIdx.y) * BIL_N, m0 = (HORIZONTAL ? blockIdx.y : blockIdx.x) * BIL_M;
     const int N = HORIZONTAL ? W : H, M = HORIZONTAL ? H : W;
     range[threadIdx.x] = T.range[threadIdx.x];
     /* neighbouring threads read neighbouring pixels of the film's rows */
@@ -386,7 +387,7 @@ cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int 
 {
     /* radius <= 127: at most 318 * 16 * 8 B = 40.7 KB */
     const size_t bytes = (size_t)(BIL_N + 2 * T.radius) * BIL_M * 8;
-    const dim3 gh((W + BIL_N - 1) / BIL_N, (H + BIL_M - 1) / BIL_M), gv((H + BIL_N - 1) / BIL_N, (W + BIL_M - 1) / BIL_M);
+    const dim3 gh((W + BIL_N - 1) / BIL_N, (H + BIL_M - 1) / BIL_M), gv((W + BIL_M - 1) / BIL_M, (H + BIL_N - 1) / BIL_N);
     k_bilateral<true><<<gh, 256, bytes, s>>>(in, tmp, W, H, T);
     k_bilateral<false><<<gv, 256, bytes, s>>>(tmp, out, W, H, T);
     return cudaGetLastError();

@@ -189,6 +189,19 @@ def test_bilateral_tiles(env, oracle, w, h, radius):
     assert np.array_equal(t.cpu().numpy(), tmp) and np.array_equal(o.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("w,h", [(65535 * 16 + 1, 1), (65535 * 16 + 20, 3), (2, 524280)])
+def test_bilateral_of_very_wide_and_tall_images(env, oracle, w, h):
+    """more columns than a grid has rows of tiles, and as many rows as an image may have"""
+    torch, lib, _ = env
+    img = np.random.default_rng(w).integers(0, 256, size=(h, w, 4), dtype=np.uint8)
+    want, tmp = np.zeros_like(img), np.zeros_like(img)
+    oracle.bilateral(OL.ptr(img), OL.ptr(tmp), OL.ptr(want), w, h, 2, 1.5, 20.0)
+    d, t, o = torch.from_numpy(img).cuda(), torch.zeros((h, w, 4), dtype=torch.uint8, device="cuda"), torch.zeros((h, w, 4), dtype=torch.uint8, device="cuda")
+    C.check(lib.er_bilateral_device(d.data_ptr(), t.data_ptr(), o.data_ptr(), w, h, 2, 1.5, 20.0, None))
+    torch.cuda.synchronize()
+    assert np.array_equal(t.cpu().numpy(), tmp) and np.array_equal(o.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("stages", [0, 1])
 @pytest.mark.parametrize("flags", [0, C.ER_BATCH_GRAPH])
 def test_batch_windows_of_one_view(env, stages, flags):
