@@ -41,9 +41,9 @@ cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int 
 cudaError_t er_launch_gradient_magnitude(const erd::Params& P, uint16_t* gm, unsigned int* max_bits, cudaStream_t s);
 /* the largest gradient magnitude alone (as er_launch_gradient_magnitude) of a
    volume it applies to, whose largest voxel is vmax: bits[0], if
-   er_gradient_max_found(bits[1]); two words, zero before */
-bool er_gradient_max_applies(const erd::Params& P);
-bool er_gradient_max_found(const erd::Params& P, int vmax, unsigned int low_bits);
+   er_gradient_max_found; four words, zero before */
+bool er_gradient_max_applies(const erd::Params& P, int vmax);
+bool er_gradient_max_found(const erd::Params& P, int vmax, const unsigned int bits[4]);
 cudaError_t er_launch_gradient_max(const erd::Params& P, int vmax, unsigned int* bits, cudaStream_t s);
 /* every step-th of n voxels into out */
 cudaError_t er_launch_sample_voxels(const uint16_t* vox, size_t n, int step, uint16_t* out, cudaStream_t s);

@@ -225,6 +225,9 @@ ER_D float voxel_gradient_magnitude(const Params& P, int X, int Y, int Z)
     return gradient_magnitude(P, p);
 }
 
+/* out of line: the pass that looks few voxels up keeps its registers for the walk */
+static __device__ __noinline__ float voxel_gradient_magnitude_c(const Params& P, int X, int Y, int Z) { return voxel_gradient_magnitude(P, X, Y, Z); }
+
 /* per-voxel gradient magnitude at voxel centres + max; the magnitude volume
    (optional) saturates at 65535 */
 __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, unsigned int* __restrict__ max_bits)
@@ -255,19 +258,26 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    with one spacing on all axes.  A voxel's six lookups lie (but for rounding)
    at its neighbours' centres, where the blend is the mean of a cell's eight
    voxels: integer sums give each magnitude to within a known error, and only
-   the voxels that may hold the maximum make their six lookups.  Two passes:
-   the largest lower bound, then the exact magnitudes of the voxels whose
-   upper bound reaches it.  tol: how far a lookup may be from its cell's mean
-   (three truncations, the weights' rounding).  Where the largest lower bound
-   is not well above that error (flat volumes, labels) most voxels would need
-   their lookups, and the exact pass leaves the volume to
-   k_gradient_magnitude (gm_bounds_tell).
+   the voxels that may hold the maximum make their six lookups: a pass for the
+   largest lower bound, then the exact magnitudes of the voxels whose upper
+   bound reaches it.  tol: how far a lookup may be from its cell's mean (three
+   truncations, the weights' rounding).
+
+   That pays where few voxels reach the bound.  Where the largest lower bound
+   is not well above the error (flat and smooth volumes: gm_bounds_tell) most
+   would, and where many do all the same (a volume of one slope) the exact pass
+   stops at a 64th of them: the volume is left to k_gradient_magnitude.  In
+   large grids an eighth of the blocks, spread over the volume, bounds first,
+   and the rest only if that tells; a volume whose values are all within the
+   error (a few labels) is not asked.  With and without the two passes, ms at
+   512^3: shells 1.6 and 4.3, one slope 5.2 and 4.3 (6.2 before it stopped),
+   smooth 4.43 and 4.32 (4.89 with all blocks first), eight labels 4.3 and 4.3
+   (4.9); at 300^3 shells 0.33 and 0.93, smooth 1.07 and 0.92.
 
    A block walks GM_Z planes of a GM_X x GM_Y tile of cells (a ring of halo
    around the voxels): a thread sums its cell's four voxels of a plane, adds
-   the plane before, and shares three planes of cell sums.  Bound by the read
-   of the volume.  Every voxel's six lookups took 1213 us at 384x384x256 and
-   4304 us at 512^3. */
+   the plane before, and shares three planes of cell sums.  Every voxel's six
+   lookups take 1213 us at 384x384x256. */
 #define GM_X 32
 #define GM_Y 16
 #define GM_Z 32
@@ -277,10 +287,22 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    blobs went the long way) */
 __host__ __device__ inline bool gm_bounds_tell(float low, float tol, float h) { return low > 3.0f * 2.0f * 1.7320508f * tol * h; }
 
-template <bool EXACT>
-__global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float tol, const unsigned int* low_in, unsigned int* out_bits)
+/* the exact pass in a grid of many waves (GM_EXACT_WIDE) at four blocks an SM,
+   its lookups out of line (all passes at 512^3 1.84 -> 1.58 ms); in a smaller
+   grid, where a block's own time counts, inline (128^3: 75 against 87 us) */
+enum { GM_FIRST = 0, GM_REST = 1, GM_EXACT = 2, GM_EXACT_WIDE = 3 };
+
+/* bits: the largest magnitude, voxels looked up, the largest lower bound of the
+   first pass and of the rest (two words: a pass decides on words that it does
+   not write, so that a block's threads all decide the same) */
+template <int PASS>
+__global__ void __launch_bounds__(GM_X * GM_Y, PASS == GM_EXACT_WIDE ? 4 : 1) k_gm_cells(const Params P, float tol, unsigned int share, unsigned int most,
+                                                              unsigned int* bits)
 {
+    constexpr bool EXACT = PASS >= GM_EXACT;
     __shared__ int cells[3][GM_Y][GM_X];
+    __shared__ int stop;
+    if (!EXACT && ((blockIdx.x + blockIdx.y + blockIdx.z) % share == 0) != (PASS == GM_FIRST)) return;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int X = (int)blockIdx.x * (GM_X - 2) - 1 + tx, Y = (int)blockIdx.y * (GM_Y - 2) - 1 + ty;
     const int z0 = (int)blockIdx.z * GM_Z, z1 = min(z0 + GM_Z, P.res[2]);
@@ -293,17 +315,25 @@ __global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float 
     };
     const bool inner = tx > 0 && tx < GM_X - 1 && ty > 0 && ty < GM_Y - 1 && X < P.res[0] && Y < P.res[1];
     const float h = 0.5f / P.spacing[0];
-    const float low = EXACT ? __uint_as_float(*low_in) : 0.0f;
-    if (EXACT && !gm_bounds_tell(low, tol, h)) return;
+    const float low = PASS == GM_FIRST ? 0.0f : __uint_as_float(EXACT ? max(bits[2], bits[3]) : bits[2]);
+    if (PASS != GM_FIRST && !gm_bounds_tell(low, tol, h)) return;
     unsigned int best = 0;
+    /* voxels looked up so far: read a plane ahead, so that nobody waits for it */
+    const bool asks = EXACT && tx == 0 && ty == 0;
+    unsigned int seen = 0;
+    if (asks) stop = 0;
     int prev = plane(z0 - 1);
     /* cell z is in cells[(z + 3) % 3]; voxel z needs cells z - 1, z and z + 1 */
     for (int z = z0 - 1; z <= z1; z++) {
         const int next = plane(z + 1);
         cells[(z + 3) % 3][ty][tx] = prev + next;
         prev = next;
+        if (asks && seen > most) stop = 1;
+        if (asks) seen = *(volatile unsigned int*)(bits + 1);
         __syncthreads();
+        if (EXACT && stop) return;
         const int Z = z - 1;
+        bool look = false;
         if (Z >= z0 && inner) {
             const int c = (Z + 3) % 3;
             const float dx = fabsf((float)(cells[c][ty][tx - 1] - cells[c][ty][tx + 1])) * 0.125f;
@@ -311,17 +341,22 @@ __global__ void __launch_bounds__(GM_X * GM_Y) k_gm_cells(const Params P, float 
             const float dz = fabsf((float)(cells[(Z + 2) % 3][ty][tx] - cells[(Z + 4) % 3][ty][tx])) * 0.125f;
             if (EXACT) {
                 const float a = (dx + 2.0f * tol) * h, b = (dy + 2.0f * tol) * h, e = (dz + 2.0f * tol) * h;
-                if (sqrtf(a * a + b * b + e * e) * 1.00001f >= low) best = max(best, __float_as_uint(voxel_gradient_magnitude(P, X, Y, Z)));
+                look = sqrtf(a * a + b * b + e * e) * 1.00001f >= low;
             } else {
                 const float a = fmaxf(dx - 2.0f * tol, 0.0f) * h, b = fmaxf(dy - 2.0f * tol, 0.0f) * h, e = fmaxf(dz - 2.0f * tol, 0.0f) * h;
                 best = max(best, __float_as_uint(sqrtf(a * a + b * b + e * e) * 0.99999f));
             }
         }
+        if (EXACT) {
+            const unsigned m = __ballot_sync(0xffffffffu, look);
+            if (tx == 0 && m) atomicAdd(bits + 1, (unsigned int)__popc(m));
+            if (look) best = max(best, __float_as_uint(PASS == GM_EXACT ? voxel_gradient_magnitude(P, X, Y, Z) : voxel_gradient_magnitude_c(P, X, Y, Z)));
+        }
         /* the next plane overwrites cell z - 2, which voxel z - 1 has read */
         __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (tx == 0 && best) atomicMax(out_bits, best);
+    if (tx == 0 && best) atomicMax(bits + (EXACT ? 0 : 2 + PASS), best);
 }
 
 __global__ void k_math_eval(int fn, int n, const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out)
@@ -401,13 +436,6 @@ cudaError_t er_launch_gradient_magnitude(const Params& P, uint16_t* gm, unsigned
     return cudaGetLastError();
 }
 
-bool er_gradient_max_applies(const Params& P)
-{
-    /* the mean's argument: one spacing, weights within a tenth of a half, and grids within the launch limits */
-    const int most = P.res[0] > P.res[1] ? (P.res[0] > P.res[2] ? P.res[0] : P.res[2]) : (P.res[1] > P.res[2] ? P.res[1] : P.res[2]);
-    return P.spacing[0] == P.spacing[1] && P.spacing[1] == P.spacing[2] && P.spacing[0] > 0.0f && most <= 50000;
-}
-
 static float gradient_max_tol(const Params& P, int vmax)
 {
     int most = P.res[0];
@@ -416,18 +444,40 @@ static float gradient_max_tol(const Params& P, int vmax)
     return 3.5f + 3e-6f * (float)most * (float)vmax;
 }
 
-bool er_gradient_max_found(const Params& P, int vmax, unsigned int low_bits)
+static unsigned int gradient_max_most(const Params& P)
 {
+    const unsigned long long n = (unsigned long long)P.res[0] * P.res[1] * P.res[2] / 64;
+    return n < 0x7fffffffull ? (unsigned int)n + 1024u : 0x7fffffffu;
+}
+
+bool er_gradient_max_applies(const Params& P, int vmax)
+{
+    /* the mean's argument: one spacing, weights within a tenth of a half, and grids within the launch limits */
+    const int most = P.res[0] > P.res[1] ? (P.res[0] > P.res[2] ? P.res[0] : P.res[2]) : (P.res[1] > P.res[2] ? P.res[1] : P.res[2]);
+    /* no lower bound is above sqrt(3) (vmax - 2 tol) h: up to 8 tol none tells */
+    return P.spacing[0] == P.spacing[1] && P.spacing[1] == P.spacing[2] && P.spacing[0] > 0.0f && most <= 50000 &&
+           (float)vmax > 8.0f * gradient_max_tol(P, vmax);
+}
+
+bool er_gradient_max_found(const Params& P, int vmax, const unsigned int bits[4])
+{
+    const unsigned int low_bits = bits[2] > bits[3] ? bits[2] : bits[3];
     float low;
     memcpy(&low, &low_bits, sizeof(low));
-    return gm_bounds_tell(low, gradient_max_tol(P, vmax), 0.5f / P.spacing[0]);
+    return gm_bounds_tell(low, gradient_max_tol(P, vmax), 0.5f / P.spacing[0]) && bits[1] <= gradient_max_most(P);
 }
 
 cudaError_t er_launch_gradient_max(const Params& P, int vmax, unsigned int* bits, cudaStream_t s)
 {
     const float tol = gradient_max_tol(P, vmax);
+    const unsigned int most = gradient_max_most(P);
     const dim3 b(GM_X, GM_Y), g((P.res[0] + GM_X - 3) / (GM_X - 2), (P.res[1] + GM_Y - 3) / (GM_Y - 2), (P.res[2] + GM_Z - 1) / GM_Z);
-    k_gm_cells<false><<<g, b, 0, s>>>(P, tol, nullptr, bits + 1);
-    k_gm_cells<true><<<g, b, 0, s>>>(P, tol, bits + 1, bits);
+    /* a grid of few waves takes about as long for an eighth of its blocks */
+    const size_t blocks = (size_t)g.x * g.y * g.z;
+    const unsigned int share = blocks < 8192 ? 1 : 8;
+    k_gm_cells<GM_FIRST><<<g, b, 0, s>>>(P, tol, share, most, bits);
+    if (share > 1) k_gm_cells<GM_REST><<<g, b, 0, s>>>(P, tol, share, most, bits);
+    if (blocks < 1024) k_gm_cells<GM_EXACT><<<g, b, 0, s>>>(P, tol, share, most, bits);
+    else k_gm_cells<GM_EXACT_WIDE><<<g, b, 0, s>>>(P, tol, share, most, bits);
     return cudaGetLastError();
 }

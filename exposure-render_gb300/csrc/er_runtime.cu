@@ -2295,20 +2295,20 @@ ER_API er_status er_gradient_magnitude(int32_t volume_id, uint16_t* d_gm, float*
     erd::Params P;
     memset(&P, 0, sizeof(P));
     volume_geometry(v, P);
-    ER_CUDA(v.gm_max_bits.ensure(2));
+    ER_CUDA(v.gm_max_bits.ensure(4));
     cudaStream_t s = ctx().stream;
-    ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, 2 * sizeof(unsigned int), s));
-    unsigned int bits[2] = { 0u, 0u };
+    ER_CUDA(cudaMemsetAsync(v.gm_max_bits.p, 0, 4 * sizeof(unsigned int), s));
+    unsigned int bits[4] = { 0u, 0u, 0u, 0u };
     auto read = [&]() -> cudaError_t {
         const cudaError_t e = cudaMemcpyAsync(bits, v.gm_max_bits.p, sizeof(bits), cudaMemcpyDeviceToHost, s);
         return e != cudaSuccess ? e : cudaStreamSynchronize(s);
     };
-    const bool bounds = !d_gm && er_gradient_max_applies(P);
+    const bool bounds = !d_gm && er_gradient_max_applies(P, (int)v.vmax);
     if (bounds) {
         ER_CUDA(er_launch_gradient_max(P, (int)v.vmax, v.gm_max_bits.p, s));
         ER_CUDA(read());
     }
-    if (!bounds || !er_gradient_max_found(P, (int)v.vmax, bits[1])) {
+    if (!bounds || !er_gradient_max_found(P, (int)v.vmax, bits)) {
         ER_CUDA(er_launch_gradient_magnitude(P, d_gm, v.gm_max_bits.p, s));
         ER_CUDA(read());
     }

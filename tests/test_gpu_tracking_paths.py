@@ -153,6 +153,28 @@ def test_gradient_maximum_equals_the_full_pass(env, shape, spacing, kind):
         r.close()
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (33, 14, 30), (70, 61, 100)])
+@pytest.mark.parametrize("kind", ["labels", "more labels", "smooth", "slope", "corner"])
+def test_gradient_maximum_of_volumes_without_few_candidates(env, shape, kind):
+    """few labels, smooth and evenly sloped volumes (most voxels hold nearly the
+    maximum), and one whose only slope is in the last block"""
+    torch, lib, runtime = env
+    z, y, x = np.indices(shape)
+    tri = lambda a: np.abs(a % 32 - 16) * 40
+    v = {"labels": np.random.default_rng(3).integers(0, 8, size=shape), "more labels": np.random.default_rng(3).integers(0, 40, size=shape),
+         "smooth": 3000 + 900 * np.sin(x / 30.0) + 900 * np.cos(y / 40.0 + z / 50.0), "slope": tri(x) + tri(y) + tri(z),
+         "corner": 1000 + 3000 * ((x >= shape[2] - 2) & (y >= shape[1] - 2) & (z >= shape[0] - 2))}[kind].astype(np.uint16)
+    sc = S.scene_tiny(film=(8, 8))
+    sc.volume = v
+    r = runtime.Renderer(sc, lib)
+    try:
+        gm = torch.zeros(shape, dtype=torch.int16, device="cuda")
+        full = r.gradient_magnitude(gm.data_ptr())
+        assert r.gradient_magnitude() == full
+    finally:
+        r.close()
+
+
 @pytest.mark.parametrize("shape,brick", [((1, 1, 1), 1), ((2, 2, 2), 1), ((5, 3, 321), 1), ((5, 3, 322), 1), ((9, 7, 640), 2), ((4, 5, 641), 3),
                                          ((65, 66, 130), 64), ((129, 4, 129), 64), ((40, 33, 31), 5)])
 def test_majorant_grid_ragged(env, oracle, shape, brick):

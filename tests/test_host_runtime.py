@@ -242,3 +242,12 @@ def test_batch_tuning_picks_the_kernels(lib, mix, tune):
     b.close()
     for r in rs:
         r.close()
+
+
+def test_gradient_maximum_of_small_values_goes_one_way(lib):
+    """a volume whose values are within the bounds' error makes the full pass alone"""
+    r = renderer(lib, S.scene_tiny(res=16, film=(8, 8)))
+    log(lib)
+    r.gradient_magnitude()
+    assert len([e for e in log(lib) if e[0] == "launch"]) == 1
+    r.close()
