@@ -7,8 +7,8 @@
  *                    in [b B, (b + 1) B] can blend with a nonzero weight (the
  *                    trackers clamp their lookups to that range,
  *                    er_path.cuh sigma_point_in_brick).
- *   k_rmq          : sparse table of running maxima over the sigma table
- *                    (sigma[I] = DensityScale * Opacity(I)).
+ *   k_rmq, k_rmq_tile, k_rmq_level : sparse table of running maxima over the
+ *                    sigma table (sigma[I] = DensityScale * Opacity(I)).
  *   k_majorant     : majorant[brick] = DensityScale * max sigma[lo..hi].
  *   k_skip_x, _yz  : distances to the nearest non-empty brick.
  *   k_occupancy    : the empty bricks of the fixed-step march.
@@ -115,10 +115,13 @@ __global__ void __launch_bounds__(BM_THREADS) k_brick_minmax(const uint16_t* __r
     }
 }
 
-/* the sparse table of running maxima, level 0 a copy of the sigma table, by
-   one block: a level needs the one before it, and at n <= 65536 a level is a
-   few iterations of the block (a launch a level cost 3 us each, 33 us at
-   n = 2600) */
+/* The sparse table of running maxima, level 0 a copy of the sigma table.  A
+   level needs the one before it.  Short tables: one block makes all levels,
+   each in a few of its iterations (a launch a level took 3 us each, 33 us at
+   n = 2600).  Long ones: blocks of RMQ_TILE entries make the levels that reach
+   no further than a tile from it, in shared memory, and the rest are a launch
+   each.  A majorant grid of 64^3 voxels at n = 2600, 16384 and 65536, us: one
+   block 21, 44 and 266, tiles 18, 32 and 42, a launch a level 57, 81 and 90. */
 __global__ void __launch_bounds__(1024) k_rmq(const float* __restrict__ sigma, float* __restrict__ table, int n, int levels)
 {
     for (int i = threadIdx.x; i < n; i += blockDim.x) table[i] = sigma[i];
@@ -133,6 +136,60 @@ __global__ void __launch_bounds__(1024) k_rmq(const float* __restrict__ sigma, f
             next[i] = b > a ? b : a;
         }
     }
+}
+
+#define RMQ_TILE 1024
+#define RMQ_TILE_LEVELS 11      /* levels 0 .. 10 reach 1023 entries further */
+
+__global__ void __launch_bounds__(RMQ_TILE) k_rmq_tile(const float* __restrict__ sigma, float* __restrict__ table, int n, int levels)
+{
+    __shared__ float v[2 * RMQ_TILE];
+    const int t = threadIdx.x, i0 = blockIdx.x * RMQ_TILE;
+    float a[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const int p = t + j * RMQ_TILE;
+        a[j] = i0 + p < n ? sigma[i0 + p] : 0.0f;
+        v[p] = a[j];
+    }
+    if (i0 + t < n) table[i0 + t] = a[0];
+    for (int k = 1; k < levels && k < RMQ_TILE_LEVELS; k++) {
+        const int half = 1 << (k - 1);
+        __syncthreads();
+        float b[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int p = t + j * RMQ_TILE;
+            b[j] = (p + half < 2 * RMQ_TILE && i0 + p + half < n) ? v[p + half] : a[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            a[j] = b[j] > a[j] ? b[j] : a[j];
+            v[t + j * RMQ_TILE] = a[j];
+        }
+        if (i0 + t < n) table[(size_t)k * n + i0 + t] = a[0];
+    }
+}
+
+__global__ void k_rmq_level(const float* __restrict__ prev, float* __restrict__ next, int n, int half)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float a = prev[i];
+    const float b = (i + half < n) ? prev[i + half] : a;
+    next[i] = b > a ? b : a;
+}
+
+static void launch_rmq(const float* sigma, float* table, int n, int levels, cudaStream_t s)
+{
+    if (n <= 4 * RMQ_TILE) {
+        k_rmq<<<1, 1024, 0, s>>>(sigma, table, n, levels);
+        return;
+    }
+    k_rmq_tile<<<(n + RMQ_TILE - 1) / RMQ_TILE, RMQ_TILE, 0, s>>>(sigma, table, n, levels);
+    for (int k = RMQ_TILE_LEVELS; k < levels; k++)
+        k_rmq_level<<<(n + 255) / 256, 256, 0, s>>>(table + (size_t)(k - 1) * n, table + (size_t)k * n, n, 1 << (k - 1));
 }
 
 __global__ void k_majorant(const uint32_t* __restrict__ minmax, const float* __restrict__ table, int n, int levels, float ds,
@@ -199,7 +256,7 @@ cudaError_t er_launch_majorant(const uint16_t* vox, const int res[3], int B, con
 {
     const long long total = (long long)nb[0] * nb[1] * nb[2];
     launch_minmax(vox, res, B, nb, minmax, s);
-    k_rmq<<<1, 1024, 0, s>>>(sigma, rmq, n, levels);
+    launch_rmq(sigma, rmq, n, levels, s);
     k_majorant<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(minmax, rmq, n, levels, density_scale, majorant, total);
     return cudaGetLastError();
 }
@@ -309,27 +366,37 @@ cudaError_t er_launch_empty_skip(float* majorant, const int nb[3], uint8_t* tmp,
    below its smaller end): a step there adds nothing to the march's sum, so
    the march may leave the lookup out.  A negative or NaN sigma counts as not
    empty. */
+/* running count of the nonzero entries (n <= 65536): a warp's ballots of 32
+   entries each, then a scan over those words, then the counts; loads and stores
+   coalesced and independent (64 neighbouring entries to a thread took 95 of the
+   235 us of a march tracer's edit and frame at n = 65536) */
 __global__ void __launch_bounds__(1024) k_nonzero_prefix(const float* __restrict__ sigma, uint32_t* __restrict__ count, int n)
 {
-    __shared__ uint32_t part[32];
-    const int per = (n + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int i0 = min((int)threadIdx.x * per, n), i1 = min(i0 + per, n);
-    uint32_t mine = 0;
-    for (int i = i0; i < i1; i++) mine += sigma[i] != 0.0f ? 1u : 0u;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t incl = mine;
+    __shared__ uint32_t word[2048], before[2048], part[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+#pragma unroll 8
+    for (int i0 = 0; i0 < n; i0 += 1024) {
+        const int i = i0 + t;
+        const uint32_t m = __ballot_sync(0xffffffffu, i < n && sigma[i] != 0.0f);
+        if (lane == 0) word[(i0 >> 5) + w] = m;
+    }
+    const int words = (n + 1023) / 1024 * 32;
+    __syncthreads();
+    const uint32_t c0 = 2 * t < words ? __popc(word[2 * t]) : 0u, c1 = 2 * t + 1 < words ? __popc(word[2 * t + 1]) : 0u;
+    uint32_t incl = c0 + c1;
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
     }
     if (lane == 31) part[w] = incl;
     __syncthreads();
-    uint32_t run = incl - mine;
+    uint32_t run = incl - c0 - c1;
     for (int k = 0; k < w; k++) run += part[k];
-    for (int i = i0; i < i1; i++) {
-        run += sigma[i] != 0.0f ? 1u : 0u;
-        count[i] = run;
-    }
+    before[2 * t] = run;
+    before[2 * t + 1] = run + c0;
+    __syncthreads();
+#pragma unroll 8
+    for (int i = t; i < n; i += 1024) count[i] = before[i >> 5] + (uint32_t)__popc(word[i >> 5] & (0xffffffffu >> (31 - (i & 31))));
 }
 
 __global__ void k_occupancy(const uint32_t* __restrict__ minmax, const uint32_t* __restrict__ count, int n, uint8_t* __restrict__ occ,

@@ -197,6 +197,41 @@ def test_majorant_grid_ragged(env, oracle, shape, brick):
     assert np.array_equal(bits(got.cpu().numpy()), bits(want))
 
 
+@pytest.mark.parametrize("n", [1, 2, 4095, 4096, 4097, 5120, 16384, 65535, 65536])
+def test_majorant_of_long_range_tables(env, oracle, n):
+    """one block's table, tiles, and the levels behind the tiles'"""
+    torch, lib, _ = env
+    rng = np.random.default_rng(n)
+    # bricks with ranges from one value to the whole table
+    vol = np.minimum(rng.integers(0, n, size=(24, 20, 28)), (n - 1) * rng.random((24, 20, 28)) ** 6).astype(np.uint16)
+    vol[8:16] = np.clip(n // 2 + rng.integers(-3, 4, size=vol[8:16].shape), 0, n - 1)
+    sig = np.abs(rng.normal(size=n)).astype(np.float32)
+    res = np.array(vol.shape[::-1], dtype=np.int32)
+    nb = [(d + 3) // 4 for d in vol.shape]
+    want = np.zeros(nb, dtype=np.float32)
+    oracle.majorant_grid(OL.ptr(vol), OL.ptr(res), 4, OL.ptr(sig), n, 3.0, OL.ptr(want))
+    d_vol, d_sig = torch.from_numpy(vol.view(np.int16)).cuda(), torch.from_numpy(sig).cuda()
+    got = torch.zeros(nb, dtype=torch.float32, device="cuda")
+    C.check(lib.er_build_majorant_device(d_vol.data_ptr(), res.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), 4, d_sig.data_ptr(), n, 3.0,
+                                         got.data_ptr(), None))
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(got.cpu().numpy()), bits(want))
+
+
+@pytest.mark.parametrize("top", [900, 4095, 4096, 40000, 65535])
+def test_march_map_of_long_tables(env, oracle, top):
+    """volumes up to the largest voxel: opacity zero but for one band of values"""
+    sc = S.scene_tiny(film=(24, 20), seed=3)
+    rng = np.random.default_rng(top)
+    v = (rng.random((22, 25, 27)) ** 8 * top).astype(np.uint16)
+    v[10:13, 9:16, 9:20] = rng.integers(top * 3 // 4, top + 1, size=(3, 7, 11))
+    v[11, 12, 13] = top
+    sc.volume = v
+    lo = 0.8 * top
+    sc.tracer.opacity = C.make_plf([(0.0, 0.0), (lo, 0.0), (lo + 1.0, 0.6), (top + 1.0, 0.6)])
+    check_sum(env, oracle, sc)
+
+
 @pytest.mark.parametrize("w,h", [(1, 1), (63, 17), (64, 16), (65, 33), (3, 200)])
 @pytest.mark.parametrize("radius", [0, 1, 5, 127])
 def test_bilateral_tiles(env, oracle, w, h, radius):

@@ -251,3 +251,13 @@ def test_gradient_maximum_of_small_values_goes_one_way(lib):
     r.gradient_magnitude()
     assert len([e for e in log(lib) if e[0] == "launch"]) == 1
     r.close()
+
+
+@pytest.mark.parametrize("n,blocks_of_one", [(300, True), (4096, True), (4097, False), (65536, False)])
+def test_long_range_tables_are_not_one_blocks_work(lib, n, blocks_of_one):
+    buf = np.zeros(1 << 21, np.float32)
+    res = (ctypes.c_int32 * 3)(8, 8, 8)
+    log(lib)
+    C.check(lib.er_build_majorant_device(buf.ctypes.data, res, 8, buf.ctypes.data, n, 1.0, buf.ctypes.data, None))
+    names = [e[2] for e in log(lib) if "k_rmq" in e[2]]
+    assert any("k_rmqPK" in x for x in names) == blocks_of_one
