@@ -72,6 +72,7 @@ struct DmParams {
     int model;           /* 0: B-spline opacity, isotropic albedo; 1: the tracer's transfer functions and shading */
     int emissive;        /* model 1: the tracer's emission TF is not zero everywhere */
     float gm_inv;        /* model 1, hybrid: 1 / gradient-magnitude range (a constant) */
+    uint32_t lit;        /* 1: the tracer has a light (0: no estimate has a job) */
     float gf3;           /* gradient_factor^3 (er_powf, the same bits on host and device) */
 };
 /* key: nonzero name of the walk (tracer build, medium, spp, view, first

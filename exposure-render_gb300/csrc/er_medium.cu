@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(256) k_dm_count(const Params P, const DmParams
                 if (!dm_track_step(P, k)) continue;
                 if (rng.get1() < M.q) {
                     dm_nee_draws(rng);
-                    n++;
+                    n += M.lit;
                 }
                 dm_track_next(P, rng, k);
             }
@@ -1422,16 +1422,29 @@ struct DmWorkspace {
     cudaError_t ensure_jobs(size_t n)
     {
         if (n <= cap) return cudaSuccess;
-        n = n + n / 4;
+        drop_jobs();
+        cudaError_t e = allocate_jobs(n + n / 4);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        drop_jobs();
+        if ((e = allocate_jobs(n)) != cudaSuccess) drop_jobs();
+        return e;
+    }
+    void drop_jobs()
+    {
         cudaFree(P); cudaFree(S); cudaFree(A); cudaFree(id); cudaFree(rng);
         P = S = A = nullptr;
         id = rng = nullptr;
+        cap = 0;
+    }
+    cudaError_t allocate_jobs(size_t n)
+    {
         cudaError_t e = cudaMalloc(&P, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&S, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&A, n * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&id, n * sizeof(uint2));
         if (e == cudaSuccess) e = cudaMalloc(&rng, n * sizeof(uint2));
-        cap = e == cudaSuccess ? n : 0;
+        if (e == cudaSuccess) cap = n;
         return e;
     }
 };
@@ -1494,11 +1507,12 @@ static cudaError_t dm_windows(const Params& P, const DmParams& M, int spp, uint3
     const bool one_window = (uint32_t)spp <= rows;
     const bool reuse = dimg && one_window && key != 0 && ws.key == key && ws.key_stream == s;
     ws.key = 0;
-    for (uint32_t s0 = 0; s0 < (uint32_t)spp; s0 += rows) {
+    for (uint32_t s0 = 0; s0 < (uint32_t)spp;) {
+        const uint32_t take = (uint32_t)spp - s0 < rows ? (uint32_t)spp - s0 : rows;
         DmWindow W;
         W.npix = npix;
         W.s0 = s0;
-        W.items = ((uint32_t)spp - s0 < rows ? (uint32_t)spp - s0 : rows) * npix;
+        W.items = take * npix;
         W.view = view;
         W.first = first;
         DmJobs J;
@@ -1515,7 +1529,14 @@ static cudaError_t dm_windows(const Params& P, const DmParams& M, int spp, uint3
             if ((e = cudaMemcpyAsync(ws.host_total, ws.total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
             if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
             njobs = *ws.host_total;
-            if ((e = ws.ensure_jobs(njobs)) != cudaSuccess) return e;
+            e = ws.ensure_jobs(njobs);
+            if (e == cudaErrorMemoryAllocation && take > 1) {
+                /* no room for the window's jobs: windows of half as many rows */
+                cudaGetLastError();
+                rows = (take + 1) / 2;
+                continue;
+            }
+            if (e != cudaSuccess) return e;
             J.P = ws.P; J.S = ws.S; J.A = ws.A; J.id = ws.id; J.rng = ws.rng; J.cap = (uint32_t)ws.cap;
             if (M.model == 1) k_dm_jobs<1><<<wave, 256, 0, s>>>(P, M, W, J);
             else k_dm_jobs<0><<<wave, 256, 0, s>>>(P, M, W, J);
@@ -1546,8 +1567,9 @@ static cudaError_t dm_windows(const Params& P, const DmParams& M, int spp, uint3
             }
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        s0 += take;
     }
-    if (one_window && key != 0) {
+    if ((uint32_t)spp <= rows && key != 0) {
         ws.key = key;
         ws.key_stream = s;
     }

@@ -2118,6 +2118,8 @@ static er_status medium_params(int32_t tracer_id, const er_medium_desc* m, erd::
     M.model = m->model;
     M.gm_inv = m->model == ER_MEDIUM_TRACER ? m->gradient_magnitude_inv : 0.0f;
     M.gf3 = er_powf(ts.gradient_factor, 3.0f);
+    M.lit = 0;
+    for (int i = 0; i < t->d.light_count; i++) M.lit |= ctx().lights.items.count(t->d.light_ids[i]) ? 1u : 0u;
     M.emissive = 0;
     if (m->model == ER_MEDIUM_TRACER)
         for (int c = 0; c < 3; c++)

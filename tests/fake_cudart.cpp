@@ -1,7 +1,7 @@
 // A CUDA runtime for the library's host code on a machine without a GPU:
 // device memory is host memory, copies are made at once, a kernel launch is a
-// line in a log (k_sample_voxels, whose output the host reads, is made here).
-// Allocations and device-to-host copies can be made to fail.
+// line in a log (k_sample_voxels and k_dm_count, whose output the host reads, are
+// made here).  Allocations and device-to-host copies can be made to fail.
 #include <cuda_runtime_api.h>
 
 #include <cstdint>
@@ -19,6 +19,8 @@ std::map<const void*, std::string>& names()
 }
 std::string text;
 int no_memory = 0;
+size_t largest = ~(size_t)0;
+unsigned jobs_each = 0;
 size_t bad_read = 0;
 
 void log(const char* what, const void* a, const std::string& b = "")
@@ -30,7 +32,7 @@ void log(const char* what, const void* a, const std::string& b = "")
 
 cudaError_t allocate(void** p, size_t n)
 {
-    if (no_memory) return cudaErrorMemoryAllocation;
+    if (no_memory || n > largest) return cudaErrorMemoryAllocation;
     *p = calloc(n ? n : 1, 1);
     return cudaSuccess;
 }
@@ -48,6 +50,8 @@ const char* fake_log() { return text.c_str(); }
 void fake_clear() { text.clear(); }
 void fake_no_memory(int on) { no_memory = on; }
 void fake_bad_read(size_t bytes) { bad_read = bytes; }
+void fake_largest_allocation(size_t bytes) { largest = bytes; }
+void fake_jobs_each(unsigned n) { jobs_each = n; }
 
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
@@ -80,6 +84,8 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void** a, size_t, cud
         uint16_t* out = *(uint16_t**)a[3];
         for (size_t i = 0; i * step < n; i++) out[i] = vox[i * step];
     }
+    /* (parameters, medium, window: (pixels, row, items, ..), jobs: seven arrays, total, ..) */
+    if (name.find("k_dm_count") != std::string::npos) *((uint32_t**)a[3])[7] = jobs_each * ((uint32_t*)a[2])[2];
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void** a, size_t sh, cudaStream_t s) { return __cudaLaunchKernel((cudaKernel_t)f, g, b, a, sh, s); }

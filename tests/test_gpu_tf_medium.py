@@ -279,3 +279,33 @@ def test_tracer_model_converges_to_the_product_image(torch, lib, pkg):
         assert d2 <= 1.5 * (var_a + var_b), (d2, var_a, var_b)
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("lights", ["none", "unbound"])
+def test_medium_without_a_light(torch, lib, pkg, oracle, lights):
+    """emission alone: no estimate of the walks has a job"""
+    runtime, medium = pkg
+    sc = S.tf_medium_scene(res=(16, 16, 16), film=(24, 20), n_nodes=12, emission=0.8)
+    if lights == "none":
+        sc.tracer.light_count = 0
+    else:
+        for i in range(sc.tracer.light_count):
+            sc.tracer.light_ids[i] = 30
+    r = runtime.Renderer(sc, lib)
+    rho_np = S.blob_density((16, 16, 16), n_blobs=4, seed=3)
+    rho, vals = torch.from_numpy(rho_np).cuda(), torch.from_numpy(S.plf_node_values(sc.tracer.opacity)).cuda()
+    m = medium.Medium(r, rho, vals, 30.0, brick=4, model="tracer", gradient_magnitude_inv=S.gradient_magnitude_range(rho_np))
+    try:
+        smp, s = m.render_samples(rho, vals, 4)
+        h = OL.MediumHandle(oracle, sc, rho_np, vals.cpu().numpy(), 30.0, np.array([0.8, 0.8, 0.8]), 0.5, m.majorant.cpu().numpy(), 4, model=1,
+                            gm_inv=m.gm_inv)
+        ref_sum, ref_smp = h.render(4, keep_samples=True, nthreads=4)
+        assert np.array_equal(bits(smp.cpu().numpy()), bits(ref_smp)) and np.abs(ref_sum).max() > 0.0
+        dimg = np.random.default_rng(2).normal(size=ref_sum.shape).astype(np.float32)
+        g_rho, g_tf = m.adjoint(rho, vals, 4, torch.from_numpy(dimg).cuda(), smp)
+        o_rho, o_tf = h.adjoint(4, dimg, ref_smp, nthreads=4)
+        h.close()
+        assert np.allclose(g_tf.cpu().numpy(), o_tf, rtol=1e-4, atol=1e-5 * np.abs(o_tf).max())
+        assert np.allclose(g_rho.cpu().numpy(), o_rho, rtol=1e-4, atol=1e-5 * np.abs(o_rho).max())
+    finally:
+        r.close()

@@ -33,11 +33,13 @@ def lib(fake_path, monkeypatch, tmp_path):
     monkeypatch.setenv("ER_TUNE_CACHE", str(tmp_path / "autotune.txt"))
     L = C.load_library(fake_path)
     L.fake_log.restype = ctypes.c_char_p
-    L.fake_bad_read.argtypes = [ctypes.c_size_t]
+    L.fake_bad_read.argtypes = L.fake_largest_allocation.argtypes = [ctypes.c_size_t]
     L.fake_no_memory(0)
     L.fake_bad_read(0)
     L.fake_clear()
     yield L
+    L.fake_jobs_each(0)
+    L.fake_largest_allocation(ctypes.c_size_t(-1).value)
     L.fake_no_memory(0)
     L.fake_bad_read(0)
     L.er_reset()
@@ -57,6 +59,13 @@ def renderer(lib, sc):
 STREAM_A, STREAM_B = 0x1000, 0x2000
 
 
+def medium_desc(p):
+    m = C.er_medium_desc()
+    m.d_density, m.d_opacity, m.n_opacity, m.scale, m.nee_probability = p, p, 16, 1.0, 0.5
+    m.d_majorant, m.brick, m.model = p, 8, C.ER_MEDIUM_SPLINE
+    return m
+
+
 @pytest.mark.parametrize("back", [False, True], ids=["forward", "adjoint"])
 def test_medium_calls_on_two_streams_take_turns(lib, back):
     """the walks of one device share their job and item arrays: a call on
@@ -65,9 +74,7 @@ def test_medium_calls_on_two_streams_take_turns(lib, back):
     r = renderer(lib, sc)
     buf = np.zeros(1 << 16, np.float32)
     p = buf.ctypes.data
-    m = C.er_medium_desc()
-    m.d_density, m.d_opacity, m.n_opacity, m.scale, m.nee_probability = p, p, 16, 1.0, 0.5
-    m.d_majorant, m.brick, m.model = p, 8, C.ER_MEDIUM_SPLINE
+    m = medium_desc(p)
 
     def call(stream):
         if back:
@@ -261,3 +268,18 @@ def test_long_range_tables_are_not_one_blocks_work(lib, n, blocks_of_one):
     C.check(lib.er_build_majorant_device(buf.ctypes.data, res, 8, buf.ctypes.data, n, 1.0, buf.ctypes.data, None))
     names = [e[2] for e in log(lib) if "k_rmq" in e[2]]
     assert any("k_rmqPK" in x for x in names) == blocks_of_one
+
+
+def test_medium_without_room_for_its_jobs_takes_smaller_windows(lib):
+    """the estimates of all samples get job slots, also those that find no light
+    sample: a window whose jobs do not fit is walked in halves"""
+    sc = S.medium_scene(res=(8, 8, 8), film=(32, 32))
+    r = renderer(lib, sc)
+    buf = np.zeros(1 << 18, np.float32)
+    m = medium_desc(buf.ctypes.data)
+    lib.fake_jobs_each(100)
+    # the items' arrays fit; 64 samples of 1024 pixels have 100 MiB of points, 16 have 25
+    lib.fake_largest_allocation((1 << 21) * 16)
+    C.check(lib.er_medium_render(r.tracer_id, ctypes.byref(m), 64, 0, 0, buf.ctypes.data, buf.ctypes.data, None))
+    assert sum("k_dm_gather" in e[2] for e in log(lib) if e[0] == "launch") == 4
+    r.close()
