@@ -270,7 +270,7 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    large grids an eighth of the blocks, spread over the volume, bounds first,
    and the rest only if that tells; a volume whose values are all within the
    error (a few labels) is not asked.  With and without the two passes, ms at
-   512^3: shells 1.6 and 4.3, one slope 5.2 and 4.3 (6.2 before it stopped),
+   512^3: shells 1.6 and 4.3, one slope 5.3 and 4.3 (6.2 before it stopped),
    smooth 4.43 and 4.32 (4.89 with all blocks first), eight labels 4.3 and 4.3
    (4.9); at 300^3 shells 0.33 and 0.93, smooth 1.07 and 0.92.
 
@@ -288,8 +288,8 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
 __host__ __device__ inline bool gm_bounds_tell(float low, float tol, float h) { return low > 3.0f * 2.0f * 1.7320508f * tol * h; }
 
 /* the exact pass in a grid of many waves (GM_EXACT_WIDE) at four blocks an SM,
-   its lookups out of line (all passes at 512^3 1.84 -> 1.58 ms); in a smaller
-   grid, where a block's own time counts, inline (128^3: 75 against 87 us) */
+   its lookups out of line (all passes at 512^3 1.84 -> 1.55 ms); in a smaller
+   grid, where a block's own time counts, inline */
 enum { GM_FIRST = 0, GM_REST = 1, GM_EXACT = 2, GM_EXACT_WIDE = 3 };
 
 /* bits: the largest magnitude, voxels looked up, the largest lower bound of the
@@ -318,20 +318,23 @@ __global__ void __launch_bounds__(GM_X * GM_Y, PASS == GM_EXACT_WIDE ? 4 : 1) k_
     const float low = PASS == GM_FIRST ? 0.0f : __uint_as_float(EXACT ? max(bits[2], bits[3]) : bits[2]);
     if (PASS != GM_FIRST && !gm_bounds_tell(low, tol, h)) return;
     unsigned int best = 0;
-    /* voxels looked up so far: read a plane ahead, so that nobody waits for it */
+    /* voxels looked up so far: asked about before a block's first and added
+       every eighth plane (in every plane it cost a tenth of the pass) */
     const bool asks = EXACT && tx == 0 && ty == 0;
-    unsigned int seen = 0;
-    if (asks) stop = 0;
+    unsigned int seen = 0, looks = 0;
+    if (asks) {
+        stop = 0;
+        seen = *(volatile unsigned int*)(bits + 1);
+    }
     int prev = plane(z0 - 1);
     /* cell z is in cells[(z + 3) % 3]; voxel z needs cells z - 1, z and z + 1 */
     for (int z = z0 - 1; z <= z1; z++) {
         const int next = plane(z + 1);
         cells[(z + 3) % 3][ty][tx] = prev + next;
         prev = next;
-        if (asks && seen > most) stop = 1;
-        if (asks) seen = *(volatile unsigned int*)(bits + 1);
+        if (asks && (z & 7) == 0 && seen > most) stop = 1;
         __syncthreads();
-        if (EXACT && stop) return;
+        if (EXACT && (z & 7) == 0 && stop) return;
         const int Z = z - 1;
         bool look = false;
         if (Z >= z0 && inner) {
@@ -347,10 +350,15 @@ __global__ void __launch_bounds__(GM_X * GM_Y, PASS == GM_EXACT_WIDE ? 4 : 1) k_
                 best = max(best, __float_as_uint(sqrtf(a * a + b * b + e * e) * 0.99999f));
             }
         }
-        if (EXACT) {
-            const unsigned m = __ballot_sync(0xffffffffu, look);
-            if (tx == 0 && m) atomicAdd(bits + 1, (unsigned int)__popc(m));
-            if (look) best = max(best, __float_as_uint(PASS == GM_EXACT ? voxel_gradient_magnitude(P, X, Y, Z) : voxel_gradient_magnitude_c(P, X, Y, Z)));
+        if (look) {
+            best = max(best, __float_as_uint(PASS == GM_EXACT ? voxel_gradient_magnitude(P, X, Y, Z) : voxel_gradient_magnitude_c(P, X, Y, Z)));
+            looks++;
+        }
+        if (EXACT && ((z & 7) == 4 || z == z1)) {
+            const unsigned int n = __reduce_add_sync(0xffffffffu, looks);
+            if (tx == 0 && n) atomicAdd(bits + 1, n);
+            if (asks) seen = *(volatile unsigned int*)(bits + 1);
+            looks = 0;
         }
         /* the next plane overwrites cell z - 2, which voxel z - 1 has read */
         __syncthreads();
