@@ -111,6 +111,11 @@ struct Clip {                /* ErClippingObject (Source/erclippingobject.h:27-5
     int invert;
 };
 
+/* the free-flight estimators of a launch's views */
+#define WF_MARCH 0
+#define WF_DELTA 1
+#define WF_MIXED 2
+
 enum { QUADS_NONE = 0, QUADS_INDEX32 = 1, QUADS_INDEX64 = 2, QUADS_BRICKED = 3 };
 
 struct Params {

@@ -484,10 +484,10 @@ ER_D bool dm_segment(const Params& P, const Ray& R, float& t0, float& t1)
 }
 
 /* ratio-tracked shadow transmittance as one loop (the binary64 evaluation) */
-template <int MODEL, typename Real>
-ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng)
+template <int MODEL>
+ER_D double dm_shadow64(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng)
 {
-    if (!P.shadows) return 1.0f;
+    if (!P.shadows) return 1.0;
     const v3 W = vnorm(vsub(P2, P1));
     Ray R;
     R.O = vadd(P1, vscale(W, ER_RAY_EPS));
@@ -495,10 +495,10 @@ ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng)
     R.MinT = 0.0f;
     R.MaxT = smin(vlen(vsub(P2, P1)) - 2.0f * ER_RAY_EPS, P.max_shadow_distance);
     float t0, t1;
-    if (!dm_segment(P, R, t0, t1)) return 1.0f;
+    if (!dm_segment(P, R, t0, t1)) return 1.0;
     Dda d;
     dda_init(P, R, t0, t1, d);
-    Real Tr = 1.0f;
+    double Tr = 1.0;
     float tau = -log_unit(rng.get1());
     int guard = 0;
     while (!d.done) {
@@ -515,12 +515,12 @@ ER_D Real dm_shadow(const Params& P, const DmParams& M, v3 P1, v3 P2, Rng& rng)
                 }
                 t = t + dt;
                 const v3 Pt = vadd(R.O, vscale(R.D, t));
-                DmLookup<Real> k;
+                DmLookup<double> k;
                 dm_density(P, M, Pt, k);
-                DmTf<Real> o;
-                dm_opacity<Real, MODEL>(P, M, k.rho, o);
-                const Real sig = (Real)M.scale * o.alpha;
-                Tr = Tr * ((Real)1.0f - sig / (Real)mu);
+                DmTf<double> o;
+                dm_opacity<double, MODEL>(P, M, k.rho, o);
+                const double sig = (double)M.scale * o.alpha;
+                Tr = Tr * (1.0 - sig / (double)mu);
                 if (++guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); return Tr; }
                 tau = -log_unit(rng.get1());
             }
@@ -571,26 +571,21 @@ ER_D void dm_shadow_stream(uint32_t seed, uint32_t view, uint32_t pix, uint32_t 
     er_seed_lanes(seed ^ er_hash32(0x51ED2705u + k), view ^ 0x6A09E667u, pix, sample, &r.s0, &r.s1);
 }
 
-/* one tentative collision of the camera ray, as the walker hands it over */
-template <typename Real>
-struct DmHit {
+/* one tentative collision of the camera ray of the binary64 evaluation */
+struct DmHit64 {
     v3 Pt;
-    float mu;
-    bool nee, has;       /* next-event estimate drawn here; it found a light sample */
+    bool has;            /* a next-event estimate drawn here found a light sample */
     uint32_t k_nee;      /* index of the estimate along the ray (its shadow stream) */
-    Real A0[3];          /* unshadowed next-event estimate */
+    double A0[3];        /* unshadowed next-event estimate */
     v3 S;                /* light sample point */
-    Real Le[3];          /* model 1: the emission at the collision */
-    v3 Wo;               /* model 1: minus the camera ray's direction */
-    v3 Wi;               /* model 1: light sample direction */
-    c3 LiK;              /* model 1: Li LightCount / (LightPdf q) */
+    double Le[3];        /* model 1: the emission at the collision */
 };
 
-/* the camera ray's tentative collisions in order; visit(hit, lookup,
-   opacity, sigma, w, T, shading) sees each with the throughput T before
-   it (shading: model 1's, prepared where a next-event estimate is drawn) */
-template <typename Real, int MODEL, typename Visit>
-ER_D void dm_walk(const Params& P, const DmParams& M, int x, int y, Rng& rng, Visit& visit)
+/* the camera ray's tentative collisions in order, the medium in binary64;
+   visit(hit, w, T) sees each with its weight sigma / mu and the throughput T
+   before it */
+template <int MODEL, typename Visit>
+ER_D void dm_walk64(const Params& P, const DmParams& M, int x, int y, Rng& rng, Visit& visit)
 {
     const v2 film_uv = rng.get2();
     const v2 lens_uv = rng.get2();
@@ -599,7 +594,7 @@ ER_D void dm_walk(const Params& P, const DmParams& M, int x, int y, Rng& rng, Vi
     if (!dm_segment(P, R, t0, t1)) return;
     Dda d;
     dda_init(P, R, t0, t1, d);
-    Real T = 1.0f;
+    double T = 1.0;
     float tau = -log_unit(rng.get1());
     uint32_t nee = 0;
     int guard = 0;
@@ -616,43 +611,35 @@ ER_D void dm_walk(const Params& P, const DmParams& M, int x, int y, Rng& rng, Vi
                     break;
                 }
                 t = t + dt;
-                DmHit<Real> h;
+                DmHit64 h;
                 h.Pt = vadd(R.O, vscale(R.D, t));
-                h.mu = mu;
-                h.Wo = vneg(R.D);
-                DmLookup<Real> k;
+                DmLookup<double> k;
                 dm_density(P, M, h.Pt, k);
-                DmTf<Real> o;
-                dm_opacity<Real, MODEL>(P, M, k.rho, o);
-                const Real sig = (Real)M.scale * o.alpha;
-                if (!(sig < (Real)mu)) atomicOr(P.err, 4);   /* the majorant no longer bounds sigma */
-                const Real w = sig / (Real)mu;
-                DmShade<Real> sd;
-                sd.type = -1;
+                DmTf<double> o;
+                dm_opacity<double, MODEL>(P, M, k.rho, o);
+                const double sig = (double)M.scale * o.alpha;
+                if (!(sig < (double)mu)) atomicOr(P.err, 4);   /* the majorant no longer bounds sigma */
+                const double w = sig / (double)mu;
 #pragma unroll
-                for (int c = 0; c < 3; c++) h.Le[c] = 0.0f;
-                if (MODEL == 1 && M.emissive) {
-#pragma unroll
-                    for (int c = 0; c < 3; c++) h.Le[c] = dm_tf_value<Real>(P.tfs->emission[c], k.rho);
-                }
+                for (int c = 0; c < 3; c++) h.Le[c] = MODEL == 1 && M.emissive ? dm_tf_value<double>(P.tfs->emission[c], k.rho) : 0.0;
                 h.has = false;
-                h.nee = rng.get1() < M.q;
-                if (h.nee) {
-                    if (MODEL == 1) dm_shade_prepare<Real>(P, M, h.Pt, k.rho, o, sd);
-                    const c3 a0 = dm_nee(P, M, h.Pt, rng, h.S, h.has, h.Wi, h.LiK);
+                if (rng.get1() < M.q) {
+                    v3 Wi;
+                    c3 LiK;
+                    const c3 a0 = dm_nee(P, M, h.Pt, rng, h.S, h.has, Wi, LiK);
+                    double S[3] = { 1.0, 1.0, 1.0 }, Sb[3], Sp[3];
                     if (MODEL == 1 && h.has) {
-                        Real S[3], Sb[3], Sp[3];
-                        dm_shade_eval<Real>(P, sd, h.Wo, h.Wi, S, Sb, Sp);
-                        h.A0[0] = S[0] * (Real)a0.r;
-                        h.A0[1] = S[1] * (Real)a0.g;
-                        h.A0[2] = S[2] * (Real)a0.b;
-                    } else {
-                        h.A0[0] = a0.r; h.A0[1] = a0.g; h.A0[2] = a0.b;
+                        DmShade<double> sd;
+                        dm_shade_prepare<double>(P, M, h.Pt, k.rho, o, sd);
+                        dm_shade_eval<double>(P, sd, vneg(R.D), Wi, S, Sb, Sp);
                     }
+                    h.A0[0] = S[0] * (double)a0.r;
+                    h.A0[1] = S[1] * (double)a0.g;
+                    h.A0[2] = S[2] * (double)a0.b;
                     h.k_nee = nee++;
                 }
-                visit(h, k, o, sig, w, T, sd);
-                T = T * ((Real)1.0f - w);
+                visit(h, w, T);
+                T = T * (1.0 - w);
                 if (++guard > ER_DELTA_MAX_COLLISIONS) { atomicOr(P.err, 2); return; }
                 tau = -log_unit(rng.get1());
             }
@@ -786,13 +773,14 @@ ER_D bool dm_track_again(DmTrack& k)
 }
 
 /* The persistent lanes of a walk.  A warp's lanes cross bricks together until
-   3/8 of them still do, then those at a collision make their lookups
-   together, and the next ones of their bricks, until as few are left (ending
-   them at 5/8 and 7/8, as the delta trackers do: 14.8 against 11.8 ms for the
-   tracer's model below; here nearly every lane has collisions to make); lanes whose ray ended take new work when a quarter of the
-   warp waits, one atomic per warp.  begin(i): sets the lane's ray up for work
-   item i (tracker not done) or leaves it done; collide(): the lane's
-   collision; end(): the ray is done. */
+   3/8 of them still do, then those at a collision make their lookups together,
+   and the next ones of their bricks, until as few are left.  (Ending them at
+   5/8 and 7/8, as the delta trackers' shadow stage does, took 14.8 against 11.8
+   ms for the tracer's model below: here nearly every lane has collisions to
+   make.)  Lanes whose ray ended take new work when a quarter of the warp
+   waits, one atomic per warp.  begin(i): sets the lane's ray up for work item i
+   (tracker not done) or leaves it done; collide(): the lane's collision; end():
+   the ray is done. */
 template <typename Begin, typename Collide, typename End>
 ER_D void dm_lanes(const Params& P, DmTrack& k, uint32_t n, uint32_t* fetch, Begin begin, Collide collide, End end)
 {
@@ -1258,8 +1246,7 @@ __global__ void __launch_bounds__(256) k_dm_forward64(const Params P, const DmPa
         const int x = (int)(pix % (uint32_t)P.film[0]), y = (int)(pix / (uint32_t)P.film[0]);
         double L0 = 0.0, L1 = 0.0, L2 = 0.0;
         double E0 = 0.0, E1 = 0.0, E2 = 0.0;
-        auto acc = [&](const DmHit<double>& h, const DmLookup<double>&, const DmTf<double>&, double, double w, double T,
-                       const DmShade<double>&) {
+        auto acc = [&](const DmHit64& h, double w, double T) {
             if (MODEL == 1) {
                 E0 += h.Le[0] * T * w;
                 E1 += h.Le[1] * T * w;
@@ -1268,12 +1255,12 @@ __global__ void __launch_bounds__(256) k_dm_forward64(const Params P, const DmPa
             if (!h.has) return;
             Rng sh;
             dm_shadow_stream(P.seed, view, pix, first + s, h.k_nee, sh);
-            const double Tr = dm_shadow<MODEL, double>(P, M, h.Pt, h.S, sh);
+            const double Tr = dm_shadow64<MODEL>(P, M, h.Pt, h.S, sh);
             L0 += h.A0[0] * Tr * T * w;
             L1 += h.A0[1] * Tr * T * w;
             L2 += h.A0[2] * Tr * T * w;
         };
-        dm_walk<double, MODEL>(P, M, x, y, rng, acc);
+        dm_walk64<MODEL>(P, M, x, y, rng, acc);
         samples[3 * i] = L0 + E0;
         samples[3 * i + 1] = L1 + E1;
         samples[3 * i + 2] = L2 + E2;

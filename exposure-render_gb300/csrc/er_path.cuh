@@ -29,11 +29,6 @@ namespace erd {
 #define ER_K_PRIMARY 4
 #define ER_K_SHADOW 4
 
-/* the free-flight estimators of a launch's views */
-#define WF_MARCH 0
-#define WF_DELTA 1
-#define WF_MIXED 2
-
 #define ER_PI_F 3.141592654f
 #define ER_INV_PI_F 0.31830988618379067154f
 #define ER_INV_TWO_PI_F 0.15915494309189533577f
@@ -435,22 +430,16 @@ ER_COLD bool clipped(const Params& P, v3 p)
     return false;
 }
 
-/* DensityScale * Opacity1D(I(p)) at a point of a free-flight or shadow
-   march, zero where a clipping object removes the volume (no lookup) */
-ER_D float sigma_point(const Params& P, v3 p)
-{
-    if (P.clip_count > 0 && clipped(P, p)) return 0.0f;
-    return sigma_at(P, get_intensity(P, p));
-}
-
-/* sigma_point where the march has the point's local coordinates already */
+/* DensityScale * Opacity1D(I(p)) at a step of a free-flight or shadow march,
+   whose point has the local coordinates (Lx, Ly, Lz); zero where a clipping
+   object removes the volume (no lookup) */
 ER_D float sigma_march(const Params& P, v3 p, float Lx, float Ly, float Lz)
 {
     if (P.clip_count > 0 && clipped(P, p)) return 0.0f;
     return sigma_at(P, get_intensity_local(P, Lx, Ly, Lz));
 }
 
-/* sigma_point at a tentative collision of a tracker in majorant brick
+/* The same at a tentative collision of a tracker in majorant brick
    (bx, by, bz): the local coordinates are clamped to the brick's extent
    [b B, (b + 1) B] per axis before the lookup, so that it blends only
    voxels of the brick's footprint (b B .. (b + 1) B), whose maximum the
@@ -939,9 +928,10 @@ ER_D long long march_budget(float t0, float t1, float step)
      to the even neighbour, leaves t even from its first on).  m d and t + m d
      are then multiples of the ulp below 2^24 of it: exact.
 
-   Measured: the reference's frame on the 512^3 shells (1024^2) 16.4 -> 3.1 ms,
-   its march at 64 samples a pixel of the 128^3 blobs (256^2) 12.9 -> 4.4 ms;
-   building the map is part of a tracer's build (0.2 ms at 512^3). */
+   Measured with the K steps in flight below: the reference's frame on the 512^3
+   shells (1024^2) 17.9 -> 2.2 ms, its march at 64 samples a pixel of the 128^3
+   blobs (256^2) 14.3 -> 4.4 ms; building the map is part of a tracer's build
+   (0.2 ms at 512^3). */
 ER_D float march_exit(const Params& P, const Ray& R, const v3& invd, float Lx, float Ly, float Lz)
 {
     const float B = (float)(1 << P.occ_shift);

@@ -138,7 +138,8 @@ cudaError_t er_launch_trace_frame(const Params& P, uint32_t* lanes, float4* fram
 {
     const dim3 b(16, 8);
     const dim3 g((P.film[0] + 15) / 16, (P.film[1] + 7) / 8);
-    /* four resident blocks an SM (128 registers): fewer do not fill it */
+    /* four resident blocks an SM (128 registers): under two waves of them a lane's own
+       chain is the frame's time (ER_K_FEW) */
     if ((size_t)g.x * g.y < 152 * 8) k_trace_frame<ER_K_FEW><<<g, b, 0, s>>>(P, lanes, frame);
     else k_trace_frame<ER_K_ONE><<<g, b, 0, s>>>(P, lanes, frame);
     return cudaGetLastError();

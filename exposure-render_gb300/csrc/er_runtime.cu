@@ -174,7 +174,7 @@ struct WfQueues {
         B.objects = 0;
         B.pt_primary = 0;
         B.pt_shadow = 0;
-        B.free_flight = 2;
+        B.free_flight = WF_MIXED;
         return cudaSuccess;
     }
     /* the shading records of the sorted shade stage, when a view mixes shaders */
@@ -581,7 +581,7 @@ er_status init_lanes(TracerItem& t)
    ER_TUNE_NO_SKIP_* bits are accepted and ignored. */
 void tracking_stages(int mode, bool all_delta, bool any_delta, WavefrontBuffers& B)
 {
-    B.free_flight = all_delta ? ER_FREE_FLIGHT_DELTA : (any_delta ? 2 : ER_FREE_FLIGHT_MARCH);   /* WF_MIXED = 2 */
+    B.free_flight = all_delta ? WF_DELTA : (any_delta ? WF_MIXED : WF_MARCH);
     mode &= 3;
     B.pt_primary = all_delta && (mode == ER_PERSISTENT_BOTH || mode == ER_PERSISTENT_PRIMARY);
     B.pt_shadow = all_delta && (mode == ER_PERSISTENT_SHADOW || mode == ER_PERSISTENT_BOTH);
