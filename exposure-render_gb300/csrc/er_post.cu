@@ -157,11 +157,15 @@ ER_D float lum255(uchar4 c)
    memory (a 4K film at radius 2: 161 us a pass before, when every tap read
    its range weight from the constant bank at a lane's own index and computed
    its luminance again).  The tile is BIL_N pixels along the pass's axis by
-   BIL_M across; the range weights sit in shared memory too. */
-#define BIL_N 64
+   BIL_M across; the range weights sit in shared memory too.  Films of under
+   600 tiles of 64 take 16 (a pixel to a thread), as four pixels one after the
+   other on a part of the chip are the longer way.  Both passes at radius 2 and
+   12, us, a tap's own reads and luminance / 64 / 16: 200 x 150 5.6, 16.2 / 9.6,
+   22.5 / 5.3, 8.7; 641 x 479 16.6, 94.7 / 13.7, 31.1 / 12.3, 22.4; 1024^2 46.6,
+   298 / 24.7, 60 / 28.1, 55.8; 3840 x 2160 341, 2312 / 134, 365 / -. */
 #define BIL_M 16
 
-template <bool HORIZONTAL>
+template <bool HORIZONTAL, int BIL_N>
 __global__ void __launch_bounds__(256) k_bilateral(const uchar4* __restrict__ in, uchar4* __restrict__ out, int W, int H, BilateralTables T)
 {
     extern __shared__ uint32_t tile[];          /* (BIL_N + 2 r) * BIL_M pixels, then as many luminances */
@@ -429,10 +433,18 @@ cudaError_t er_launch_bilateral(const uchar4* in, uchar4* tmp, uchar4* out, int 
                                 cudaStream_t s)
 {
     /* radius <= 127: at most 318 * 16 * 8 B = 40.7 KB */
-    const size_t bytes = (size_t)(BIL_N + 2 * T.radius) * BIL_M * 8;
-    const dim3 gh((W + BIL_N - 1) / BIL_N, (H + BIL_M - 1) / BIL_M), gv((W + BIL_M - 1) / BIL_M, (H + BIL_N - 1) / BIL_N);
-    k_bilateral<true><<<gh, 256, bytes, s>>>(in, tmp, W, H, T);
-    k_bilateral<false><<<gv, 256, bytes, s>>>(tmp, out, W, H, T);
+    const size_t rows = (size_t)((H + BIL_M - 1) / BIL_M), columns = (size_t)((W + BIL_M - 1) / BIL_M);
+    const bool few = (size_t)((W + 63) / 64) * rows < 600;
+    const int n = few ? 16 : 64;
+    const size_t bytes = (size_t)(n + 2 * T.radius) * BIL_M * 8;
+    const dim3 gh((W + n - 1) / n, (unsigned)rows), gv((unsigned)columns, (H + n - 1) / n);
+    if (few) {
+        k_bilateral<true, 16><<<gh, 256, bytes, s>>>(in, tmp, W, H, T);
+        k_bilateral<false, 16><<<gv, 256, bytes, s>>>(tmp, out, W, H, T);
+    } else {
+        k_bilateral<true, 64><<<gh, 256, bytes, s>>>(in, tmp, W, H, T);
+        k_bilateral<false, 64><<<gv, 256, bytes, s>>>(tmp, out, W, H, T);
+    }
     return cudaGetLastError();
 }
 

@@ -246,9 +246,10 @@ def test_bilateral_tiles(env, oracle, w, h, radius):
     assert np.array_equal(t.cpu().numpy(), tmp) and np.array_equal(o.cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("w,h", [(65535 * 16 + 1, 1), (65535 * 16 + 20, 3), (2, 524280)])
-def test_bilateral_of_very_wide_and_tall_images(env, oracle, w, h):
-    """more columns than a grid has rows of tiles, and as many rows as an image may have"""
+@pytest.mark.parametrize("w,h", [(65535 * 16 + 1, 1), (65535 * 16 + 20, 3), (2, 524280), (1030, 1001), (64 * 30, 16 * 20 - 1), (64 * 30 + 1, 16 * 20 - 1)])
+def test_bilateral_of_large_images(env, oracle, w, h):
+    """more columns than a grid has rows of tiles, as many rows as an image may
+    have, and the last film of short tiles and the first of long ones"""
     torch, lib, _ = env
     img = np.random.default_rng(w).integers(0, 256, size=(h, w, 4), dtype=np.uint8)
     want, tmp = np.zeros_like(img), np.zeros_like(img)
