@@ -274,9 +274,9 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    large grids an eighth of the blocks, spread over the volume, bounds first,
    and the rest only if that tells; a volume whose values are all within the
    error (a few labels) is not asked.  With and without the two passes, ms at
-   512^3: shells 1.6 and 4.3, one slope 5.3 and 4.3 (6.2 before it stopped),
+   512^3: shells 1.5 and 4.3, one slope 5.2 and 4.3 (6.2 before it stopped),
    smooth 4.43 and 4.32 (4.89 with all blocks first), eight labels 4.3 and 4.3
-   (4.9); at 300^3 shells 0.33 and 0.93, smooth 1.07 and 0.92.
+   (4.9); at 300^3 shells 0.30 and 0.93, smooth 1.07 and 0.92.
 
    A block walks GM_Z planes of a GM_X x GM_Y tile of cells (a ring of halo
    around the voxels): a thread sums its cell's four voxels of a plane, adds
@@ -291,16 +291,17 @@ __global__ void k_gradient_magnitude(const Params P, uint16_t* __restrict__ gm, 
    blobs went the long way) */
 __host__ __device__ inline bool gm_bounds_tell(float low, float tol, float h) { return low > 3.0f * 2.0f * 1.7320508f * tol * h; }
 
-/* the exact pass in a grid of many waves (GM_EXACT_WIDE) at four blocks an SM,
-   its lookups out of line (all passes at 512^3 1.84 -> 1.55 ms); in a smaller
-   grid, where a block's own time counts, inline */
+/* Four blocks an SM (32 registers) for the bounds, and for the exact pass in a
+   grid of many waves (GM_EXACT_WIDE), its lookups out of line: all passes at
+   512^3 1.46 ms, the exact one at two blocks 1.84.  In a smaller grid, where a
+   block's own time counts, inline at two (128^3: 75 us, out of line 87). */
 enum { GM_FIRST = 0, GM_REST = 1, GM_EXACT = 2, GM_EXACT_WIDE = 3 };
 
 /* bits: the largest magnitude, voxels looked up, the largest lower bound of the
    first pass and of the rest (two words: a pass decides on words that it does
    not write, so that a block's threads all decide the same) */
 template <int PASS>
-__global__ void __launch_bounds__(GM_X * GM_Y, PASS == GM_EXACT_WIDE ? 4 : 1) k_gm_cells(const Params P, float tol, unsigned int share, unsigned int most,
+__global__ void __launch_bounds__(GM_X * GM_Y, PASS == GM_EXACT ? 2 : 4) k_gm_cells(const Params P, float tol, unsigned int share, unsigned int most,
                                                               unsigned int* bits)
 {
     constexpr bool EXACT = PASS >= GM_EXACT;
@@ -497,7 +498,7 @@ cudaError_t er_launch_gradient_max(const Params& P, int vmax, unsigned int* bits
     const unsigned int share = blocks < 8192 ? 1 : 8;
     k_gm_cells<GM_FIRST><<<g, b, 0, s>>>(P, tol, share, most, bits);
     if (share > 1) k_gm_cells<GM_REST><<<g, b, 0, s>>>(P, tol, share, most, bits);
-    if (blocks < 1024) k_gm_cells<GM_EXACT><<<g, b, 0, s>>>(P, tol, share, most, bits);
+    if (blocks < 2500) k_gm_cells<GM_EXACT><<<g, b, 0, s>>>(P, tol, share, most, bits);
     else k_gm_cells<GM_EXACT_WIDE><<<g, b, 0, s>>>(P, tol, share, most, bits);
     return cudaGetLastError();
 }
