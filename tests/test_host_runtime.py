@@ -181,6 +181,27 @@ def test_tuning_key_made_late_equals_one_made_at_once(lib, monkeypatch, tmp_path
     assert keys[0] == keys[1]
 
 
+@pytest.mark.parametrize("memory", [True, False], ids=["room", "no-room"])
+def test_tuning_key_of_a_volume_bound_again(lib, monkeypatch, tmp_path, memory):
+    """an ID that held another, edited volume gives the new one's key"""
+    keys = []
+    for again in (False, True):
+        path = tmp_path / f"{again}.txt"
+        monkeypatch.setenv("ER_TUNE_CACHE", str(path))
+        sc = S.scene_tiny(res=32, film=(8, 8), seed=5)
+        r = renderer(lib, sc)
+        lib.fake_no_memory(0 if memory else 1)
+        if again:
+            C.check(edit(lib, r, BOXES[1], 77))
+            vd, vid = sc.volume_desc(), ctypes.c_int32(r.volume_id)
+            C.check(lib.er_bind_volume(ctypes.byref(vd), ctypes.byref(vid)))
+        C.check(edit(lib, r, BOXES[0], 100))
+        lib.fake_no_memory(0)
+        keys.append(tune_key(lib, r, path))
+        r.close()
+    assert keys[0] == keys[1]
+
+
 def test_an_edit_stands_when_its_key_cannot_be_made(lib):
     """edits whose log is over a megabyte make the key: a failure there leaves
     the edit made, and the next render with its tables"""
